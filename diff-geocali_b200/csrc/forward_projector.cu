@@ -11,8 +11,9 @@
 //
 // B200 design (not the reference's):
 //   * Z-fastest quad layout.  Per call the volume is re-laid out into an
-//     edge-replicated copy Q[y+1][x+1][z+1] = float4(v(z,y,x), v(z,y+1,x),
-//     v(z,y,x+1), v(z,y+1,x+1)) with z the fastest index.  The detector's V
+//     edge-replicated copy of quads with z the fastest index: Q[y+1][x+1][z+1]
+//     = float4(v, dv/dy, dv/dx, d2v/dxdy), the bilinear coefficients of the
+//     four corners (z,y..y+1,x..x+1) as finite differences.  The detector's V
 //     axis is parallel to z for every view, so the 32 lanes of a warp -- 32
 //     consecutive detector rows of one column -- sample nearly the same (x, y)
 //     at consecutive z: each 16-byte load of a warp touches a few contiguous
@@ -48,6 +49,23 @@ namespace dgc {
 // Volume re-layout: [D][H][W] -> Z-fastest edge-replicated quads
 // ---------------------------------------------------------------------------
 
+// A quad: the bilinear coefficients (v, dv/dy, dv/dx, d2v/dxdy) of the corners
+// (x0,y0), (x0,y1), (x1,y0), (x1,y1).  Its 64-bit halves are the pairs (value,
+// y difference) at x0 and their x differences, so the interpolation along x is
+// one packed fused multiply-add without a subtraction per sample, along y one
+// scalar one, and a quad gives the spatial gradient without further
+// differences.  The x differences are those a lerp of the corners forms.  The
+// marches are bound by the FP32 pipe and issue slots (65 % each) together with
+// the latency of L1 misses, so instructions out of the loop count: against
+// quads of the four corner values, forward 38.1 -> 35.6 ms at 256^3 / 360 x
+// 384^2, 3.51 -> 3.17 ms at 128^3 / 180 x 256^2, 89.4 -> 86.7 ms at 512^3 / 96
+// x 768^2; fused calibration step 50.4 -> 46.7 ms, geometry gradients alone
+// 54.4 -> 48.6 ms, all nine gradients 109.2 -> 104.9 ms at 256^3.
+__device__ __forceinline__ float4 quad_coefficients(float v00, float v01, float v10, float v11) {
+    const float dx = v10 - v00;
+    return make_float4(v00, v01 - v00, dx, (v11 - v01) - dx);
+}
+
 // One 32 x 32 (x, z) tile of the quads at padded row yp: block (32, 8).
 __device__ __forceinline__ void quads_tile(const float* __restrict__ vol, int D, int H, int W,
                                            float4* __restrict__ Q, int bx, int by,
@@ -64,12 +82,10 @@ __device__ __forceinline__ void quads_tile(const float* __restrict__ vol, int D,
         for (int zl = ty; zl < 32; zl += 8) {
             const int z = min(max(zp0 + zl - 1, 0), D - 1);
             const float* plane = vol + (long long)z * H * W;
-            // (x0,y0), (x0,y1), (x1,y0), (x1,y1): the y-pairs of each x are
-            // 64-bit halves, the operands of the packed lerps
-            tile[zl][tx] = make_float4(__ldg(plane + (long long)y0 * W + x0),
-                                       __ldg(plane + (long long)y1 * W + x0),
-                                       __ldg(plane + (long long)y0 * W + x1),
-                                       __ldg(plane + (long long)y1 * W + x1));
+            tile[zl][tx] = quad_coefficients(__ldg(plane + (long long)y0 * W + x0),
+                                             __ldg(plane + (long long)y1 * W + x0),
+                                             __ldg(plane + (long long)y0 * W + x1),
+                                             __ldg(plane + (long long)y1 * W + x1));
         }
     }
     __syncthreads();
@@ -100,8 +116,8 @@ int build_volume_quads(const float* vol, int D, int H, int W, float4* quads, cud
 // (v(z0, y, x), v(z1, y, x)) with y = yq-1, x = xq-1, z0 = zp-1, z1 = zp, all
 // clamped to the volume -- half the quads' bytes (8 per padded voxel).  A
 // cell's eight corners are four pairs (x and y neighbours at +(D+1) and
-// +(W+2)(D+1)), regrouped in registers into the two quads of the cell, so
-// the interpolation is bitwise the quad arm's.
+// +(W+2)(D+1)), made into the two quads of the cell in registers, so the
+// interpolation is bitwise the quad arm's.
 // grid: x = ceil((W+2)/32) * (H+2), y = ceil((D+1)/32); block (32, 8)
 __global__ void build_volume_pairs_kernel(const float* __restrict__ vol, int D, int H, int W,
                                           float2* __restrict__ P) {
@@ -303,18 +319,26 @@ __device__ __forceinline__ Cell locate(float x, float y, float z, const FpArgs& 
     return c;
 }
 
-// Loop invariants of the packed (x, y) sample position.
+// Loop invariants of the packed (x, y) sample position and of z.  They are
+// used where the voxel size is a power of two: source, direction and offset
+// scaled by 1/voxel beforehand are exact, so adding the half extent to the
+// scaled position rounds exactly as to_voxel's fused multiply-add of the
+// unscaled one, with two registers fewer (35.6 -> 35.2 ms at 256^3 / 360 x
+// 384^2, 3.17 -> 3.10 ms at 128^3 / 180 x 256^2).
 struct XYPacks {
-    f32x2 dxy, oxy, offxy, inv2, hxy, magic2;
+    f32x2 dxy, oxy, offxy, hxy, magic2;
+    float dz, oz, offz;
 };
 
 __device__ __forceinline__ XYPacks make_xy_packs(const RaySetup& r, const ViewGeo& vg,
                                                  const FpArgs& p) {
     XYPacks k;
-    k.dxy = pack2(r.dx, r.dy);
-    k.oxy = pack2(vg.ox, vg.oy);
-    k.offxy = pack2(p.off_x, p.off_y);
-    k.inv2 = pack2(p.inv_voxel, p.inv_voxel);
+    k.dxy = pack2(r.dx * p.inv_voxel, r.dy * p.inv_voxel);
+    k.oxy = pack2(vg.ox * p.inv_voxel, vg.oy * p.inv_voxel);
+    k.offxy = pack2(p.off_x * p.inv_voxel, p.off_y * p.inv_voxel);
+    k.dz = r.dz * p.inv_voxel;
+    k.oz = vg.oz * p.inv_voxel;
+    k.offz = p.off_z * p.inv_voxel;
     k.hxy = pack2(p.W * 0.5f, p.H * 0.5f);
     k.magic2 = pack2(kFloorMagic, kFloorMagic);
     return k;
@@ -332,13 +356,12 @@ __device__ __forceinline__ Cell sample_cell(float t, const RaySetup& r, const Vi
     const float hz = p.D * 0.5f;
     if constexpr (PACK && !CLAMP && !DIV) {
         const f32x2 pxy = fma2(pack2(t, t), k.dxy, k.oxy);
-        const f32x2 vxy = fma2(OFF ? sub2(pxy, k.offxy) : pxy, k.inv2, k.hxy);
+        const f32x2 vxy = add2(OFF ? sub2(pxy, k.offxy) : pxy, k.hxy);
         const f32x2 fxy = add2_rd(vxy, k.magic2);
         const float2 frac = unpack2(sub2(vxy, sub2(fxy, k.magic2)));
         const uint2 bits = unpack2_bits(fxy);
-        const FloorSplit sz =
-            floor_split(to_voxel<false, OFF>(fmaf(t, r.dz, vg.oz), p.off_z, p.voxel_size,
-                                             p.inv_voxel, hz));
+        const float pz = fmaf(t, k.dz, k.oz);
+        const FloorSplit sz = floor_split((OFF ? pz - k.offz : pz) + hz);
         Cell c;
         c.bx = bits.x;
         c.by = bits.y;
@@ -382,9 +405,19 @@ __device__ __forceinline__ void load_cell(const ulonglong2* __restrict__ Q, uint
     }
 }
 
-// Sum of the trilinear samples along the ray (fp.cu:321-335).  The quads
-// hold the y-pairs of x0 and x1 as 64-bit halves, so the interpolation runs
-// as packed pairs: along x for (y0, y1) at z0 and z1, along z, then along y.
+// Trilinear value of a cell's two quads at a sample's weights.
+__device__ __forceinline__ float quad_value(const ulonglong2& q0, const ulonglong2& q1,
+                                            const Cell& c) {
+    const f32x2 wx = pack2(c.fx, c.fx);
+    const f32x2 e0 = fma2(wx, q0.y, q0.x);  // (value, y difference) at z0
+    const f32x2 e1 = fma2(wx, q1.y, q1.x);  // (value, y difference) at z1
+    const float2 e = unpack2(lerp2(e0, e1, pack2(c.fz, c.fz)));
+    return fmaf(c.fy, e.y, e.x);
+}
+
+// Sum of the trilinear samples along the ray (fp.cu:321-335).  The
+// interpolation runs on packed (value, y difference) pairs: along x at z0 and
+// z1, along z, then along y.
 // UNROLL: the march loop unrolled by the compiler (1 or 2; the same samples
 // and sums either way, a tuned dimension of the forward).
 template <bool CLAMP, bool DIV, bool OFF, bool GUARD = true, int UNROLL = 1>
@@ -401,11 +434,7 @@ __device__ __forceinline__ float march_sum(const RaySetup& r, const ViewGeo& vg,
         const Cell c = sample_cell<CLAMP, DIV, OFF, true>(t, r, vg, p, k);
         load_cell(Q, quad_index(c, p), cq);
         const ulonglong2 q0 = cq.q0, q1 = cq.q1;
-        const f32x2 wx = pack2(c.fx, c.fx);
-        const f32x2 e0 = lerp2(q0.x, q0.y, wx);  // (y0, y1) at z0
-        const f32x2 e1 = lerp2(q1.x, q1.y, wx);  // (y0, y1) at z1
-        const float2 e = unpack2(lerp2(e0, e1, pack2(c.fz, c.fz)));
-        acc += lerpf(e.x, e.y, c.fy);
+        acc += quad_value(q0, q1, c);
     }
     return acc;
 }
@@ -515,7 +544,7 @@ __global__ void __launch_bounds__(256) fp_forward_kernel(FpArgs p) {
 // ---------------------------------------------------------------------------
 
 // march_sum over the z-pair layout: the same samples, cells and packed lerps
-// (the four pairs of a cell regrouped into its two quads), four 8-byte loads
+// (the four pairs of a cell made into its two quads), four 8-byte loads
 // per new cell instead of two 16-byte ones.
 template <bool CLAMP, bool DIV, bool OFF, bool GUARD = true>
 __device__ __forceinline__ float march_sum_pairs(const RaySetup& r, const ViewGeo& vg,
@@ -535,18 +564,18 @@ __device__ __forceinline__ float march_sum_pairs(const RaySetup& r, const ViewGe
         const Cell c = sample_cell<CLAMP, DIV, OFF, true>(t, r, vg, p, k);
         const uint32_t pi = c.bz + c.bx * sx + c.by * sy + bias;
         if (pi != cq.qi) {
-            const float2 p00 = unpack2(__ldg(P + pi)), p10 = unpack2(__ldg(P + pi + sx));
-            const float2 p01 = unpack2(__ldg(P + pi + sy)), p11 = unpack2(__ldg(P + pi + sy + sx));
-            cq.q0 = make_ulonglong2(pack2(p00.x, p01.x), pack2(p10.x, p11.x));
-            cq.q1 = make_ulonglong2(pack2(p00.y, p01.y), pack2(p10.y, p11.y));
+            // the coefficients of quad_coefficients at z0 and z1 as packed pairs
+            const unsigned long long p00 = __ldg(P + pi), p10 = __ldg(P + pi + sx);
+            const unsigned long long p01 = __ldg(P + pi + sy), p11 = __ldg(P + pi + sy + sx);
+            const f32x2 d10 = sub2(p10, p00);
+            const float2 v = unpack2(p00), dy = unpack2(sub2(p01, p00)), dx = unpack2(d10);
+            const float2 dxy = unpack2(sub2(sub2(p11, p01), d10));
+            cq.q0 = make_ulonglong2(pack2(v.x, dy.x), pack2(dx.x, dxy.x));
+            cq.q1 = make_ulonglong2(pack2(v.y, dy.y), pack2(dx.y, dxy.y));
             cq.qi = pi;
         }
         const ulonglong2 q0 = cq.q0, q1 = cq.q1;
-        const f32x2 wx = pack2(c.fx, c.fx);
-        const f32x2 e0 = lerp2(q0.x, q0.y, wx);
-        const f32x2 e1 = lerp2(q1.x, q1.y, wx);
-        const float2 e = unpack2(lerp2(e0, e1, pack2(c.fz, c.fz)));
-        acc += lerpf(e.x, e.y, c.fy);
+        acc += quad_value(q0, q1, c);
     }
     return acc;
 }
@@ -683,11 +712,7 @@ __device__ __forceinline__ void tma_march_slab(const RaySetup& r, const ViewGeo&
             q0 = __ldg(Q + qi);
             q1 = __ldg(Q + qi + 1);
         }
-        const f32x2 wx = pack2(c.fx, c.fx);
-        const f32x2 e0 = lerp2(q0.x, q0.y, wx);
-        const f32x2 e1 = lerp2(q1.x, q1.y, wx);
-        const float2 e = unpack2(lerp2(e0, e1, pack2(c.fz, c.fz)));
-        acc += lerpf(e.x, e.y, c.fy);
+        acc += quad_value(q0, q1, c);
     }
 }
 
@@ -866,6 +891,30 @@ struct RayGrad {
     float s1x, s1y, s1z, s2x, s2y, s2z;
 };
 
+// Value (exactly quad_value's) and spatial gradient in voxel units of the
+// trilinear interpolant at a sample, from the same packed pairs: d/dy is the
+// interpolated y difference, d/dz the difference of the two z levels, d/dx the
+// x differences interpolated along z and y.
+struct QuadGradient {
+    float value, x, y, z;
+};
+
+__device__ __forceinline__ QuadGradient quad_gradient(const ulonglong2& q0, const ulonglong2& q1,
+                                                      const Cell& c) {
+    const f32x2 wx = pack2(c.fx, c.fx), wz = pack2(c.fz, c.fz);
+    const f32x2 e0 = fma2(wx, q0.y, q0.x), e1 = fma2(wx, q1.y, q1.x);
+    const f32x2 ez = sub2(e1, e0);
+    const float2 e = unpack2(fma2(wz, ez, e0));
+    const float2 dx = unpack2(lerp2(q0.y, q1.y, wz));
+    const float2 dz = unpack2(ez);
+    QuadGradient g;
+    g.value = fmaf(c.fy, e.y, e.x);
+    g.x = fmaf(c.fy, dx.y, dx.x);
+    g.y = e.y;
+    g.z = fmaf(c.fy, dz.y, dz.x);
+    return g;
+}
+
 // GRADVOL: also scatter the adjoint of every sample into p.grad_pad, a
 // cell-major buffer of 16-byte level records R[(cy*(W+1) + cx)*(D+2) + cz]
 // (cells at padded index floor+1): record c holds the weights of the four
@@ -894,25 +943,14 @@ __device__ __forceinline__ RayGrad march_grad(const RaySetup& r, const ViewGeo& 
         const uint32_t qi = quad_index(c, p);
         const ulonglong2 q0 = __ldg(Q + qi);
         const ulonglong2 q1 = __ldg(Q + qi + 1);
-        // d/dx, d/dy, d/dz of the trilinear interpolant (voxel units), from
-        // packed (y0, y1) pairs: .x of a quad is x0, .y is x1
-        const f32x2 wx = pack2(c.fx, c.fx), wz = pack2(c.fz, c.fz);
-        const f32x2 d0 = sub2(q0.y, q0.x), d1 = sub2(q1.y, q1.x);  // x1 - x0
-        const f32x2 e0 = fma2(wx, d0, q0.x), e1 = fma2(wx, d1, q1.x);
-        const f32x2 ez = sub2(e1, e0);
-        const float2 e = unpack2(fma2(wz, ez, e0));
-        const float2 dx = unpack2(fma2(wz, sub2(d1, d0), d0));
-        const float2 dz = unpack2(ez);
-        const float gx = lerpf(dx.x, dx.y, c.fy);
-        const float gy = e.y - e.x;
-        const float gz = lerpf(dz.x, dz.y, c.fy);
+        const QuadGradient g = quad_gradient(q0, q1, c);
         const float tau = t - r.tmin;
-        rg.s1x += gx;
-        rg.s1y += gy;
-        rg.s1z += gz;
-        rg.s2x = fmaf(gx, tau, rg.s2x);
-        rg.s2y = fmaf(gy, tau, rg.s2y);
-        rg.s2z = fmaf(gz, tau, rg.s2z);
+        rg.s1x += g.x;
+        rg.s1y += g.y;
+        rg.s1z += g.z;
+        rg.s2x = fmaf(g.x, tau, rg.s2x);
+        rg.s2y = fmaf(g.y, tau, rg.s2y);
+        rg.s2z = fmaf(g.z, tau, rg.s2z);
         if (GRADVOL) {
             // adjoint of the trilinear sample (fp.cu:231-240) into the level records
             const float mx = 1.0f - c.fx, my = 1.0f - c.fy, mz = 1.0f - c.fz;
@@ -1096,31 +1134,15 @@ __device__ __forceinline__ RayValueGrad march_value_grad(const RaySetup& r, cons
         const uint32_t qi = quad_index(c, p);
         const ulonglong2 q0 = __ldg(Q + qi);
         const ulonglong2 q1 = __ldg(Q + qi + 1);
-        // value: exactly the forward kernel's packed lerps (lerp2(a, b, w) =
-        // fma2(w, b - a, a)), keeping the intermediate pairs
-        const f32x2 wx = pack2(c.fx, c.fx), wz = pack2(c.fz, c.fz);
-        const f32x2 d0 = sub2(q0.y, q0.x);  // x1 - x0 at (y0, y1), z0
-        const f32x2 d1 = sub2(q1.y, q1.x);  // x1 - x0 at (y0, y1), z1
-        const f32x2 e0 = fma2(wx, d0, q0.x);
-        const f32x2 e1 = fma2(wx, d1, q1.x);
-        const f32x2 ez = sub2(e1, e0);
-        const float2 e = unpack2(fma2(wz, ez, e0));
-        out.sum += lerpf(e.x, e.y, c.fy);
-        // spatial gradient from the same pairs (the trilinear interpolant is
-        // linear along each axis): d/dx = lerp_y(lerp_z(x1 - x0)),
-        // d/dy = Y1 - Y0, d/dz = lerp_y(lerp_x(z1) - lerp_x(z0))
-        const float2 dx = unpack2(fma2(wz, sub2(d1, d0), d0));
-        const float2 dz = unpack2(ez);
-        const float gx = lerpf(dx.x, dx.y, c.fy);
-        const float gy = e.y - e.x;
-        const float gz = lerpf(dz.x, dz.y, c.fy);
+        const QuadGradient g = quad_gradient(q0, q1, c);
+        out.sum += g.value;
         const float tau = t - r.tmin;
-        out.g.s1x += gx;
-        out.g.s1y += gy;
-        out.g.s1z += gz;
-        out.g.s2x = fmaf(gx, tau, out.g.s2x);
-        out.g.s2y = fmaf(gy, tau, out.g.s2y);
-        out.g.s2z = fmaf(gz, tau, out.g.s2z);
+        out.g.s1x += g.x;
+        out.g.s1y += g.y;
+        out.g.s1z += g.z;
+        out.g.s2x = fmaf(g.x, tau, out.g.s2x);
+        out.g.s2y = fmaf(g.y, tau, out.g.s2y);
+        out.g.s2z = fmaf(g.z, tau, out.g.s2z);
     }
     return out;
 }

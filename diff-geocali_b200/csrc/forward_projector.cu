@@ -347,9 +347,10 @@ __device__ __forceinline__ XYPacks make_xy_packs(const RaySetup& r, const ViewGe
 // Cell of the sample at t.  With PACK, no clamping and the multiplying voxel
 // conversion, x and y run as packed pairs (fma.rn / sub.rn / add.rm on
 // f32x2): lane by lane the same IEEE operations as the scalar path, so the
-// cell and weights are bitwise those of locate(to_voxel(...)).  Measured on
-// the forward sum 1-3 % faster; in the gradient marches (more live values)
-// the scalar form is faster, so they keep it.
+// cell and weights are bitwise those of locate(to_voxel(...)).  On the forward
+// sum 1-3 % faster; the gradient marches, together with dropping the iteration
+// counter and a zero ROI offset, 48.6 -> 43.2 ms (geometry gradients) and 46.7
+// -> 45.5 ms (fused calibration step) at 256^3 / 360 x 384^2.
 template <bool CLAMP, bool DIV, bool OFF, bool PACK>
 __device__ __forceinline__ Cell sample_cell(float t, const RaySetup& r, const ViewGeo& vg,
                                             const FpArgs& p, const XYPacks& k) {
@@ -922,7 +923,7 @@ __device__ __forceinline__ QuadGradient quad_gradient(const ulonglong2& q0, cons
 // its z level to its cell's record and its z+1 level to the next record;
 // fold_record_gradient_kernel then sums the records onto the voxels.  A
 // lane's consecutive samples of one cell are first added in registers.
-template <bool CLAMP, bool GRADVOL>
+template <bool CLAMP, bool GRADVOL, bool POW2, bool OFF, bool GUARD>
 __device__ __forceinline__ RayGrad march_grad(const RaySetup& r, const ViewGeo& vg,
                                               const FpArgs& p, float gs) {
     const ulonglong2* __restrict__ Q = reinterpret_cast<const ulonglong2*>(p.quads);
@@ -938,8 +939,8 @@ __device__ __forceinline__ RayGrad march_grad(const RaySetup& r, const ViewGeo& 
     float t = r.tmin;
     int n = 0;
 #pragma unroll 1
-    for (; t <= r.tmax && n < nmax; t += p.step_size, ++n) {
-        const Cell c = sample_cell<CLAMP, false, true, false>(t, r, vg, p, k);
+    for (; t <= r.tmax && (!GUARD || n < nmax); t += p.step_size, n += GUARD ? 1 : 0) {
+        const Cell c = sample_cell<CLAMP, false, OFF, POW2>(t, r, vg, p, k);
         const uint32_t qi = quad_index(c, p);
         const ulonglong2 q0 = __ldg(Q + qi);
         const ulonglong2 q1 = __ldg(Q + qi + 1);
@@ -1046,7 +1047,7 @@ __device__ __forceinline__ void ray_geometry_terms(const FpArgs& p, const ViewGe
 // The eight per-view geometry terms of one ray (zero for rays outside the
 // detector, missing the volume or with a zero upstream gradient); with
 // GRADVOL (march_grad) the ray's adjoint samples go into p.grad_pad.
-template <bool GRADVOL>
+template <bool GRADVOL, bool POW2, bool OFF>
 __device__ __forceinline__ void backward_ray(const FpArgs& p, const ViewGeo& vg, int a, int u,
                                              int v, float (&terms)[8]) {
 #pragma unroll
@@ -1059,9 +1060,14 @@ __device__ __forceinline__ void backward_ray(const FpArgs& p, const ViewGeo& vg,
         const RaySetup r = setup_ray(vg, u, v, p);
         if (r.ok && r.hit) {
             const float gs = grad_out * p.step_size;
-            const RayGrad rg = ray_inside_pad<false>(r, vg, p)
-                                   ? march_grad<false, GRADVOL>(r, vg, p, gs)
-                                   : march_grad<true, GRADVOL>(r, vg, p, gs);
+            const bool inside = ray_inside_pad<false>(r, vg, p);
+            RayGrad rg;
+            if (steps_advance(r, p.step_size))
+                rg = inside ? march_grad<false, GRADVOL, POW2, OFF, false>(r, vg, p, gs)
+                            : march_grad<true, GRADVOL, POW2, OFF, false>(r, vg, p, gs);
+            else
+                rg = inside ? march_grad<false, GRADVOL, POW2, OFF, true>(r, vg, p, gs)
+                            : march_grad<true, GRADVOL, POW2, OFF, true>(r, vg, p, gs);
             ray_geometry_terms(p, vg, r, u, rg, gs, terms);
         }
     }
@@ -1087,7 +1093,10 @@ __device__ __forceinline__ void reduce_terms_to_partials(const float (&terms)[8]
     }
 }
 
-template <int TU, bool GRADVOL>
+// POW2 without OFF is the march for power-of-two voxel sizes and no ROI offset
+// (sample_cell's packed form); every other case runs the general one, POW2 =
+// false and OFF = true, which is right for all of them.
+template <int TU, bool GRADVOL, bool POW2, bool OFF>
 __global__ void __launch_bounds__(256) fp_backward_kernel(FpArgs p) {
     constexpr int TV = 256 / TU;
     __shared__ ViewGeo s_view;
@@ -1103,7 +1112,7 @@ __global__ void __launch_bounds__(256) fp_backward_kernel(FpArgs p) {
     int u, v;
     tile_ray<TU>(tc, u, v);
     float terms[8];
-    backward_ray<GRADVOL>(p, vg, a, u, v, terms);
+    backward_ray<GRADVOL, POW2, OFF>(p, vg, a, u, v, terms);
     reduce_terms_to_partials(terms, s_red, p.partials + ((long long)a * tiles + tile) * 8);
 }
 
@@ -1130,7 +1139,7 @@ __device__ __forceinline__ RayValueGrad march_value_grad(const RaySetup& r, cons
     int n = 0;
 #pragma unroll 1
     for (; t <= r.tmax && (!GUARD || n < nmax); t += p.step_size, n += GUARD ? 1 : 0) {
-        const Cell c = sample_cell<CLAMP, DIV, OFF, false>(t, r, vg, p, k);
+        const Cell c = sample_cell<CLAMP, DIV, OFF, true>(t, r, vg, p, k);
         const uint32_t qi = quad_index(c, p);
         const ulonglong2 q0 = __ldg(Q + qi);
         const ulonglong2 q1 = __ldg(Q + qi + 1);
@@ -1387,11 +1396,19 @@ __global__ void __launch_bounds__(256, 6) batch_forward_kernel(BatchTables t) {
 
 template <int TU>
 __device__ __forceinline__ void backward_item(const FpArgs& p, const ViewGeo& vg,
-                                              const TileCoord& tc, float (&terms)[8]) {
+                                              const TileCoord& tc, int flags, float (&terms)[8]) {
     int u, v;
     tile_ray<TU>(tc, u, v);
-    if (p.grad_pad) backward_ray<true>(p, vg, tc.a, u, v, terms);
-    else backward_ray<false>(p, vg, tc.a, u, v, terms);
+    switch (flags & (kBatchDiv | kBatchOff)) {
+        case 0:
+            if (p.grad_pad) backward_ray<true, true, false>(p, vg, tc.a, u, v, terms);
+            else backward_ray<false, true, false>(p, vg, tc.a, u, v, terms);
+            break;
+        default:
+            if (p.grad_pad) backward_ray<true, false, true>(p, vg, tc.a, u, v, terms);
+            else backward_ray<false, false, true>(p, vg, tc.a, u, v, terms);
+            break;
+    }
 }
 
 __global__ void __launch_bounds__(256, 4) batch_backward_kernel(BatchTables t) {
@@ -1407,8 +1424,8 @@ __global__ void __launch_bounds__(256, 4) batch_backward_kernel(BatchTables t) {
         const ViewGeo vg = s_view;
         const TileCoord tc = s_tc;
         float terms[8];
-        if (s_tu == 8) backward_item<8>(p, vg, tc, terms);
-        else backward_item<4>(p, vg, tc, terms);
+        if (s_tu == 8) backward_item<8>(p, vg, tc, s_flags, terms);
+        else backward_item<4>(p, vg, tc, s_flags, terms);
         const long long tiles = fp_tiles_per_view_dev(p.U, p.V, s_tu);
         reduce_terms_to_partials(terms, s_red, p.partials + ((long long)tc.a * tiles + s_tile) * 8);
         __syncthreads();
@@ -1466,8 +1483,15 @@ template <int TU>
 int launch_backward_tu(const FpArgs& p, bool gradvol, cudaStream_t s) {
     DGC_TRACE(gradvol ? "fp_backward_kernel<gradvol>" : "fp_backward_kernel", s);
     const long long blocks = fp_tiles_per_view(p.U, p.V, TU) * (long long)p.A;
-    if (gradvol) fp_backward_kernel<TU, true><<<(unsigned)blocks, 256, 0, s>>>(p);
-    else fp_backward_kernel<TU, false><<<(unsigned)blocks, 256, 0, s>>>(p);
+    const bool fast = is_pow2_float(p.voxel_size) && p.off_x == 0.0f && p.off_y == 0.0f &&
+                      p.off_z == 0.0f;
+    if (gradvol) {
+        if (fast) fp_backward_kernel<TU, true, true, false><<<(unsigned)blocks, 256, 0, s>>>(p);
+        else fp_backward_kernel<TU, true, false, true><<<(unsigned)blocks, 256, 0, s>>>(p);
+    } else {
+        if (fast) fp_backward_kernel<TU, false, true, false><<<(unsigned)blocks, 256, 0, s>>>(p);
+        else fp_backward_kernel<TU, false, false, true><<<(unsigned)blocks, 256, 0, s>>>(p);
+    }
     DGC_LAUNCH_CHECK("fp_backward_kernel");
     return DGC_OK;
 }

@@ -8,7 +8,7 @@
 //   view[n+1] | fold_block[n+1] | counters[2] |
 //   per instance: quads | partials            | ... |
 //   per instance with a volume gradient: gradient buffer | ...
-// (level records).  The gradient buffers are contiguous, so one memset
+// (edge records).  The gradient buffers are contiguous, so one memset
 // clears all of them.
 #include <string>
 #include <vector>
@@ -25,10 +25,8 @@ size_t quads_bytes(const dgc_fp_instance& in) {
     return align256(sizeof(float4) * (size_t)(in.D + 2) * (size_t)(in.H + 1) * (size_t)(in.W + 1));
 }
 
-// volume-gradient buffer (level records)
-size_t gpad_bytes(const dgc_fp_instance& in) {
-    return align256(sizeof(float) * fp_record_buffer_floats(in.D, in.H, in.W));
-}
+// volume-gradient buffer: the edge records (fp_edge_bytes) take about half of it
+size_t gpad_bytes(const dgc_fp_instance& in) { return quads_bytes(in); }
 
 int tile_fwd(const dgc_fp_instance& in) { return in.tile_forward == 0 ? 8 : in.tile_forward; }
 int tile_bwd(const dgc_fp_instance& in) { return in.tile_backward == 0 ? 8 : in.tile_backward; }
@@ -166,7 +164,7 @@ int dgc_batch_prepare(const dgc_fp_instance* instances, int n, void* workspace,
         p.projections = in.projections;
         p.grad_projections = in.grad_projections;
         if (in.grad_volume) {
-            p.grad_pad = reinterpret_cast<float*>(base + gpad_off + gpad_total);
+            p.grad_edges = reinterpret_cast<float2*>(base + gpad_off + gpad_total);
             gpad_total += gpad_bytes(in);
         }
         b.volume = in.volume;
@@ -179,13 +177,14 @@ int dgc_batch_prepare(const dgc_fp_instance* instances, int n, void* workspace,
                   ((in.off_x != 0.0f || in.off_y != 0.0f || in.off_z != 0.0f) ? kBatchOff : 0);
         b.quad_gx = ceil_div(in.W + 1, 32) * (in.H + 1);
         b.tiles_bwd = fp_tiles_per_view(in.U, in.V, b.tile_bwd);
-        host[i] = b;
         item_fwd[i + 1] = item_fwd[i] + fp_tiles_per_view(in.U, in.V, b.tile_fwd) * in.A;
         item_bwd[i + 1] = item_bwd[i] + b.tiles_bwd * in.A;
         quad_block[i + 1] = quad_block[i] + (long long)b.quad_gx * ceil_div(in.D + 2, 32);
         view[i + 1] = view[i] + in.A;
-        const long long voxels = (long long)in.D * in.H * in.W;
-        fold_block[i + 1] = fold_block[i] + (in.grad_volume ? (voxels + kFoldChunk - 1) / kFoldChunk : 0);
+        b.fold_gx = ceil_div(in.W, 32) * in.H;
+        fold_block[i + 1] =
+            fold_block[i] + (in.grad_volume ? (long long)b.fold_gx * ceil_div(in.D, 32) : 0);
+        host[i] = b;
         rays += (long long)in.A * in.U * in.V;
         if (!in.grad_projections || !in.grad_geometry) backward_ready = 0;
     }

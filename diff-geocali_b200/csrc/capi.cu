@@ -48,10 +48,8 @@ size_t quad_volume_bytes(int D, int H, int W) {
     return Workspace::align(sizeof(float4) * (size_t)(D + 2) * (size_t)(H + 1) * (size_t)(W + 1));
 }
 
-// volume-gradient buffer (level records)
-size_t gradient_buffer_bytes(int D, int H, int W) {
-    return Workspace::align(sizeof(float) * fp_record_buffer_floats(D, H, W));
-}
+// volume-gradient buffer: the edge records (fp_edge_bytes) take about half of it
+size_t gradient_buffer_bytes(int D, int H, int W) { return quad_volume_bytes(D, H, W); }
 
 // Ray tile of the forward projector (8 detector columns x 32 rows per CTA):
 // the batched launches take per-instance tiles from the autotuner.
@@ -271,10 +269,11 @@ int dgc_project_backward(const float* grad_projection, const float* volume, int 
     const long long tiles = fp_tiles_per_view(U, V, kBackwardTile.tu);
     Workspace ws(workspace, workspace_bytes);
     float4* quads = ws.take<float4>((size_t)(D + 2) * (H + 1) * (W + 1));
-    const size_t gfloats = fp_record_buffer_floats(D, H, W);
-    float* gpad = compute_grad_volume ? ws.take<float>(gfloats) : nullptr;
+    float2* edges = compute_grad_volume ? reinterpret_cast<float2*>(ws.take<char>(
+                                              gradient_buffer_bytes(D, H, W)))
+                                        : nullptr;
     double* partials = ws.take<double>((size_t)8 * A * tiles);
-    if (!quads || !partials || (compute_grad_volume && !gpad)) {
+    if (!quads || !partials || (compute_grad_volume && !edges)) {
         set_error("workspace too small: dgc_project_backward needs " +
                   std::to_string(dgc_project_backward_workspace_bytes(D, H, W, A, U, V,
                                                                       compute_grad_volume)) +
@@ -283,17 +282,66 @@ int dgc_project_backward(const float* grad_projection, const float* volume, int 
     }
     p.quads = quads;
     p.grad_projections = grad_projection;
-    p.grad_pad = gpad;
+    p.grad_edges = edges;
     p.partials = partials;
     rc = build_volume_quads(volume, D, H, W, quads, s);
     if (rc != DGC_OK) return rc;
-    if (gpad) DGC_CUDA(cudaMemsetAsync(gpad, 0, sizeof(float) * gfloats, s));
+    if (edges) DGC_CUDA(cudaMemsetAsync(edges, 0, fp_edge_bytes(p), s));
     rc = fp_launch_backward(p, kBackwardTile, compute_grad_volume != 0, s);
     if (rc != DGC_OK) return rc;
     rc = fp_reduce_partials(partials, A, tiles, out, s);
     if (rc != DGC_OK) return rc;
-    if (gpad) return fp_fold_records(gpad, D, H, W, grad_volume, s);
+    if (edges) return fp_fold_edges(p, grad_volume, s);
     return DGC_OK;
+}
+
+// ------------------------------------------------- volume gradient alone
+
+size_t dgc_project_adjoint_workspace_bytes(int D, int H, int W) {
+    if (D <= 0 || H <= 0 || W <= 0) return 0;
+    return gradient_buffer_bytes(D, H, W);
+}
+
+int dgc_project_adjoint(const float* grad_projection, int D, int H, int W, const float* angles,
+                        const float* sid, const float* sod, const float* det_u0,
+                        const float* det_v0, const float* src_x, const float* src_y,
+                        const float* src_z, int A, float pixel_size, int U, int V,
+                        float step_size, float voxel_size, float off_x, float off_y, float off_z,
+                        float* grad_volume, void* workspace, size_t workspace_bytes,
+                        void* stream) {
+    clear_error();
+    cudaStream_t s = (cudaStream_t)stream;
+    const Geometry g = make_geometry(angles, sid, sod, det_u0, det_v0, src_x, src_y, src_z);
+    int rc = check_fp_common(D, H, W, A, U, V, pixel_size, step_size, voxel_size, g);
+    if (rc != DGC_OK) return rc;
+    DGC_REQUIRE(grad_projection && grad_volume, "grad_projection and grad_volume must be non-null");
+    FpArgs p;
+    memset(&p, 0, sizeof(p));
+    p.g = g;
+    p.D = D;
+    p.H = H;
+    p.W = W;
+    p.A = A;
+    p.U = U;
+    p.V = V;
+    p.pixel_size = pixel_size;
+    p.step_size = step_size;
+    p.voxel_size = voxel_size;
+    p.off_x = off_x;
+    p.off_y = off_y;
+    p.off_z = off_z;
+    fp_fill_layout(p);
+    Workspace ws(workspace, workspace_bytes);
+    p.grad_projections = grad_projection;
+    p.grad_edges = reinterpret_cast<float2*>(ws.take<char>(gradient_buffer_bytes(D, H, W)));
+    if (!p.grad_edges) {
+        set_error("workspace too small: dgc_project_adjoint needs " +
+                  std::to_string(dgc_project_adjoint_workspace_bytes(D, H, W)) + " bytes");
+        return DGC_ERR_WORKSPACE;
+    }
+    DGC_CUDA(cudaMemsetAsync(p.grad_edges, 0, fp_edge_bytes(p), s));
+    if ((rc = fp_launch_adjoint(p, s)) != DGC_OK) return rc;
+    return fp_fold_edges(p, grad_volume, s);
 }
 
 // ------------------------------------------- fused calibration loss + grads

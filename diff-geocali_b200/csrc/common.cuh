@@ -190,22 +190,12 @@ __device__ __forceinline__ void red_add_global(float* p, float v) {
     asm volatile("red.global.add.f32 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "f"(v));
 }
 
-// Four float adds to 16-byte-aligned global memory as one vector reduction
-// (red.global.add.v4.f32; each element is added atomically), without a
+// Two float adds to 8-byte-aligned global memory as one vector reduction
+// (red.global.add.v2.f32; each element is added atomically), without a
 // memory clobber like red_add_global.
-__device__ __forceinline__ void red_add4_global(float* p, float a, float b, float c, float d) {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(__cvta_generic_to_global(p)),
-                 "f"(a), "f"(b), "f"(c), "f"(d));
-}
-
-// red_add4_global under a predicate inside the asm (a predicated
-// instruction, not a branch around it).
-__device__ __forceinline__ void red_add4_global_if(bool on, float* p, float a, float b, float c,
-                                                   float d) {
-    asm volatile(
-        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-        "@q red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n\t}"
-        ::"l"(__cvta_generic_to_global(p)), "f"(a), "f"(b), "f"(c), "f"(d), "r"((int)on));
+__device__ __forceinline__ void red_add2_global(float* p, float a, float b) {
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(__cvta_generic_to_global(p)), "f"(a),
+                 "f"(b));
 }
 
 __device__ __forceinline__ double warp_sum(double v) {

@@ -30,10 +30,10 @@
 //   * Geometry gradients are reduced per CTA in FP64 with warp shuffles and a
 //     fixed-order tree, then per view over CTAs in a second fixed-order pass:
 //     the eight per-view gradients are bitwise reproducible.
-//   * The volume gradient is scattered into an edge-padded z-fastest buffer
-//     (consecutive lanes hit consecutive addresses) and folded back onto the
-//     clamped edge voxels afterwards (the sums of the reference's clamped-index
-//     atomics).
+//   * The volume gradient is gathered per ray in registers, emitted at cell
+//     crossings into z-fastest edge records (consecutive lanes hit consecutive
+//     addresses) and folded onto the clamped voxels afterwards (the sums of the
+//     reference's clamped-index atomics).
 #include <cstdlib>
 #include <mutex>
 #include <climits>
@@ -916,13 +916,105 @@ __device__ __forceinline__ QuadGradient quad_gradient(const ulonglong2& q0, cons
     return g;
 }
 
-// GRADVOL: also scatter the adjoint of every sample into p.grad_pad, a
-// cell-major buffer of 16-byte level records R[(cy*(W+1) + cx)*(D+2) + cz]
-// (cells at padded index floor+1): record c holds the weights of the four
-// corners (cz, cy+dy, cx+dx) of its z level at dy*2 + dx, so a sample adds
-// its z level to its cell's record and its z+1 level to the next record;
-// fold_record_gradient_kernel then sums the records onto the voxels.  A
-// lane's consecutive samples of one cell are first added in registers.
+// Volume gradient: the adjoint of a ray's samples, gathered in registers.
+//
+// The gradient is accumulated in vertical edge records E[cy][cx][cz] = (weight
+// of the padded voxel (cz, cy, cx), weight of the one above it), 8 bytes, z
+// fastest (fold_edges_tile folds them onto the voxels).  A cell has four edges;
+// a ray adds its samples' weights to its cell's four edges in registers and,
+// when it moves to the next cell across a vertical face, emits only the two
+// edges it leaves behind and carries the two of the shared face along.  Seen
+// along the ray, "behind" and "ahead" are fixed per axis by the sign of its
+// direction, so an x crossing always leaves the edges behind in x, a y
+// crossing those behind in y.  A move in z (rare: the rays are nearly
+// horizontal) or of more than a cell emits all four.
+//
+// Why: reductions cost by the element, not by the instruction (1.2-1.45e12 float
+// additions/s in L2 on a B200 whatever the vector width), and a crossing emits
+// 4 elements instead of the 8 of both z levels of all four columns (16-byte
+// level records, which the reductions bound: 1.36e11 additions a call at 256^3 /
+// 360 x 384^2).  What binds now is issue, 117 instructions a sample with the
+// gradient sums and 72 without, at 77 % of the slots, beside L2 additions at 60
+// % in the march without the sums.  Level records -> edges, all nine gradients:
+// 103.1 -> 101.2 ms (256^3 / 360 x 384^2), 280 -> 266 ms (512^3 / 96 x 768^2).
+// Emitting through a branch per edge with the columns recomputed took 153.7 ms.
+struct EdgeRun {
+    uint32_t eb;  // record index of the pending cell's edge behind in x and y
+    f32x2 bb = 0, ba = 0, ab = 0, aa = 0;  // (x, y) behind / ahead: z and z+1 weights
+};
+
+// Per ray: one cell ahead in x, in y and in both as record-index steps, and the
+// bias that turns biased floors into the index of the edge behind.  An axis one
+// voxel thick has stride 0 (all its padded voxels are the one voxel), so its
+// crossings change no index and its edges coincide.
+struct EdgeSteps {
+    uint32_t dx, dy, bias;
+    bool fx, fy;  // direction >= 0 along x, y
+};
+
+__device__ __forceinline__ EdgeSteps edge_steps(const RaySetup& r, const FpArgs& p) {
+    EdgeSteps e;
+    e.fx = r.dx >= 0.0f;
+    e.fy = r.dy >= 0.0f;
+    e.dx = e.fx ? p.ge_x : 0u - p.ge_x;
+    e.dy = e.fy ? p.ge_y : 0u - p.ge_y;
+    e.bias = (1u - kFloorMagicBits) * (1u + p.ge_x + p.ge_y) + (e.fx ? 0u : p.ge_x) +
+             (e.fy ? 0u : p.ge_y);
+    return e;
+}
+
+__device__ __forceinline__ uint32_t edge_index(const Cell& c, const FpArgs& p, const EdgeSteps& s) {
+    return c.bz + c.bx * p.ge_x + c.by * p.ge_y + s.bias;
+}
+
+__device__ __forceinline__ void emit_edge(bool on, const FpArgs& p, uint32_t index, f32x2 w) {
+    const float2 v = unpack2(w);
+    float* e = reinterpret_cast<float*>(p.grad_edges + index);
+    if (on) red_add2_global(e, v.x, v.y);
+}
+
+// The ray enters the cell with record index eb: emit the edges that its pending
+// cell does not share with it, carry the shared ones over.  The index difference
+// tells the kind of move: |dz| < ge_x and |dx * ge_x + dz| < ge_y for any two
+// cells, so no other move has the difference of a single step.
+__device__ __forceinline__ void enter_cell(EdgeRun& run, const FpArgs& p, const EdgeSteps& s,
+                                           uint32_t eb) {
+    const uint32_t d = eb - run.eb;
+    const bool mx = d == s.dx, my = d == s.dy, mxy = d == s.dx + s.dy;
+    emit_edge(true, p, run.eb, run.bb);
+    emit_edge(!my, p, run.eb + s.dy, run.ba);
+    emit_edge(!mx, p, run.eb + s.dx, run.ab);
+    emit_edge(!(mx || my || mxy), p, run.eb + s.dx + s.dy, run.aa);
+    run.bb = mx ? run.ab : my ? run.ba : mxy ? run.aa : 0ull;
+    run.ba = mx ? run.aa : 0ull;
+    run.ab = my ? run.aa : 0ull;
+    run.aa = 0ull;
+    run.eb = eb;
+}
+
+__device__ __forceinline__ void flush_edges(const EdgeRun& run, const FpArgs& p,
+                                            const EdgeSteps& s) {
+    emit_edge(true, p, run.eb, run.bb);
+    emit_edge(true, p, run.eb + s.dy, run.ba);
+    emit_edge(true, p, run.eb + s.dx, run.ab);
+    emit_edge(true, p, run.eb + s.dx + s.dy, run.aa);
+}
+
+// One sample's adjoint weights (fp.cu:231-240), times gs, added to the pending cell.
+__device__ __forceinline__ void add_sample(EdgeRun& run, const Cell& c, const EdgeSteps& s,
+                                           float gs) {
+    const float mx = 1.0f - c.fx, my = 1.0f - c.fy;
+    const float xb = s.fx ? mx : c.fx, xa = s.fx ? c.fx : mx;
+    const float yb = gs * (s.fy ? my : c.fy), ya = gs * (s.fy ? c.fy : my);
+    const f32x2 z = pack2(1.0f - c.fz, c.fz);
+    const float bb = xb * yb, ba = xb * ya, ab = xa * yb, aa = xa * ya;
+    run.bb = fma2(pack2(bb, bb), z, run.bb);
+    run.ba = fma2(pack2(ba, ba), z, run.ba);
+    run.ab = fma2(pack2(ab, ab), z, run.ab);
+    run.aa = fma2(pack2(aa, aa), z, run.aa);
+}
+
+// Spatial-gradient sums of a ray; GRADVOL: also its adjoint into p.grad_edges.
 template <bool CLAMP, bool GRADVOL, bool POW2, bool OFF, bool GUARD>
 __device__ __forceinline__ RayGrad march_grad(const RaySetup& r, const ViewGeo& vg,
                                               const FpArgs& p, float gs) {
@@ -930,12 +1022,10 @@ __device__ __forceinline__ RayGrad march_grad(const RaySetup& r, const ViewGeo& 
     const XYPacks k = make_xy_packs(r, vg, p);
     RayGrad rg{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     const int nmax = step_bound(r, p.step_size);
-    // this lane's pending level records (cell run_ci: its z level and z+1
-    // level), flushed when the ray leaves the cell
-    const f32x2 zero = pack2(0.0f, 0.0f);
-    uint32_t run_ci = 0u;
-    bool run_have = false;
-    f32x2 run_lo[2] = {zero, zero}, run_hi[2] = {zero, zero};
+    const EdgeSteps es = edge_steps(r, p);
+    EdgeRun run;
+    if (GRADVOL)
+        run.eb = edge_index(sample_cell<CLAMP, false, OFF, POW2>(r.tmin, r, vg, p, k), p, es);
     float t = r.tmin;
     int n = 0;
 #pragma unroll 1
@@ -953,52 +1043,120 @@ __device__ __forceinline__ RayGrad march_grad(const RaySetup& r, const ViewGeo& 
         rg.s2y = fmaf(g.y, tau, rg.s2y);
         rg.s2z = fmaf(g.z, tau, rg.s2z);
         if (GRADVOL) {
-            // adjoint of the trilinear sample (fp.cu:231-240) into the level records
-            const float mx = 1.0f - c.fx, my = 1.0f - c.fy, mz = 1.0f - c.fz;
-            const float gy0 = gs * my, gy1 = gs * c.fy;
-            // (x, y) corner columns 00, 10, 01, 11 at the cell's z (lo) and z+1
-            // (hi) as packed pairs: w0 = (w00, w01), w1 = (w10, w11), the
-            // products lane by lane those of the scalar form
-            const f32x2 wxs = pack2(mx, c.fx);
-            const f32x2 w0 = mul2(pack2(gy0, gy0), wxs), w1 = mul2(pack2(gy1, gy1), wxs);
-            const f32x2 zl = pack2(mz, mz), zh = pack2(c.fz, c.fz);
-            f32x2 lo2[2] = {mul2(w0, zl), mul2(w1, zl)};
-            f32x2 hi2[2] = {mul2(w0, zh), mul2(w1, zh)};
-            const uint32_t gi = c.bz + c.bx * p.gz_x + c.by * p.gz_y + p.gz_bias;
-            {
-                // Consecutive samples of the ray mostly share a cell: add them
-                // in registers and emit a cell's two level records when the
-                // ray moves on.  A move to the cell above (below) in z shares a
-                // level, which stays pending.  Branch-free: predicated
-                // reductions of the pending records, then selects.
-                const int d = (int)(gi - run_ci);
-                const bool same = run_have && d == 0, up = run_have && d == 1,
-                           down = run_have && d == -1;
-                float* o = p.grad_pad + 4ull * run_ci;
-                const float2 a0 = unpack2(run_lo[0]), a1 = unpack2(run_lo[1]);
-                const float2 b0 = unpack2(run_hi[0]), b1 = unpack2(run_hi[1]);
-                red_add4_global_if(run_have && !same && !down, o, a0.x, a0.y, a1.x, a1.y);
-                red_add4_global_if(run_have && !same && !up, o + 4, b0.x, b0.y, b1.x, b1.y);
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    const f32x2 base_lo = same ? run_lo[j] : up ? run_hi[j] : zero;
-                    const f32x2 base_hi = same ? run_hi[j] : down ? run_lo[j] : zero;
-                    run_lo[j] = add2(base_lo, lo2[j]);
-                    run_hi[j] = add2(base_hi, hi2[j]);
-                }
-                run_ci = gi;
-                run_have = true;
-            }
+            const uint32_t eb = edge_index(c, p, es);
+            if (eb != run.eb) enter_cell(run, p, es, eb);
+            add_sample(run, c, es, gs);
         }
     }
-    if (GRADVOL && run_have) {
-        float* o = p.grad_pad + 4ull * run_ci;
-        const float2 a0 = unpack2(run_lo[0]), a1 = unpack2(run_lo[1]);
-        const float2 b0 = unpack2(run_hi[0]), b1 = unpack2(run_hi[1]);
-        red_add4_global(o, a0.x, a0.y, a1.x, a1.y);
-        red_add4_global(o + 4, b0.x, b0.y, b1.x, b1.y);
-    }
+    if (GRADVOL) flush_edges(run, p, es);
     return rg;
+}
+
+// ---------------------------------------------------------------------------
+// Adjoint kernel: the volume gradient alone
+// ---------------------------------------------------------------------------
+
+// March of one ray for the volume gradient alone: no volume samples, only
+// weights.  109.2 -> 66.9 ms at 256^3 / 360 x 384^2, 10.1 -> 5.6 ms at 128^3 /
+// 180 x 256^2 and 287 -> 185 ms at 512^3 / 96 x 768^2 against the march with the
+// gradient sums and level records (the volume's quads are not built either).
+// Per sample and SM it takes 23.4 cycles against about 20 for its 3.1 additions a
+// lane and 18 for its 72 instructions; view blocks change nothing (186 ms).  x and y run mirrored (negated) where the ray travels towards lower
+// indices, so that "behind" is the floor along every ray and neither weights nor
+// indices need a selection by direction; the negated multiply-adds round as the
+// original ones.  At a coordinate exactly on a voxel the mirrored cell is the
+// one on its other side, with the same weights.
+template <bool CLAMP, bool POW2, bool OFF, bool GUARD>
+__device__ __forceinline__ void march_adjoint(const RaySetup& r, const ViewGeo& vg,
+                                              const FpArgs& p, float gs) {
+    const float sx = r.dx >= 0.0f ? 1.0f : -1.0f, sy = r.dy >= 0.0f ? 1.0f : -1.0f;
+    const float k = POW2 ? p.inv_voxel : 1.0f;  // scaled beforehand where that is exact
+    const f32x2 dxy = pack2(sx * r.dx * k, sy * r.dy * k);
+    const f32x2 oxy = pack2(sx * vg.ox * k, sy * vg.oy * k);
+    const f32x2 offxy = pack2(sx * p.off_x * k, sy * p.off_y * k);
+    const f32x2 hxy = pack2(sx * p.W * 0.5f, sy * p.H * 0.5f);
+    const f32x2 inv2 = pack2(p.inv_voxel, p.inv_voxel);
+    const f32x2 magic2 = pack2(kFloorMagic, kFloorMagic);
+    const f32x2 one2 = pack2(1.0f, 1.0f);
+    const float dz = r.dz * k, oz = vg.oz * k, offz = p.off_z * k, hz = p.D * 0.5f;
+    // a mirrored coordinate is clamped below 1, so that its cell stays inside
+    // the pad (the weight that this moves folds onto the same voxel)
+    const float xlo = sx > 0.0f ? -1.0f : 1.0f - p.W, xhi = sx > 0.0f ? p.W - 1.0f : 0.99999994f;
+    const float ylo = sy > 0.0f ? -1.0f : 1.0f - p.H, yhi = sy > 0.0f ? p.H - 1.0f : 0.99999994f;
+    EdgeSteps es;
+    es.dx = sx > 0.0f ? p.ge_x : 0u - p.ge_x;
+    es.dy = sy > 0.0f ? p.ge_y : 0u - p.ge_y;
+    es.bias = 1u + p.ge_x + p.ge_y - kFloorMagicBits * (1u + es.dx + es.dy);
+
+    struct Place {
+        f32x2 ahead;
+        float fz;
+        uint32_t eb;
+    };
+    auto place = [&](float t) {
+        f32x2 pxy = fma2(pack2(t, t), dxy, oxy);
+        if (OFF) pxy = sub2(pxy, offxy);
+        f32x2 vxy = POW2 ? add2(pxy, hxy) : fma2(pxy, inv2, hxy);
+        float vz = fmaf(t, dz, oz);
+        if (OFF) vz -= offz;
+        vz = POW2 ? vz + hz : fmaf(vz, p.inv_voxel, hz);
+        if (CLAMP) {
+            const float2 v = unpack2(vxy);
+            vxy = pack2(fminf(fmaxf(v.x, xlo), xhi), fminf(fmaxf(v.y, ylo), yhi));
+            vz = fminf(fmaxf(vz, -1.0f), (float)(p.D - 1));
+        }
+        const f32x2 fxy = add2_rd(vxy, magic2);
+        const FloorSplit z = floor_split(vz);
+        const uint2 b = unpack2_bits(fxy);
+        return Place{sub2(vxy, sub2(fxy, magic2)), z.frac,
+                     z.biased + b.x * es.dx + b.y * es.dy + es.bias};
+    };
+
+    EdgeRun run;
+    run.eb = place(r.tmin).eb;
+    const int nmax = step_bound(r, p.step_size);
+    float t = r.tmin;
+    int n = 0;
+#pragma unroll 1
+    for (; t <= r.tmax && (!GUARD || n < nmax); t += p.step_size, n += GUARD ? 1 : 0) {
+        const Place c = place(t);
+        if (c.eb != run.eb) enter_cell(run, p, es, c.eb);
+        const float2 wa = unpack2(c.ahead), wb = unpack2(sub2(one2, c.ahead));
+        const float yb = gs * wb.y, ya = gs * wa.y;
+        const f32x2 zz = pack2(1.0f - c.fz, c.fz);
+        const float bb = wb.x * yb, ba = wb.x * ya, ab = wa.x * yb, aa = wa.x * ya;
+        run.bb = fma2(pack2(bb, bb), zz, run.bb);
+        run.ba = fma2(pack2(ba, ba), zz, run.ba);
+        run.ab = fma2(pack2(ab, ab), zz, run.ab);
+        run.aa = fma2(pack2(aa, aa), zz, run.aa);
+    }
+    flush_edges(run, p, es);
+}
+
+template <int TU, bool POW2, bool OFF>
+__global__ void __launch_bounds__(256) fp_adjoint_kernel(FpArgs p) {
+    __shared__ ViewGeo s_view;
+    const TileCoord tc = tile_coord(p, (p.U + TU - 1) / TU);
+    if (threadIdx.x == 0) load_view(p.g, tc.a, s_view);
+    __syncthreads();
+    const ViewGeo vg = s_view;
+    int u, v;
+    tile_ray<TU>(tc, u, v);
+    if (u >= p.U || v >= p.V) return;
+    const float grad_out = p.grad_projections[((long long)tc.a * p.U + u) * p.V + v];
+    // fp.cu:381 -- rays with a zero upstream gradient contribute nothing.
+    if (grad_out == 0.0f) return;
+    const RaySetup r = setup_ray(vg, u, v, p);
+    if (!(r.ok && r.hit)) return;
+    const float gs = grad_out * p.step_size;
+    const bool inside = ray_inside_pad<false>(r, vg, p);
+    if (steps_advance(r, p.step_size)) {
+        if (inside) march_adjoint<false, POW2, OFF, false>(r, vg, p, gs);
+        else march_adjoint<true, POW2, OFF, false>(r, vg, p, gs);
+    } else {
+        if (inside) march_adjoint<false, POW2, OFF, true>(r, vg, p, gs);
+        else march_adjoint<true, POW2, OFF, true>(r, vg, p, gs);
+    }
 }
 
 // The eight per-view geometry terms of a ray that hits the volume, from its
@@ -1046,7 +1204,7 @@ __device__ __forceinline__ void ray_geometry_terms(const FpArgs& p, const ViewGe
 
 // The eight per-view geometry terms of one ray (zero for rays outside the
 // detector, missing the volume or with a zero upstream gradient); with
-// GRADVOL (march_grad) the ray's adjoint samples go into p.grad_pad.
+// GRADVOL (march_grad) the ray's adjoint samples go into p.grad_edges.
 template <bool GRADVOL, bool POW2, bool OFF>
 __device__ __forceinline__ void backward_ray(const FpArgs& p, const ViewGeo& vg, int a, int u,
                                              int v, float (&terms)[8]) {
@@ -1241,49 +1399,52 @@ __global__ void __launch_bounds__(256) reduce_view_partials_kernel(const double*
     if (lane == 0) out.g[k][a] = (float)acc;
 }
 
-// Volume gradient from the level records R[((cy*(W+1) + cx)*(D+2) + cz)*4 + k]
-// (march_grad; cells at padded index floor+1 in [0, n]): a padded corner P
-// gets entry k = dy*2 + dx of record P - (0, dy, dx) for every record in range,
-// and padded corners fold onto the clamped voxels (index 0 onto 0, n+1 onto
-// n-1, as the clamped neighbours of fp.cu:200-213 sample them).
-__device__ __forceinline__ float fold_record_voxel(const float* __restrict__ O, int D, int H, int W,
-                                                   long long i) {
-    const long long CZ = D + 2, CX = W + 1;
-    const int x = (int)(i % W);
-    const long long r = i / W;
-    const int y = (int)(r % H);
-    const int z = (int)(r / H);
-    int xs[3], ys[3], zs[3];
-    int nx = 0, ny = 0, nz = 0;
-    xs[nx++] = x + 1;
-    if (x == 0) xs[nx++] = 0;
-    if (x == W - 1) xs[nx++] = W + 1;
-    ys[ny++] = y + 1;
-    if (y == 0) ys[ny++] = 0;
-    if (y == H - 1) ys[ny++] = H + 1;
-    zs[nz++] = z + 1;
-    if (z == 0) zs[nz++] = 0;
-    if (z == D - 1) zs[nz++] = D + 1;
-    float acc = 0.0f;
-    for (int iy = 0; iy < ny; ++iy)
-        for (int ix = 0; ix < nx; ++ix)
-            for (int iz = 0; iz < nz; ++iz)
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int dy = k >> 1, dx = k & 1;
-                    const int cz = zs[iz], cy = ys[iy] - dy, cx = xs[ix] - dx;
-                    if (cy < 0 || cy > H || cx < 0 || cx > W) continue;
-                    acc += O[((cy * CX + cx) * CZ + cz) * 4 + k];
-                }
+// Volume gradient from the edge records: a padded voxel (zp, yp, xp) is the low
+// end of edge zp and the high end of edge zp - 1 of its column, and padded
+// border voxels fold onto the clamped ones (0 onto voxel 0, n+1 onto n-1, as the
+// clamped neighbours of fp.cu:200-213 sample them; along an axis one voxel thick
+// all three are one column already).
+__device__ __forceinline__ float fold_column(const float2* __restrict__ e, int D, int z) {
+    // zp = z + 1: records z and z + 1 of the column (z + 1 <= D always holds one)
+    float acc = e[z + 1].x + e[z].y;
+    if (z == 0) acc += e[0].x;
+    if (z == D - 1) acc += e[D].y;
     return acc;
 }
 
-__global__ void fold_record_gradient_kernel(const float* __restrict__ O, int D, int H, int W,
-                                            float* __restrict__ grad) {
-    const long long total = (long long)D * H * W;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x)
-        grad[i] = fold_record_voxel(O, D, H, W, i);
+// One 32 x 32 (x, z) tile of the folded gradient at row y: block (32, 8).  Reads
+// run along z and writes along x, through shared memory.
+__device__ __forceinline__ void fold_edges_tile(const FpArgs& p, float* __restrict__ grad, int bx,
+                                                int by, float (&tile)[32][33]) {
+    const int xtiles = (p.W + 31) / 32;
+    const int y = bx / xtiles;
+    const int x0 = (bx - y * xtiles) * 32, z0 = by * 32;
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    for (int xl = ty; xl < 32; xl += 8) {
+        const int x = x0 + xl, z = z0 + tx;
+        float acc = 0.0f;
+        if (x < p.W && z < p.D) {
+            const float2* e = p.grad_edges + (size_t)(y + 1) * p.ge_y + (size_t)(x + 1) * p.ge_x;
+            const int xlo = p.ge_x && x == 0 ? -1 : 0, xhi = p.ge_x && x == p.W - 1 ? 1 : 0;
+            const int ylo = p.ge_y && y == 0 ? -1 : 0, yhi = p.ge_y && y == p.H - 1 ? 1 : 0;
+            for (int dy = ylo; dy <= yhi; ++dy)
+                for (int dx = xlo; dx <= xhi; ++dx)
+                    acc += fold_column(e + dy * (long long)p.ge_y + dx * (long long)p.ge_x, p.D, z);
+        }
+        tile[xl][tx] = acc;
+    }
+    __syncthreads();
+    for (int zl = ty; zl < 32; zl += 8) {
+        const int x = x0 + tx, z = z0 + zl;
+        if (x < p.W && z < p.D) grad[((long long)z * p.H + y) * p.W + x] = tile[tx][zl];
+    }
+}
+
+// grid: x = ceil(W/32) * H, y = ceil(D/32); block (32, 8).  Bound by memory: 12
+// bytes a voxel.
+__global__ void __launch_bounds__(256) fold_edges_kernel(FpArgs p, float* __restrict__ grad) {
+    __shared__ float tile[32][33];
+    fold_edges_tile(p, grad, blockIdx.x, blockIdx.y, tile);
 }
 
 // ---------------------------------------------------------------------------
@@ -1401,11 +1562,11 @@ __device__ __forceinline__ void backward_item(const FpArgs& p, const ViewGeo& vg
     tile_ray<TU>(tc, u, v);
     switch (flags & (kBatchDiv | kBatchOff)) {
         case 0:
-            if (p.grad_pad) backward_ray<true, true, false>(p, vg, tc.a, u, v, terms);
+            if (p.grad_edges) backward_ray<true, true, false>(p, vg, tc.a, u, v, terms);
             else backward_ray<false, true, false>(p, vg, tc.a, u, v, terms);
             break;
         default:
-            if (p.grad_pad) backward_ray<true, false, true>(p, vg, tc.a, u, v, terms);
+            if (p.grad_edges) backward_ray<true, false, true>(p, vg, tc.a, u, v, terms);
             else backward_ray<false, false, true>(p, vg, tc.a, u, v, terms);
             break;
     }
@@ -1446,15 +1607,13 @@ __global__ void __launch_bounds__(256) batch_reduce_kernel(BatchTables t) {
     if (lane == 0) in.gout.g[k][a] = (float)acc;
 }
 
-// kFoldChunk voxels of one instance per block.
+// One (x, z) tile of one instance's gradient per block (32, 8).
 __global__ void __launch_bounds__(256) batch_fold_kernel(BatchTables t) {
+    __shared__ float tile[32][33];
     const int i = find_instance(t.fold_block, t.n, blockIdx.x);
     const BatchInstance& in = t.inst[i];
-    const long long total = (long long)in.p.D * in.p.H * in.p.W;
-    const long long v0 = (blockIdx.x - t.fold_block[i]) * (long long)kFoldChunk;
-    const long long v1 = v0 + kFoldChunk < total ? v0 + kFoldChunk : total;
-    for (long long v = v0 + threadIdx.x; v < v1; v += blockDim.x)
-        in.grad_volume[v] = fold_record_voxel(in.p.grad_pad, in.p.D, in.p.H, in.p.W, v);
+    const long long b = blockIdx.x - t.fold_block[i];
+    fold_edges_tile(in.p, in.grad_volume, (int)(b % in.fold_gx), (int)(b / in.fold_gx), tile);
 }
 
 // ---------------------------------------------------------------------------
@@ -1498,16 +1657,15 @@ int launch_backward_tu(const FpArgs& p, bool gradvol, cudaStream_t s) {
 
 }  // namespace
 
-size_t fp_record_buffer_floats(int D, int H, int W) {
-    return 4 * (size_t)(D + 2) * (size_t)(H + 1) * (size_t)(W + 1);
+size_t fp_edge_bytes(const FpArgs& p) {
+    return sizeof(float2) * p.ge_count;
 }
 
-int fp_fold_records(const float* records, int D, int H, int W, float* grad, cudaStream_t s) {
-    DGC_TRACE("fold_record_gradient", s);
-    const long long total = (long long)D * H * W;
-    const int blocks = (int)std::min<long long>((total + 255) / 256, 148LL * 16);
-    fold_record_gradient_kernel<<<blocks, 256, 0, s>>>(records, D, H, W, grad);
-    DGC_LAUNCH_CHECK("fold_record_gradient");
+int fp_fold_edges(const FpArgs& p, float* grad, cudaStream_t s) {
+    DGC_TRACE("fold_edges", s);
+    const dim3 grid((unsigned)(ceil_div(p.W, 32) * (long long)p.H), (unsigned)ceil_div(p.D, 32));
+    fold_edges_kernel<<<grid, dim3(32, 8), 0, s>>>(p, grad);
+    DGC_LAUNCH_CHECK("fold_edges");
     return DGC_OK;
 }
 
@@ -1522,11 +1680,13 @@ void fp_fill_layout(FpArgs& p) {
     p.zq_x = (uint32_t)(p.D + 2);
     p.zq_y = (uint32_t)(p.W + 1) * (uint32_t)(p.D + 2);
     p.zq_bias = (1u + p.zq_x + p.zq_y) - kFloorMagicBits * (1u + p.zq_x + p.zq_y);
-    // level records of the volume gradient: record index of padded cell
-    // (floor+1) from the biased floors, R[(yp*(W+1) + xp)*(D+2) + zp]
-    p.gz_x = (uint32_t)(p.D + 2);
-    p.gz_y = (uint32_t)(p.W + 1) * (uint32_t)(p.D + 2);
-    p.gz_bias = (1u + p.gz_x + p.gz_y) - kFloorMagicBits * (1u + p.gz_x + p.gz_y);
+    // edge records of the volume gradient: D+1 per column (columns on 32-byte
+    // boundaries unless the volume is shallow), W+2 columns, H+2 rows; an axis one
+    // voxel thick has stride 0.  At most 2 records per padded quad for every size.
+    const uint32_t column = (uint32_t)(p.D >= 16 ? (p.D + 4) & ~3 : p.D + 1);
+    p.ge_x = p.W > 1 ? column : 0u;
+    p.ge_y = p.H > 1 ? column * (uint32_t)(p.W > 1 ? p.W + 2 : 1) : 0u;
+    p.ge_count = (size_t)column * (size_t)(p.W > 1 ? p.W + 2 : 1) * (size_t)(p.H > 1 ? p.H + 2 : 1);
     p.inv_voxel = 1.0f / p.voxel_size;
 }
 
@@ -1674,6 +1834,21 @@ int fp_launch_forward(const FpArgs& args, const FpTile& tile, const FpArm& a, cu
     }
 }
 
+int fp_launch_adjoint(const FpArgs& p, cudaStream_t s) {
+    DGC_TRACE("fp_adjoint_kernel", s);
+    const long long blocks = fp_tiles_per_view(p.U, p.V, 8) * (long long)p.A;
+    const bool off = p.off_x != 0.0f || p.off_y != 0.0f || p.off_z != 0.0f;
+    if (is_pow2_float(p.voxel_size)) {
+        if (off) fp_adjoint_kernel<8, true, true><<<(unsigned)blocks, 256, 0, s>>>(p);
+        else fp_adjoint_kernel<8, true, false><<<(unsigned)blocks, 256, 0, s>>>(p);
+    } else {
+        if (off) fp_adjoint_kernel<8, false, true><<<(unsigned)blocks, 256, 0, s>>>(p);
+        else fp_adjoint_kernel<8, false, false><<<(unsigned)blocks, 256, 0, s>>>(p);
+    }
+    DGC_LAUNCH_CHECK("fp_adjoint_kernel");
+    return DGC_OK;
+}
+
 int fp_launch_backward(const FpArgs& p, const FpTile& tile, bool gradvol, cudaStream_t s) {
     switch (tile.tu) {
         case 8: return launch_backward_tu<8>(p, gradvol, s);
@@ -1776,7 +1951,7 @@ int batch_launch_backward(const BatchTables& t, int grid, long long views, long 
     }
     if (fold_blocks > 0) {
         DGC_TRACE("batch_fold", s);
-        batch_fold_kernel<<<(unsigned)fold_blocks, 256, 0, s>>>(t);
+        batch_fold_kernel<<<(unsigned)fold_blocks, dim3(32, 8), 0, s>>>(t);
         DGC_LAUNCH_CHECK("batch_fold");
     }
     return DGC_OK;

@@ -17,8 +17,9 @@ struct FpArgs {
     float* projections;
     // backward
     const float* grad_projections;  // [A][U][V]
-    float* grad_pad;                // level records R[(yp*(W+1) + xp)*(D+2) + zp][4] or null
-    uint32_t gz_x, gz_y, gz_bias;
+    float2* grad_edges;             // edge records E[yp*ge_y + xp*ge_x + zp] or null
+    uint32_t ge_x, ge_y;
+    size_t ge_count;                // records in all
     double* partials;  // [A][tiles][8]
     int* error;        // device word set to 1 when a bounded wait gives up (TMA arm), or null
     int view_block;    // CTA order: 0 = u tile fastest; B > 0 = views in blocks of B (tile_coord),
@@ -34,7 +35,6 @@ struct FpTile {
 
 // One instance of a batched launch (an entry of the device-resident table).
 enum : int { kBatchDiv = 1, kBatchOff = 2 };
-constexpr int kFoldChunk = 2048;
 
 struct BatchInstance {
     FpArgs p;              // arguments with this instance's quads, outputs and workspace slices
@@ -45,6 +45,7 @@ struct BatchInstance {
     int flags;             // kBatchDiv (non power-of-two voxel) | kBatchOff (non-zero ROI
                            // offset)
     int quad_gx;           // blocks along x of the quads build
+    int fold_gx;           // blocks along x of the gradient fold
     long long tiles_bwd;   // backward tiles per view
 };
 
@@ -72,12 +73,12 @@ int fp_check_args(int D, int H, int W, int A, int U, int V, float pixel_size, fl
 
 void fp_fill_layout(FpArgs& p);
 long long fp_tiles_per_view(int U, int V, int tu);
-// Volume gradient of the backward: the weights of a lane's consecutive
-// samples in one cell are added in registers and emitted as 16-byte vector
-// reductions into a cell-major buffer of level records (4 floats per cell,
-// fp_record_buffer_floats), then folded onto the voxels (fp_fold_records).
-size_t fp_record_buffer_floats(int D, int H, int W);
-int fp_fold_records(const float* records, int D, int H, int W, float* grad, cudaStream_t s);
+// Volume gradient of the backward: the weights of a ray's samples are gathered
+// in registers and emitted as 8-byte reductions into edge records
+// (fp_edge_bytes, after fp_fill_layout; at most the 16 bytes per padded quad
+// that the workspace queries grant), then folded onto the voxels.
+size_t fp_edge_bytes(const FpArgs& p);
+int fp_fold_edges(const FpArgs& p, float* grad, cudaStream_t s);
 int build_volume_quads(const float* vol, int D, int H, int W, float4* quads, cudaStream_t s);
 // The forward's arm, slab, unroll and CTA order for a volume (the arm rules).
 struct FpArm {
@@ -95,6 +96,8 @@ int fp_add_arm_rule(long long voxels_max, int arm, int slab, int unroll, int vie
 void fp_clear_arm_rules();
 void fp_forward_arm(int D, int H, int W, int* arm, int* slab, int* unroll, int* view_block);
 FpArm fp_forward_arm(int D, int H, int W);
+// The volume gradient alone: into p.grad_edges (zeroed), no partials and no quads.
+int fp_launch_adjoint(const FpArgs& p, cudaStream_t s);
 int fp_launch_backward(const FpArgs& p, const FpTile& tile, bool gradvol, cudaStream_t s);
 int fp_launch_counts(const FpArgs& p, int64_t* counts, cudaStream_t s);
 // Fused projection -> masked squared error -> geometry-gradient terms (8-column

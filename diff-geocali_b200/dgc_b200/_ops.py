@@ -87,8 +87,10 @@ def fp_forward(volume, angles, sid, sod, det_u0_arr, det_v0_arr, src_x_arr, src_
 
 def fp_backward(grad_projection, volume, angles, sid, sod, det_u0_arr, det_v0_arr, src_x_arr,
                 src_y_arr, src_z_arr, pixel_size, step_size, voxel_size, compute_grad_volume=True,
-                off_x=0.0, off_y=0.0, off_z=0.0):
-    """Nine gradients (replaces ``src_cbct_forwardprojector_cuda.backward``)."""
+                off_x=0.0, off_y=0.0, off_z=0.0, compute_grad_geometry=True):
+    """Nine gradients (replaces ``src_cbct_forwardprojector_cuda.backward``);
+    with ``compute_grad_geometry=False`` the eight geometry gradients are
+    ``None`` and their march is skipped (the volume gradient alone)."""
     geometry = (angles, sid, sod, det_u0_arr, det_v0_arr, src_x_arr, src_y_arr, src_z_arr)
     pixel_size, step_size, voxel_size = float(pixel_size), float(step_size), float(voxel_size)
     _require(volume.dim() == 3, "volume must have shape [D,H,W]")
@@ -110,8 +112,16 @@ def fp_backward(grad_projection, volume, angles, sid, sod, det_u0_arr, det_v0_ar
     dev = vol.device
     compute = bool(compute_grad_volume)
     grad_volume = torch.zeros_like(vol) if compute else torch.empty(0, dtype=vol.dtype, device=dev)
-    grads = [torch.zeros_like(g) for g in geom]
     lib = _native.lib()
+    if compute and not compute_grad_geometry:
+        with torch.cuda.device(dev):
+            ws = _workspace(lib.dgc_project_adjoint_workspace_bytes(D, H, W), dev)
+            _native.check(lib.dgc_project_adjoint(
+                gp.data_ptr(), D, H, W, *[g.data_ptr() for g in geom], A, pixel_size, U, V,
+                step_size, voxel_size, float(off_x), float(off_y), float(off_z),
+                grad_volume.data_ptr(), _p(ws), 0 if ws is None else ws.numel(), _stream(dev)))
+        return [grad_volume, *[None] * 8]
+    grads = [torch.zeros_like(g) for g in geom]
     with torch.cuda.device(dev):
         ws = _workspace(lib.dgc_project_backward_workspace_bytes(D, H, W, A, U, V, int(compute)), dev)
         _native.check(lib.dgc_project_backward(

@@ -90,7 +90,7 @@ class DifferentiableSourceOnlyForwardProjector(Function):
         wanted = ctx.needs_input_grad[:9]
         grads = _ops.fp_backward(grad_projection.contiguous(), *ctx.saved_tensors,
                                  pixel_size, step_size, voxel_size, bool(wanted[0]),
-                                 off_x, off_y, off_z)
+                                 off_x, off_y, off_z, compute_grad_geometry=any(wanted[1:]))
         result = tuple(g if need else None for g, need in zip(grads, wanted)) + (None,) * 8
         return result[:ctx.num_inputs]
 

@@ -99,6 +99,22 @@ int dgc_project_backward(const float* grad_projection, const float* volume,
                          float* grad_src_x, float* grad_src_y, float* grad_src_z,
                          void* workspace, size_t workspace_bytes, void* stream);
 
+/* Scratch of dgc_project_adjoint. */
+size_t dgc_project_adjoint_workspace_bytes(int D, int H, int W);
+
+/* The volume gradient of dgc_project alone (dgc_project_backward without the
+ * geometry gradients, which an autograd call with fixed geometry drops): the
+ * volume itself is not read.  No counterpart in the reference, whose backward
+ * always computes the geometry gradients
+ * (csrc/src_cbct_forwardprojector_cuda.cu:634-729). */
+int dgc_project_adjoint(const float* grad_projection, int D, int H, int W,
+                        const float* angles, const float* sid, const float* sod,
+                        const float* det_u0, const float* det_v0,
+                        const float* src_x, const float* src_y, const float* src_z, int A,
+                        float pixel_size, int U, int V, float step_size, float voxel_size,
+                        float off_x, float off_y, float off_z, float* grad_volume,
+                        void* workspace, size_t workspace_bytes, void* stream);
+
 /* ---------------------------------------------------------------------- */
 /* Voxel-driven FDK-weighted backprojector                                  */
 /* ---------------------------------------------------------------------- */

@@ -24,6 +24,7 @@
 //     applies the (column, view) chain-rule coefficients once per warp; the
 //     eight per-view gradients are reduced in FP64 in a fixed order.
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "backprojector.cuh"
@@ -400,7 +401,8 @@ __device__ __forceinline__ float warp_transpose_sum(float (&v)[N], int lane) {
 constexpr int kBpGroup = 4;
 
 // GP: projection gradient 0 = not computed (p.grad_projections null), 1 = four
-// float reductions per voxel-view into grad_projections.
+// float reductions per voxel-view into grad_projections.  GEO: the geometry
+// gradients (without them the projections are not read).
 //
 // A warp owns one (x, y) column and 32*KZ of its voxels along z.  Views go in
 // passes of 32: lane j evaluates the column geometry of view a0+j (and, at
@@ -412,10 +414,10 @@ constexpr int kBpGroup = 4;
 // reduced over the warp at once (warp_transpose_sum) and kept by the lane
 // that owns the view; after the pass all 32 lanes apply the chain rule at
 // once.
-template <int KZ, int GP>
+template <int KZ, int GP, bool GEO>
 __global__ void __launch_bounds__(256) bp_backward_kernel(BpArgs p) {
     constexpr int G = kBpGroup;
-    __shared__ double s_terms[8][32][8];
+    __shared__ double s_terms[GEO ? 8 : 1][32][8];
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int cols_x = (p.W + 7) >> 3;
@@ -499,7 +501,7 @@ __global__ void __launch_bounds__(256) bp_backward_kernel(BpArgs p) {
                     vik[k] = okk[k] ? (int)vi : 0;
                     fvk[k] = fv;
                     dvk[k] = dv;
-                    q[k] = __ldg(rq + vik[k]);
+                    if (GEO) q[k] = __ldg(rq + vik[k]);
                 };
                 if constexpr (KZ % 2 == 0) {
                     const f32x2 t2 = pack2(t, t), d2 = pack2(dsv, dsv), o2 = pack2(v0, v0);
@@ -528,6 +530,8 @@ __global__ void __launch_bounds__(256) bp_backward_kernel(BpArgs p) {
                     if (okk[k]) {
                         const float fv = fvk[k], dv = dvk[k];
                         const int vi = vik[k];
+                        const float g = gval[k];
+                        if (GEO) {
                         // column pairs (rows u, u+1) at v and v+1: the lerp along v
                         // and the difference along v as packed pairs
                         const float2 e = unpack2(lerp2(q[k].x, q[k].y, pack2(fv, fv)));
@@ -536,11 +540,11 @@ __global__ void __launch_bounds__(256) bp_backward_kernel(BpArgs p) {
                         const float interp = lerpf(e.x, e.y, fu);
                         const float iu = lerpf(c0.y - c0.x, c1.y - c1.x, fv);
                         const float iv = lerpf(d.x, d.y, fu);
-                        const float g = gval[k];
                         acc[4 * i + 0] = fmaf(g, iu, acc[4 * i + 0]);
                         acc[4 * i + 1] = fmaf(g, iv, acc[4 * i + 1]);
                         acc[4 * i + 2] = fmaf(g * iv, dv, acc[4 * i + 2]);
                         acc[4 * i + 3] = fmaf(g, interp, acc[4 * i + 3]);
+                        }
                         if (GP) {
                             const float gb = g * w;
                             const float g0 = gb * (1.0f - fu), g1 = gb * fu;
@@ -552,6 +556,7 @@ __global__ void __launch_bounds__(256) bp_backward_kernel(BpArgs p) {
                     }
                 }
             }
+            if (!GEO) continue;
             // lane 4i+q: sum q of view b+i; the view's owner (lane b+i) keeps its four
             const float total = warp_transpose_sum<4 * G>(acc, lane);
             const int src = 4 * ((lane - b) & (G - 1));
@@ -566,6 +571,7 @@ __global__ void __launch_bounds__(256) bp_backward_kernel(BpArgs p) {
                 m_int = s_int;
             }
         }
+        if (!GEO) continue;
         float terms[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         if (my_ok) {
             const ColumnGrad g = column_grad(p.vt[a0 + lane], vx, vy, col_ok, p);
@@ -596,6 +602,324 @@ __global__ void __launch_bounds__(256) bp_reduce_partials_kernel(const double* _
     for (long long i = lane; i < nblocks; i += 32) acc += src[i];
     acc = warp_sum(acc);
     if (lane == 0) out.g[k][a] = (float)acc;
+}
+
+// ---------------------------------------------------------------------------
+// Projection gradient as a gather
+// ---------------------------------------------------------------------------
+//
+// grad P[a,u,v] = sum over columns (x, y) and z of g w hat(u - u_idx) hat(v - v_idx),
+// the adjoint of the bilinear taps.  Scattering it costs four float reductions
+// per voxel-view, which bound that kernel (1.0-1.4e12 additions/s in L2).  Here a
+// CTA takes a few detector bins b (u_idx in [b, b+1)) of one view and lists, bin
+// by bin, the columns that project into it: those between the rays of the bin's
+// two edges, found per row of the volume from the rays' equations with a margin
+// and then tested exactly, so that every column falls into the bin its own FP32
+// u_idx says.  A thread owns detector pixels v: per listed column it gathers the
+// two voxels whose v_idx can lie within a pixel of v (more where a voxel is
+// finer than a pixel), weights them by that v_idx, the backprojection's own, and
+// adds the sum to rows u = b and b + 1 in registers.  Only a CTA's first and last
+// row meet another CTA's: two additions onto zero, so the result does not
+// depend on scheduling.
+//
+// Bound by issue (73 % of the slots): 34 instructions a column and pixel, the
+// listing among them 2 %.
+
+// Upstream volume as z-fastest columns, zeros around them:
+// G[(y*W + x)*(D+3) + z + 1], z in [-1, D+1].
+// grid: x = ceil(W/32) * H, y = ceil((D+3)/32); block (32, 8)
+__global__ void __launch_bounds__(256) bp_columns_kernel(const float* __restrict__ g, int D, int H,
+                                                         int W, float* __restrict__ G) {
+    __shared__ float tile[32][33];
+    const int xtiles = (W + 31) / 32;
+    const int y = blockIdx.x / xtiles;
+    const int x0 = (blockIdx.x - y * xtiles) * 32, z0 = blockIdx.y * 32 - 1;
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    for (int zl = ty; zl < 32; zl += 8) {
+        const int z = z0 + zl, x = x0 + tx;
+        tile[zl][tx] = (z >= 0 && z < D && x < W) ? __ldg(g + ((long long)z * H + y) * W + x) : 0.0f;
+    }
+    __syncthreads();
+    for (int xl = ty; xl < 32; xl += 8) {
+        const int x = x0 + xl, zp = z0 + 1 + tx;
+        if (x < W && zp < D + 3) G[((long long)y * W + x) * (D + 3) + zp] = tile[tx][xl];
+    }
+}
+
+constexpr int kAdjMaxWarps = 8;
+constexpr int kAdjList = 96;  // columns that a warp lists between two passes over them
+
+struct AdjColumn {
+    float t, rt;   // magnification; d(z index)/d(v_phys - ds_v)
+    float wa, wb;  // FDK weight times the bilinear weights of rows b and b + 1
+};
+
+// Where the ray of detector coordinate q = u_phys - ds_u crosses the rows of a
+// volume axis, as a line over the row index: voxel coordinate e0 + e1*row, and
+// the source's distance along the view's normal there, d0 + d1*row.  along_y:
+// rows are y and the coordinate x, else the other way round.
+struct AdjLine {
+    float e0, e1, d0, d1;
+};
+
+__device__ __forceinline__ AdjLine adj_line(const ViewRow& r, float q, bool along_y, const BpArgs& p) {
+    const float sdn = r.sid + r.ds_n, m = r.sod + r.ds_n;
+    // w = alpha + beta*o solves u_phys = ds_u + sdn/denom*(px - ds_u) at row coordinate o
+    const float k = 1.0f / (along_y ? q * r.s - sdn * r.c : q * r.c + sdn * r.s);
+    const float alpha = (along_y ? -sdn * r.ds_u - q * m : q * m + sdn * r.ds_u) * k;
+    const float beta = (along_y ? sdn * r.s + q * r.c : q * r.s - sdn * r.c) * k;
+    const int rows = along_y ? p.H : p.W, cross = along_y ? p.W : p.H;
+    const float off_o = along_y ? p.off_y : p.off_x, off_i = along_y ? p.off_x : p.off_y;
+    const float o0 = off_o - rows * 0.5f * p.voxel_size;  // row 0
+    const float w0 = alpha + beta * o0;
+    AdjLine l;
+    l.e0 = (w0 - off_i) / p.voxel_size + cross * 0.5f;
+    l.e1 = beta;
+    l.d0 = along_y ? m + w0 * r.s - o0 * r.c : m + o0 * r.s - w0 * r.c;
+    l.d1 = (along_y ? beta * r.s - r.c : r.s - beta * r.c) * p.voxel_size;
+    return l;
+}
+
+// First and last detector row that the volume can reach, with a margin, from its
+// four corners' magnifications (all rows if a corner is not in front of the source).
+__device__ __forceinline__ float2 adj_reach(const ViewRow& r, const BpArgs& p) {
+    const float sdn = r.sid + r.ds_n, m = r.sod + r.ds_n;
+    float tlo = FLT_MAX, thi = -FLT_MAX;
+    bool front = true;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const float x = ((c & 1 ? p.W - 1 : 0) - p.W * 0.5f) * p.voxel_size + p.off_x;
+        const float y = ((c & 2 ? p.H - 1 : 0) - p.H * 0.5f) * p.voxel_size + p.off_y;
+        const float denom = m + x * r.s - y * r.c;
+        front = front && denom > 1e-3f * fabsf(r.sod);
+        tlo = fminf(tlo, sdn / denom);
+        thi = fmaxf(thi, sdn / denom);
+    }
+    const float za = -p.D * 0.5f * p.voxel_size + p.off_z - r.ds_v;
+    const float zb = za + (p.D - 1) * p.voxel_size;
+    const float lo = fminf(tlo * za, thi * za), hi = fmaxf(tlo * zb, thi * zb);
+    return front ? make_float2((r.ds_v + lo) * p.inv_pixel + r.v0 - 2.0f,
+                               (r.ds_v + hi) * p.inv_pixel + r.v0 + 2.0f)
+                 : make_float2(-FLT_MAX, FLT_MAX);
+}
+
+// Work item: `bins` bins of one view, one tile of V; NV pixels a thread, a warp's
+// 32*NV of them contiguous.  Dynamic shared memory: the warps' lists.
+template <int NV>
+__global__ void __launch_bounds__(32 * kAdjMaxWarps, NV < 3 ? 4 : 3)
+    bp_adjoint_kernel(BpArgs p, const float* __restrict__ G, int bins, int bin_blocks, int tiles) {
+    extern __shared__ AdjColumn s_col[];  // [warps][kAdjList]
+    __shared__ int s_count[kAdjMaxWarps];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int warps = blockDim.x >> 5;
+    unsigned* s_off = reinterpret_cast<unsigned*>(s_col + warps * kAdjList);
+    const int tile = blockIdx.x % tiles;
+    const int block = blockIdx.x / tiles;
+    const int a = block / bin_blocks;
+    const int b0 = (block - a * bin_blocks) * bins;
+    const int b1 = min(b0 + bins, p.U - 1);
+    const ViewRow r = p.vt[a];
+    const float vox = p.voxel_size;
+
+    // this thread's detector pixels and their heights above the source
+    float vf[NV], vp[NV], acc_a[NV], acc_b[NV];
+    // the bilinear weight of a voxel at distance d from a pixel, as min(1 + below*d,
+    // above0 - above*d) limited to [0, 1]: a tap exists for 0 <= v_idx < V-1 only, so
+    // pixel 0 has no voxels below it, pixel V-1 none at or above it and pixels past
+    // the detector none
+    float below[NV], above[NV], above0[NV];
+    const int v_first = (tile * warps + warp) * NV * 32 + lane;
+    bool inner = true;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int v = v_first + 32 * j;
+        vf[j] = (float)v;
+        vp[j] = (vf[j] - r.v0) * p.pixel_size - r.ds_v;
+        below[j] = v == 0 ? 1e30f : 1.0f;
+        above[j] = v == p.V - 1 ? 1e30f : v >= p.V ? 0.0f : 1.0f;
+        above0[j] = v >= p.V - 1 ? 0.0f : 1.0f;
+        inner = inner && v > 0 && v < p.V - 1;
+        acc_b[j] = 0.0f;
+    }
+    inner = __all_sync(0xffffffffu, inner);
+    const float2 reach_v = adj_reach(r, p);
+    // a warp whose pixels the volume cannot reach only lists
+    const bool reached = (float)(v_first - lane + 32 * NV) >= reach_v.x &&
+                         (float)(v_first - lane) <= reach_v.y;
+    const auto weight = [&](int j, float d) {
+        return fminf(__saturatef(fmaf(d, below[j], 1.0f)),
+                     __saturatef(fmaf(d, -above[j], above0[j])));
+    };
+    const float half_z = p.D * 0.5f;
+    const float zc = (r.ds_v - p.off_z) / vox + half_z;
+
+    // The listed columns' contributions to rows b (acc_a) and b + 1 (acc_b), where
+    // every voxel is at least a pixel high: the voxels within a pixel of v are
+    // z0, the floor of the pixel's own z, and z0 + 1.  EDGE: some pixel of the
+    // warp is at the detector's edge or past it.
+    const f32x2 vox2 = pack2(vox, vox), off2 = pack2(p.off_z, p.off_z);
+    const f32x2 dsv2 = pack2(r.ds_v, r.ds_v), ip2 = pack2(p.inv_pixel, p.inv_pixel);
+    const f32x2 v02 = pack2(r.v0, r.v0);
+    auto sum_list = [&](const AdjColumn* cols, const unsigned* offs, int count, auto edge) {
+        constexpr bool EDGE = decltype(edge)::value;
+        const unsigned top = (unsigned)p.D + 1u;
+#pragma unroll 2
+        for (int i = 0; i < count; ++i) {
+            const AdjColumn col = cols[i];
+            const float* __restrict__ g = G + offs[i] * (unsigned long long)(p.D + 3);
+            const f32x2 t2 = pack2(col.t, col.t);
+#pragma unroll
+            for (int j = 0; j < NV; ++j) {
+                const float f = __fadd_rd(fmaf(vp[j], col.rt, zc), kFloorMagic);
+                // pixels beyond the column (any bit pattern) read its zeros
+                const unsigned zi = min(__float_as_uint(f) - (kFloorMagicBits - 1u), top);
+                const float ga = __ldg(g + zi), gb = __ldg(g + zi + 1);
+                const float z0 = __fsub_rn(f, kFloorMagic) - half_z;
+                // v_idx of the two voxels, the backprojection's arithmetic
+                const f32x2 dv = sub2(fma2(pack2(z0, z0 + 1.0f), vox2, off2), dsv2);
+                const f32x2 vi = fma2(fma2(t2, dv, dsv2), ip2, v02);
+                const float2 d = unpack2(sub2(vi, pack2(vf[j], vf[j])));
+                const float ka = EDGE ? weight(j, d.x) : __saturatef(1.0f - fabsf(d.x));
+                const float kb = EDGE ? weight(j, d.y) : __saturatef(1.0f - fabsf(d.y));
+                const float h = fmaf(kb, gb, ka * ga);
+                acc_a[j] = fmaf(col.wa, h, acc_a[j]);
+                acc_b[j] = fmaf(col.wb, h, acc_b[j]);
+            }
+        }
+    };
+    // The same for any pixel and voxel size; a voxel out of reach contributes
+    // nothing even if it is not finite.
+    auto sum_list_general = [&](const AdjColumn* cols, const unsigned* offs, int count) {
+#pragma unroll 1
+        for (int i = 0; i < count; ++i) {
+            const AdjColumn col = cols[i];
+            const float* __restrict__ g = G + offs[i] * (unsigned long long)(p.D + 3) + 1;
+            const float reach = 1.0f / (col.t * (vox * p.inv_pixel)) + 1.0f;
+#pragma unroll
+            for (int j = 0; j < NV; ++j) {
+                const float zf = fmaf(vp[j], col.rt, zc);
+                const int z_lo = (int)fmaxf(ceilf(zf - reach), 0.0f);
+                const int z_hi = (int)fminf(floorf(zf + reach), (float)(p.D - 1));
+                float h = 0.0f;
+#pragma unroll 1
+                for (int z = z_lo; z <= z_hi; ++z) {
+                    const float dv = fmaf(z - half_z, vox, p.off_z) - r.ds_v;
+                    const float d = fmaf(fmaf(col.t, dv, r.ds_v), p.inv_pixel, r.v0) - vf[j];
+                    const float k = weight(j, d);
+                    if (k > 0.0f) h = fmaf(k, __ldg(g + z), h);
+                }
+                acc_a[j] = fmaf(col.wa, h, acc_a[j]);
+                acc_b[j] = fmaf(col.wb, h, acc_b[j]);
+            }
+        }
+    };
+
+    const float sdn = r.sid + r.ds_n;
+    const float front = 1e-3f * fabsf(r.sod);
+    const float rt_scale = 1.0f / (sdn * vox);
+    float* __restrict__ out = p.grad_projections + (long long)a * p.U * p.V;
+    for (int b = b0; b < b1; ++b) {
+        // row b starts with what the bin before it left
+        float from[NV];
+#pragma unroll
+        for (int j = 0; j < NV; ++j) from[j] = acc_b[j];
+        // rows of the volume along the axis that the bin's rays run along more
+        const float q0 = ((float)b - r.u0) * p.pixel_size - r.ds_u;
+        const float q1 = ((float)(b + 1) - r.u0) * p.pixel_size - r.ds_u;
+        const float qm = 0.5f * (q0 + q1);
+        const bool along_y = fabsf(qm * r.s - sdn * r.c) >= fabsf(qm * r.c + sdn * r.s);
+        const int n_rows = along_y ? p.H : p.W, n_cross = along_y ? p.W : p.H;
+        const AdjLine l0 = adj_line(r, q0, along_y, p), l1 = adj_line(r, q1, along_y, p);
+        const float margin = 0.02f + 1e-5f * n_cross;
+        // a second time, voxel by voxel, if a sum is not finite: the first lets
+        // a voxel that is not finite reach pixels whose weight for it is zero
+        for (int careful = 0;; ++careful) {
+#pragma unroll
+            for (int j = 0; j < NV; ++j) {
+                acc_a[j] = from[j];
+                acc_b[j] = 0.0f;
+            }
+            for (int row0 = 0; row0 < n_rows; row0 += blockDim.x) {
+                const int row = row0 + tid;
+                int i = 0, i_end = 0;
+                if (row < n_rows) {
+                    // both crossings in front of the source: the columns between
+                    // them; otherwise (or not finite) the whole row is tested
+                    i_end = n_cross;
+                    const float e0 = fmaf(l0.e1, (float)row, l0.e0);
+                    const float e1 = fmaf(l1.e1, (float)row, l1.e0);
+                    if (fmaf(l0.d1, (float)row, l0.d0) > front &&
+                        fmaf(l1.d1, (float)row, l1.d0) > front && fabsf(e0) < 1e9f &&
+                        fabsf(e1) < 1e9f) {
+                        i = (int)fmaxf(ceilf(fminf(e0, e1) - margin), 0.0f);
+                        i_end = (int)fminf(floorf(fmaxf(e0, e1) + margin) + 1.0f, (float)n_cross);
+                    }
+                }
+                // every warp lists its rows' columns in its own list, in order; all
+                // lists are summed when every warp is through or has a full one
+                bool more;
+                do {
+                    int count = 0;
+                    bool fine = false;  // a listed voxel is less than a pixel high
+                    while (count <= kAdjList - 32 && __any_sync(0xffffffffu, i < i_end)) {
+                        bool take = false;
+                        AdjColumn col;
+                        unsigned off = 0;
+                        if (i < i_end) {
+                            const int x = along_y ? i : row, y = along_y ? row : i;
+                            const float vx = (x - p.W * 0.5f) * vox + p.off_x;
+                            const float vy = (y - p.H * 0.5f) * vox + p.off_y;
+                            const ColumnGrad cg = column_grad(r, vx, vy, true, p);
+                            take = cg.ok && cg.ui == b;
+                            col.t = cg.t;
+                            col.rt = cg.denom * rt_scale;
+                            col.wa = cg.w * (1.0f - cg.fu);
+                            col.wb = cg.w * cg.fu;
+                            off = (unsigned)(y * (long long)p.W + x);
+                            fine = fine || (take && cg.t * (vox * p.inv_pixel) < 1.0001f);
+                            ++i;
+                        }
+                        const unsigned mask = __ballot_sync(0xffffffffu, take);
+                        if (take) {
+                            const int at =
+                                warp * kAdjList + count + __popc(mask & ((1u << lane) - 1u));
+                            s_col[at] = col;
+                            s_off[at] = off;
+                        }
+                        count += __popc(mask);
+                    }
+                    if (lane == 0) s_count[warp] = count;
+                    more = __syncthreads_or(i < i_end);
+                    fine = __syncthreads_or(fine);
+                    if (reached) {
+                        for (int list = 0; list < warps; ++list) {
+                            const AdjColumn* cols = s_col + list * kAdjList;
+                            const unsigned* offs = s_off + list * kAdjList;
+                            const int n = s_count[list];
+                            if (fine || careful) sum_list_general(cols, offs, n);
+                            else if (inner) sum_list(cols, offs, n, std::false_type());
+                            else sum_list(cols, offs, n, std::true_type());
+                        }
+                    }
+                    __syncthreads();
+                } while (more);
+            }
+            bool bad = false;
+#pragma unroll
+            for (int j = 0; j < NV; ++j) bad = bad || !isfinite(acc_a[j]) || !isfinite(acc_b[j]);
+            if (!__syncthreads_or(bad && !careful)) break;
+        }
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int v = v_first + 32 * j;
+            if (v < p.V) {
+                float* o = out + (long long)b * p.V + v;
+                if (b == b0) red_add_global(o, acc_a[j]);  // the CTA before adds its last row
+                else *o = acc_a[j];
+                if (b == b1 - 1) red_add_global(o + p.V, acc_b[j]);
+            }
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -701,9 +1025,10 @@ int launch_bp_forward_kz(const BpArgs& p, bool pixdiv, bool fdk, dim3 grid, cuda
 }
 
 template <int KZ>
-int launch_bp_backward_kz(const BpArgs& p, int gp, dim3 grid, cudaStream_t s) {
-    if (gp) bp_backward_kernel<KZ, 1><<<grid, 256, 0, s>>>(p);
-    else bp_backward_kernel<KZ, 0><<<grid, 256, 0, s>>>(p);
+int launch_bp_backward_kz(const BpArgs& p, int gp, bool geo, dim3 grid, cudaStream_t s) {
+    if (!geo) bp_backward_kernel<KZ, 1, false><<<grid, 256, 0, s>>>(p);
+    else if (gp) bp_backward_kernel<KZ, 1, true><<<grid, 256, 0, s>>>(p);
+    else bp_backward_kernel<KZ, 0, true><<<grid, 256, 0, s>>>(p);
     DGC_LAUNCH_CHECK("bp_backward_kernel");
     return DGC_OK;
 }
@@ -734,12 +1059,77 @@ int bp_launch_backward(const BpArgs& p, cudaStream_t s) {
     bp_grid(p.D, p.H, p.W, kz, gx, gy);
     const dim3 grid(gx, gy);
     const int gp = p.grad_projections ? 1 : 0;
+    const bool geo = p.partials != nullptr;
     switch (kz) {
-        case 1: return launch_bp_backward_kz<1>(p, gp, grid, s);
-        case 2: return launch_bp_backward_kz<2>(p, gp, grid, s);
-        case 4: return launch_bp_backward_kz<4>(p, gp, grid, s);
-        default: return launch_bp_backward_kz<8>(p, gp, grid, s);
+        case 1: return launch_bp_backward_kz<1>(p, gp, geo, grid, s);
+        case 2: return launch_bp_backward_kz<2>(p, gp, geo, grid, s);
+        case 4: return launch_bp_backward_kz<4>(p, gp, geo, grid, s);
+        default: return launch_bp_backward_kz<8>(p, gp, geo, grid, s);
     }
+}
+
+size_t bp_column_floats(int D, int H, int W) { return (size_t)(D + 3) * H * W; }
+
+// Detector rows that the volume spans, at about twofold magnification.
+static float bp_shadow(const BpArgs& p) { return 2.2f * p.D * p.voxel_size * p.inv_pixel; }
+
+// Gather or scatter?  The gather's work is a column times the detector's rows
+// (those in the volume's shadow), whatever the number of voxels along z, and its
+// columns come in bins that must feed whole CTAs.  Measured gather / scatter,
+// the projection gradient alone: 10.0 / 18.5 ms (256^3 / 360 x 384^2), 3.4 / 5.1
+// (200 x 180 x 150 / 300 x 260 x 290), 1.07 / 1.63 (128^3 / 180 x 256^2), 0.26 /
+// 0.35 (96^3), 0.11 / 0.15 (64^3 / 90 x 128^2), 0.14 / 0.18 (48^3), but 0.028 /
+// 0.017 ms (16 x 20 x 24), 4.0 / 1.3 ms for a slab of 32 slices under 384 rows
+// 1.3 / 0.18 ms for voxels below a pixel (0.64; more than two candidates) and
+// 0.47 / 0.44 ms for voxels of 6.7 pixels (most pixels of a column wasted; 1.1 /
+// 1.5 ms at 3.3).
+// With the geometry gradients the scatter shares its march with theirs: 20.4 /
+// 24.4 ms at 256^3, 1.89 / 2.06 at 128^3, but 0.48 / 0.44 at 96^3.
+bool bp_gathers(const BpArgs& p, bool with_geometry) {
+    const long long area = (long long)p.H * p.W;
+    return p.voxel_size >= 0.75f * p.pixel_size && p.voxel_size <= 3.0f * p.pixel_size &&
+           bp_shadow(p) >= 0.6f * p.V && area >= (with_geometry ? 128 * 128 : 32 * 32);
+}
+
+int bp_launch_gather(const BpArgs& p, float* columns, cudaStream_t s) {
+    {
+        DGC_TRACE("bp_columns", s);
+        const dim3 grid((unsigned)(ceil_div(p.W, 32) * (long long)p.H), (unsigned)ceil_div(p.D + 3, 32));
+        bp_columns_kernel<<<grid, dim3(32, 8), 0, s>>>(p.grad_volume, p.D, p.H, p.W, columns);
+        DGC_LAUNCH_CHECK("bp_columns");
+    }
+    DGC_TRACE("bp_adjoint_kernel", s);
+    // pixels a thread and warps a CTA: the fewest idle slots, a column's own
+    // instructions (about 10) against 25 a pixel; a warp that the volume's shadow
+    // does not reach costs little
+    const float shadow = bp_shadow(p);
+    int nv = 1, warps = 1, tiles = 1;
+    float best = FLT_MAX;
+    for (int n = 1; n <= 3; ++n) {
+        const int t = ceil_div(p.V, 32LL * n * kAdjMaxWarps);
+        const int w = ceil_div(ceil_div(p.V, t), 32 * n);
+        const float slots = std::min(32.0f * n * w * t, shadow + 32.0f * n);
+        const float cost = slots * (25.0f + 10.0f / n);
+        if (cost < best) {
+            best = cost;
+            nv = n;
+            warps = w;
+            tiles = t;
+        }
+    }
+    // bins per CTA: up to 16, as many as leave every SM some 32 CTAs
+    int bins = 16;
+    while (bins > 2 && (long long)p.A * ceil_div(p.U - 1, bins) * tiles < 148LL * 32) bins >>= 1;
+    const int bin_blocks = ceil_div(p.U - 1, bins);
+    const unsigned grid = (unsigned)((long long)p.A * bin_blocks * tiles);
+    const size_t smem = (size_t)warps * kAdjList * (sizeof(AdjColumn) + sizeof(unsigned));
+    switch (nv) {
+        case 1: bp_adjoint_kernel<1><<<grid, 32 * warps, smem, s>>>(p, columns, bins, bin_blocks, tiles); break;
+        case 2: bp_adjoint_kernel<2><<<grid, 32 * warps, smem, s>>>(p, columns, bins, bin_blocks, tiles); break;
+        default: bp_adjoint_kernel<3><<<grid, 32 * warps, smem, s>>>(p, columns, bins, bin_blocks, tiles); break;
+    }
+    DGC_LAUNCH_CHECK("bp_adjoint_kernel");
+    return DGC_OK;
 }
 
 __global__ void clamp_volume_kernel(float* __restrict__ v, long long n) {

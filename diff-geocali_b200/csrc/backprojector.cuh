@@ -33,13 +33,19 @@ struct BpArgs {
     // backward
     const float* grad_volume;  // [D][H][W]
     float* grad_projections;   // [A][U][V], zeroed by the caller; null: not computed
-    double* partials;          // [A][8][blocks]
+    double* partials;          // [A][8][blocks]; null: no geometry gradients
 };
 
 int bp_view_table(const Geometry& g, int A, ViewRow* vt, cudaStream_t s);
 int build_proj_quads(const float* P, int A, int U, int V, float4* PQ, cudaStream_t s);
 int bp_launch_forward(const BpArgs& p, bool fdk, cudaStream_t s);
 int bp_launch_backward(const BpArgs& p, cudaStream_t s);
+// Projection gradient as a gather (where bp_gathers says so): the upstream volume
+// as z-fastest columns (scratch of bp_column_floats), then every pixel of
+// p.grad_projections (zeroed).
+bool bp_gathers(const BpArgs& p, bool with_geometry);
+size_t bp_column_floats(int D, int H, int W);
+int bp_launch_gather(const BpArgs& p, float* columns, cudaStream_t s);
 int bp_clamp_volume(float* volume, long long n, cudaStream_t s);
 long long bp_backward_blocks(int D, int H, int W, int kz);
 // Tiles of a call with volume depth D and A views (rules, overrides, built-in

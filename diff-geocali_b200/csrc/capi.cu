@@ -453,8 +453,14 @@ int dgc_backproject(const float* projections, int A, int U, int V, const float* 
 
 size_t dgc_backproject_backward_workspace_bytes(int A, int U, int V, int D, int H, int W) {
     if (A <= 0 || U < 2 || V < 2 || D <= 0 || H <= 0 || W <= 0) return 0;
-    return bp_table_bytes(A) + bp_quads_bytes(A, U, V) +
-           Workspace::align(sizeof(double) * 8 * (size_t)A * (size_t)bp_backward_blocks(D, H, W, bp_kz_backward(D, A)));
+    // the projection gradient as a gather is done with its columns before the
+    // quads and partials of the geometry gradients are written in their place
+    const size_t columns = Workspace::align(sizeof(float) * bp_column_floats(D, H, W));
+    const size_t geometry =
+        bp_quads_bytes(A, U, V) +
+        Workspace::align(sizeof(double) * 8 * (size_t)A *
+                         (size_t)bp_backward_blocks(D, H, W, bp_kz_backward(D, A)));
+    return bp_table_bytes(A) + std::max(columns, geometry);
 }
 
 int dgc_backproject_backward(const float* grad_volume, const float* projections, int A, int U,
@@ -480,26 +486,69 @@ int dgc_backproject_backward(const float* grad_volume, const float* projections,
     const long long nblocks = bp_backward_blocks(D, H, W, kz);
     Workspace ws(workspace, workspace_bytes);
     ViewRow* vt = ws.take<ViewRow>((size_t)A);
+    Workspace ws_columns = ws;  // shares its memory with the quads and partials
+    float* columns = grad_projections ? ws_columns.take<float>(bp_column_floats(D, H, W)) : nullptr;
     float4* pq = ws.take<float4>((size_t)A * (U - 1) * (V - 1));
     double* partials = ws.take<double>((size_t)8 * A * nblocks);
-    if (!vt || !pq || !partials) {
+    if (!vt || !pq || !partials || (grad_projections && !columns)) {
         set_error("workspace too small: dgc_backproject_backward needs " +
                   std::to_string(dgc_backproject_backward_workspace_bytes(A, U, V, D, H, W)) +
                   " bytes");
         return DGC_ERR_WORKSPACE;
     }
     if ((rc = bp_view_table(g, A, vt, s)) != DGC_OK) return rc;
-    if ((rc = build_proj_quads(projections, A, U, V, pq, s)) != DGC_OK) return rc;
     BpArgs p = bp_args(vt, pq, A, U, V, D, H, W, pixel_size, voxel_size, off_x, off_y, off_z);
     if (grad_projections) {
-        DGC_CUDA(cudaMemsetAsync(grad_projections, 0, sizeof(float) * (size_t)A * U * V, s));
+        p.grad_volume = grad_volume;
         p.grad_projections = grad_projections;
+        DGC_CUDA(cudaMemsetAsync(grad_projections, 0, sizeof(float) * (size_t)A * U * V, s));
+        if (bp_gathers(p, true)) {
+            if ((rc = bp_launch_gather(p, columns, s)) != DGC_OK) return rc;
+            p.grad_projections = nullptr;  // done: the geometry gradients alone remain
+        }
     }
+    if ((rc = build_proj_quads(projections, A, U, V, pq, s)) != DGC_OK) return rc;
     p.grad_volume = grad_volume;
     p.partials = partials;
     p.kz_backward = kz;
     if ((rc = bp_launch_backward(p, s)) != DGC_OK) return rc;
     return bp_reduce_partials(partials, A, nblocks, out, s);
+}
+
+// --------------------------------------------- projection gradient alone
+
+size_t dgc_backproject_adjoint_workspace_bytes(int A, int D, int H, int W) {
+    if (A <= 0 || D <= 0 || H <= 0 || W <= 0) return 0;
+    return bp_table_bytes(A) + Workspace::align(sizeof(float) * bp_column_floats(D, H, W));
+}
+
+int dgc_backproject_adjoint(const float* grad_volume, int A, int U, int V, const float* angles,
+                            const float* sid, const float* sod, const float* det_u0,
+                            const float* det_v0, const float* src_x, const float* src_y,
+                            const float* src_z, float pixel_size, int D, int H, int W,
+                            float voxel_size, float off_x, float off_y, float off_z,
+                            float* grad_projections, void* workspace, size_t workspace_bytes,
+                            void* stream) {
+    clear_error();
+    cudaStream_t s = (cudaStream_t)stream;
+    const Geometry g = make_geometry(angles, sid, sod, det_u0, det_v0, src_x, src_y, src_z);
+    int rc = check_bp_common(A, U, V, D, H, W, pixel_size, voxel_size, off_x, off_y, off_z, g);
+    if (rc != DGC_OK) return rc;
+    DGC_REQUIRE(grad_volume && grad_projections, "grad_vol and grad_proj must be non-null");
+    Workspace ws(workspace, workspace_bytes);
+    ViewRow* vt = ws.take<ViewRow>((size_t)A);
+    float* columns = ws.take<float>(bp_column_floats(D, H, W));
+    if (!vt || !columns) {
+        set_error("workspace too small: dgc_backproject_adjoint needs " +
+                  std::to_string(dgc_backproject_adjoint_workspace_bytes(A, D, H, W)) + " bytes");
+        return DGC_ERR_WORKSPACE;
+    }
+    if ((rc = bp_view_table(g, A, vt, s)) != DGC_OK) return rc;
+    BpArgs p = bp_args(vt, nullptr, A, U, V, D, H, W, pixel_size, voxel_size, off_x, off_y, off_z);
+    p.grad_volume = grad_volume;
+    p.grad_projections = grad_projections;
+    DGC_CUDA(cudaMemsetAsync(grad_projections, 0, sizeof(float) * (size_t)A * U * V, s));
+    return bp_gathers(p, false) ? bp_launch_gather(p, columns, s) : bp_launch_backward(p, s);
 }
 
 // --------------------------------------------------------------------- FDK

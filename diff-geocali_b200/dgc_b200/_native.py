@@ -67,6 +67,9 @@ SIGNATURES = {
     "dgc_backproject_backward_workspace_bytes": (_S, [_I] * 6),
     "dgc_backproject_backward": (_I, [_P, _P, _I, _I, _I, *_GEOM, _F, _I, _I, _I, _F, _F, _F, _F,
                                       *([_P] * 9), _P, _S, _P]),
+    "dgc_backproject_adjoint_workspace_bytes": (_S, [_I] * 4),
+    "dgc_backproject_adjoint": (_I, [_P, _I, _I, _I, *_GEOM, _F, _I, _I, _I, _F, _F, _F, _F, _P, _P,
+                                     _S, _P]),
     "dgc_fdk_filter_taps": (_I, [_I, _D, _D, ctypes.POINTER(_D)]),
     "dgc_fdk_filter_workspace_bytes": (_S, [_I] * 3),
     "dgc_fdk_filter": (_I, [_P, _I, _I, _I, _F, _P, _P, _F, _P, _P, _S, _P]),

@@ -65,7 +65,8 @@ class _Backproject(torch.autograd.Function):
         pixel_size, voxel_size, offset = ctx.settings
         wanted = ctx.needs_input_grad[:9]
         grads = _ops.bp_backward(grad_volume.contiguous(), *ctx.saved_tensors,
-                                 pixel_size, voxel_size, *offset, compute_grad_proj=wanted[0])
+                                 pixel_size, voxel_size, *offset, compute_grad_proj=wanted[0],
+                                 compute_grad_geometry=any(wanted[1:]))
         return tuple(g if need else None for g, need in zip(grads, wanted)) + (None,) * 4
 
 

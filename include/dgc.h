@@ -140,8 +140,8 @@ size_t dgc_backproject_backward_workspace_bytes(int A, int U, int V, int D, int 
  * (csrc/src_cbct_backprojector_cuda.cu:423-522, kernel 101-295).
  * Writes grad_projections [A,U,V] and the eight geometry gradients [A]
  * (per-view FP64 reductions in a fixed order).  grad_projections may be NULL:
- * the projection gradient (the bilinear scatter) is then skipped, which the
- * reference always computes. */
+ * the projection gradient (the adjoint of the bilinear taps) is then
+ * skipped, which the reference always computes. */
 int dgc_backproject_backward(const float* grad_volume, const float* projections,
                              int A, int U, int V,
                              const float* angles, const float* sid, const float* sod,
@@ -153,6 +153,22 @@ int dgc_backproject_backward(const float* grad_volume, const float* projections,
                              float* grad_sod, float* grad_det_u0, float* grad_det_v0,
                              float* grad_src_x, float* grad_src_y, float* grad_src_z,
                              void* workspace, size_t workspace_bytes, void* stream);
+
+/* Scratch of dgc_backproject_adjoint. */
+size_t dgc_backproject_adjoint_workspace_bytes(int A, int D, int H, int W);
+
+/* The projection gradient of dgc_backproject alone (dgc_backproject_backward
+ * without the geometry gradients, which an autograd call with fixed geometry
+ * drops): the projections are not read.  No counterpart in the reference, whose
+ * backward always computes the geometry gradients
+ * (csrc/src_cbct_backprojector_cuda.cu:423-522). */
+int dgc_backproject_adjoint(const float* grad_volume, int A, int U, int V,
+                            const float* angles, const float* sid, const float* sod,
+                            const float* det_u0, const float* det_v0,
+                            const float* src_x, const float* src_y, const float* src_z,
+                            float pixel_size, int D, int H, int W, float voxel_size,
+                            float off_x, float off_y, float off_z, float* grad_projections,
+                            void* workspace, size_t workspace_bytes, void* stream);
 
 /* ---------------------------------------------------------------------- */
 /* FDK                                                                      */

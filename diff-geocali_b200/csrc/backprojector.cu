@@ -116,7 +116,8 @@ __device__ __forceinline__ ColumnView column_view(const ViewRow& r, int a, float
     const float t = sdn / denom;
     const float u_phys = r.ds_u + t * (px - r.ds_u);
     const float sw = (r.sod + r.ds_n) / denom;
-    const float u_idx = PIXDIV ? u_phys / p.pixel_size + r.u0 : fmaf(u_phys, p.inv_pixel, r.u0);
+    const float u_idx = PIXDIV ? div_by(u_phys, p.pixel_size, p.inv_pixel) + r.u0
+                               : fmaf(u_phys, p.inv_pixel, r.u0);
     if (!(u_idx >= 0.0f && u_idx < (p.U - 1.0f))) return cv;
     const int ui = (int)floorf(u_idx);
     cv.valid = true;
@@ -215,6 +216,7 @@ __global__ void __maxnreg__(KZ == 1 ? 40 : KZ == 2 ? 48 : KZ == 4 ? 64 : 96) bp_
 #pragma unroll
         for (int k = 0; k + 1 < KZ; k += 2) pz2[k / 2] = pack2(pz[k], pz[k + 1]);
         const f32x2 ip2 = pack2(p.inv_pixel, p.inv_pixel);
+        const f32x2 npix2 = pack2(-p.pixel_size, -p.pixel_size);
         const f32x2 magic2 = pack2(kFloorMagic, kFloorMagic);
         for (int a0 = 0; a0 < p.A; a0 += 32) {
             ColumnView mine;
@@ -246,12 +248,13 @@ __global__ void __maxnreg__(KZ == 1 ? 40 : KZ == 2 ? 48 : KZ == 4 ? 64 : 96) bp_
                             part[k] = fmaf(w, lerpf(e.x, e.y, fu), part[k]);
                         }
                     };
-                    if constexpr (!PIXDIV && KZ % 2 == 0) {
+                    if constexpr (KZ % 2 == 0) {
                         const f32x2 t2 = pack2(t, t), d2 = pack2(dsv, dsv), o2 = pack2(v0, v0);
 #pragma unroll
                         for (int k = 0; k < KZ; k += 2) {
                             const f32x2 vp = fma2(t2, sub2(pz2[k / 2], d2), d2);
-                            const f32x2 vx2 = fma2(vp, ip2, o2);
+                            const f32x2 vx2 = PIXDIV ? add2(div_by2(vp, npix2, ip2), o2)
+                                                     : fma2(vp, ip2, o2);
                             const f32x2 f2 = add2_rd(vx2, magic2);
                             const float2 fr = unpack2(sub2(vx2, sub2(f2, magic2)));
                             const uint2 bits = unpack2_bits(f2);
@@ -263,7 +266,8 @@ __global__ void __maxnreg__(KZ == 1 ? 40 : KZ == 2 ? 48 : KZ == 4 ? 64 : 96) bp_
                         for (int k = 0; k < KZ; ++k) {
                             const float v_phys = dsv + t * (pz[k] - dsv);
                             const float v_idx =
-                                PIXDIV ? v_phys / p.pixel_size + v0 : fmaf(v_phys, p.inv_pixel, v0);
+                                PIXDIV ? div_by(v_phys, p.pixel_size, p.inv_pixel) + v0
+                                       : fmaf(v_phys, p.inv_pixel, v0);
                             const FloorSplit fs = floor_split(v_idx);
                             tap(k, fs.biased, fs.frac);
                         }

@@ -271,7 +271,7 @@ template <bool DIV, bool OFF = true>
 __device__ __forceinline__ float to_voxel(float pos, float off, float voxel, float inv_voxel,
                                           float half) {
     const float q = OFF ? pos - off : pos;
-    if (DIV) return __fdiv_rn(q, voxel) + half;
+    if (DIV) return div_by(q, voxel, inv_voxel) + half;
     return fmaf(q, inv_voxel, half);
 }
 
@@ -326,26 +326,30 @@ __device__ __forceinline__ Cell locate(float x, float y, float z, const FpArgs& 
 // unscaled one, with two registers fewer (35.6 -> 35.2 ms at 256^3 / 360 x
 // 384^2, 3.17 -> 3.10 ms at 128^3 / 180 x 256^2).
 struct XYPacks {
-    f32x2 dxy, oxy, offxy, hxy, magic2;
+    f32x2 dxy, oxy, offxy, hxy, magic2, nvox2, inv2;
     float dz, oz, offz;
 };
 
+// DIV: any voxel size, nothing scaled (nvox2, inv2: the division's operands).
+template <bool DIV>
 __device__ __forceinline__ XYPacks make_xy_packs(const RaySetup& r, const ViewGeo& vg,
                                                  const FpArgs& p) {
+    const float scale = DIV ? 1.0f : p.inv_voxel;
     XYPacks k;
-    k.dxy = pack2(r.dx * p.inv_voxel, r.dy * p.inv_voxel);
-    k.oxy = pack2(vg.ox * p.inv_voxel, vg.oy * p.inv_voxel);
-    k.offxy = pack2(p.off_x * p.inv_voxel, p.off_y * p.inv_voxel);
-    k.dz = r.dz * p.inv_voxel;
-    k.oz = vg.oz * p.inv_voxel;
-    k.offz = p.off_z * p.inv_voxel;
+    k.dxy = pack2(r.dx * scale, r.dy * scale);
+    k.oxy = pack2(vg.ox * scale, vg.oy * scale);
+    k.offxy = pack2(p.off_x * scale, p.off_y * scale);
+    k.dz = r.dz * scale;
+    k.oz = vg.oz * scale;
+    k.offz = p.off_z * scale;
+    k.nvox2 = pack2(-p.voxel_size, -p.voxel_size);
+    k.inv2 = pack2(p.inv_voxel, p.inv_voxel);
     k.hxy = pack2(p.W * 0.5f, p.H * 0.5f);
     k.magic2 = pack2(kFloorMagic, kFloorMagic);
     return k;
 }
 
-// Cell of the sample at t.  With PACK, no clamping and the multiplying voxel
-// conversion, x and y run as packed pairs (fma.rn / sub.rn / add.rm on
+// Cell of the sample at t.  With PACK and no clamping, x and y run as packed pairs (fma.rn / sub.rn / add.rm on
 // f32x2): lane by lane the same IEEE operations as the scalar path, so the
 // cell and weights are bitwise those of locate(to_voxel(...)).  On the forward
 // sum 1-3 % faster; the gradient marches, together with dropping the iteration
@@ -355,14 +359,17 @@ template <bool CLAMP, bool DIV, bool OFF, bool PACK>
 __device__ __forceinline__ Cell sample_cell(float t, const RaySetup& r, const ViewGeo& vg,
                                             const FpArgs& p, const XYPacks& k) {
     const float hz = p.D * 0.5f;
-    if constexpr (PACK && !CLAMP && !DIV) {
+    if constexpr (PACK && !CLAMP) {
         const f32x2 pxy = fma2(pack2(t, t), k.dxy, k.oxy);
-        const f32x2 vxy = add2(OFF ? sub2(pxy, k.offxy) : pxy, k.hxy);
+        const f32x2 qxy = OFF ? sub2(pxy, k.offxy) : pxy;
+        const f32x2 vxy = add2(DIV ? div_by2(qxy, k.nvox2, k.inv2) : qxy, k.hxy);
         const f32x2 fxy = add2_rd(vxy, k.magic2);
         const float2 frac = unpack2(sub2(vxy, sub2(fxy, k.magic2)));
         const uint2 bits = unpack2_bits(fxy);
         const float pz = fmaf(t, k.dz, k.oz);
-        const FloorSplit sz = floor_split((OFF ? pz - k.offz : pz) + hz);
+        const float qz = OFF ? pz - k.offz : pz;
+        const FloorSplit sz =
+            floor_split((DIV ? div_by(qz, p.voxel_size, p.inv_voxel) : qz) + hz);
         Cell c;
         c.bx = bits.x;
         c.by = bits.y;
@@ -424,7 +431,7 @@ __device__ __forceinline__ float quad_value(const ulonglong2& q0, const ulonglon
 template <bool CLAMP, bool DIV, bool OFF, bool GUARD = true, int UNROLL = 1>
 __device__ __forceinline__ float march_sum(const RaySetup& r, const ViewGeo& vg, const FpArgs& p) {
     const ulonglong2* __restrict__ Q = reinterpret_cast<const ulonglong2*>(p.quads);
-    const XYPacks k = make_xy_packs(r, vg, p);
+    const XYPacks k = make_xy_packs<DIV>(r, vg, p);
     const int nmax = step_bound(r, p.step_size);
     float acc = 0.0f;
     float t = r.tmin;
@@ -552,7 +559,7 @@ __device__ __forceinline__ float march_sum_pairs(const RaySetup& r, const ViewGe
                                                  const FpArgs& p) {
     const unsigned long long* __restrict__ P =
         reinterpret_cast<const unsigned long long*>(p.quads);
-    const XYPacks k = make_xy_packs(r, vg, p);
+    const XYPacks k = make_xy_packs<DIV>(r, vg, p);
     const int nmax = step_bound(r, p.step_size);
     const uint32_t sx = (uint32_t)(p.D + 1), sy = (uint32_t)(p.W + 2) * (uint32_t)(p.D + 1);
     const uint32_t bias = (1u + sx + sy) - kFloorMagicBits * (1u + sx + sy);
@@ -802,7 +809,7 @@ __global__ void __launch_bounds__(256, 4) fp_forward_tma_kernel(FpArgs p,
         }
     }
     __syncthreads();
-    const XYPacks k = make_xy_packs(r, vg, p);
+    const XYPacks k = make_xy_packs<DIV>(r, vg, p);
     const bool inside = active ? ray_inside_pad<DIV>(r, vg, p) : true;
     const int nmax = active ? step_bound(r, p.step_size) : 0;
     float t = r.tmin, acc = 0.0f;
@@ -1019,7 +1026,7 @@ template <bool CLAMP, bool GRADVOL, bool POW2, bool OFF, bool GUARD>
 __device__ __forceinline__ RayGrad march_grad(const RaySetup& r, const ViewGeo& vg,
                                               const FpArgs& p, float gs) {
     const ulonglong2* __restrict__ Q = reinterpret_cast<const ulonglong2*>(p.quads);
-    const XYPacks k = make_xy_packs(r, vg, p);
+    const XYPacks k = make_xy_packs<!POW2>(r, vg, p);
     RayGrad rg{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     const int nmax = step_bound(r, p.step_size);
     const EdgeSteps es = edge_steps(r, p);
@@ -1290,7 +1297,7 @@ template <bool CLAMP, bool DIV, bool OFF, bool GUARD = true>
 __device__ __forceinline__ RayValueGrad march_value_grad(const RaySetup& r, const ViewGeo& vg,
                                                          const FpArgs& p) {
     const ulonglong2* __restrict__ Q = reinterpret_cast<const ulonglong2*>(p.quads);
-    const XYPacks k = make_xy_packs(r, vg, p);
+    const XYPacks k = make_xy_packs<DIV>(r, vg, p);
     RayValueGrad out{0.0f, {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}};
     const int nmax = step_bound(r, p.step_size);
     float t = r.tmin;

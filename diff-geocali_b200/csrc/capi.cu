@@ -130,6 +130,24 @@ int fp_check_args(int D, int H, int W, int A, int U, int V, float pixel_size, fl
 
 using namespace dgc;
 
+// Long reductions with few output tiles (weight gradients): split K over CTAs and
+// sum into a zeroed fp32 C with atomics.
+static int gemm_split_k(GemmArgs p, cudaStream_t s) {
+    const long long tiles = (long long)ceil_div(p.M, 128) * ceil_div(p.N, p.N <= 64 ? 64 : 128);
+    const int ktiles = ceil_div(p.K, 64);
+    if (!p.c_bf16 && !p.relu && tiles < 148 && ktiles >= 32) {
+        const int splits = (int)std::min<long long>(std::max<long long>(296 / tiles, 1), ktiles / 8);
+        if (splits > 1) {
+            p.k_tiles_per_split = ceil_div(ktiles, splits);
+            // zero only the M x N window: C may be a column slice of a wider array
+            if (!p.accumulate)
+                DGC_CUDA(cudaMemset2DAsync(p.C, sizeof(float) * (size_t)p.ldc, 0,
+                                           sizeof(float) * (size_t)p.N, (size_t)p.M, s));
+        }
+    }
+    return tc_gemm(p, s);
+}
+
 extern "C" {
 
 int dgc_abi_version(void) { return DGC_ABI_VERSION; }
@@ -887,21 +905,24 @@ int dgc_gemm_bf16(const void* A, const void* B, void* C, const float* bias, int 
     DGC_REQUIRE(ceil_div(M, 128) <= 65535, "M too large for one launch");
     GemmArgs p{static_cast<const __nv_bfloat16*>(A), static_cast<const __nv_bfloat16*>(B), C, bias,
                M, N, K, lda, ldb, ldc, c_bf16, relu, accumulate, alpha, error_flag, 0};
-    // Long reductions with few output tiles (weight gradients): split K over
-    // CTAs and sum into a zeroed fp32 C with atomics.
-    const long long tiles = (long long)ceil_div(M, 128) * ceil_div(N, N <= 64 ? 64 : 128);
-    const int ktiles = ceil_div(K, 64);
-    if (!c_bf16 && !relu && tiles < 148 && ktiles >= 32) {
-        const int splits = (int)std::min<long long>(std::max<long long>(296 / tiles, 1), ktiles / 8);
-        if (splits > 1) {
-            p.k_tiles_per_split = ceil_div(ktiles, splits);
-            // zero only the M x N window: C may be a column slice of a wider array
-            if (!accumulate)
-                DGC_CUDA(cudaMemset2DAsync(C, sizeof(float) * (size_t)ldc, 0, sizeof(float) * (size_t)N,
-                                           (size_t)M, (cudaStream_t)stream));
-        }
-    }
-    return tc_gemm(p, (cudaStream_t)stream);
+    return gemm_split_k(p, (cudaStream_t)stream);
+}
+
+int dgc_gemm_bf16_tn(const void* A, const void* B, float* C, int M, int N, int K, int lda, int ldb,
+                     int ldc, int accumulate, float alpha, int* error_flag, void* stream) {
+    clear_error();
+    DGC_REQUIRE(A && B && C && error_flag, "A, B, C and error_flag must be non-null");
+    DGC_REQUIRE(M > 0 && N > 0 && K > 0, "M, N, K must be positive");
+    DGC_REQUIRE(lda % 8 == 0 && ldb % 8 == 0 && lda >= M && ldb >= N,
+                "lda and ldb must be multiples of 8 (16-byte rows) with lda >= M, ldb >= N");
+    DGC_REQUIRE(ldc >= N, "ldc must be >= N");
+    DGC_REQUIRE(((uintptr_t)A % 16) == 0 && ((uintptr_t)B % 16) == 0,
+                "A and B must be 16-byte aligned");
+    DGC_REQUIRE(ceil_div(M, 128) <= 65535, "M too large for one launch");
+    GemmArgs p{static_cast<const __nv_bfloat16*>(A), static_cast<const __nv_bfloat16*>(B), C,
+               nullptr, M, N, K, lda, ldb, ldc, 0, 0, accumulate, alpha, error_flag, 0, 1};
+    return gemm_split_k(p, (cudaStream_t)stream);
 }
 
 }  // extern "C"
+

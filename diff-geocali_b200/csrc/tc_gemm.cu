@@ -4,7 +4,9 @@
 //
 //   C[m, n] (+)= sum_k A[m, k] * B[n, k]  (+ bias[n], optional ReLU)
 //
-// A (M x K) and B (N x K) are row-major bf16 ("K-major"); C is fp32 or bf16.
+// A (M x K) and B (N x K) are row-major bf16 ("K-major"); C is fp32 or bf16.  The
+// TMA kernel also takes both operands as stored [K][M] and [K][N] ("MN-major"):
+// a weight gradient reduces over the rows of activations that lie that way.
 //
 // Structure of a CTA (128 threads, one 128 x BN output tile):
 //   * warp 0 allocates BN tensor-memory columns (a 128-lane x BN fp32
@@ -106,10 +108,25 @@ __device__ __forceinline__ uint64_t kmajor_sw128_desc(uint32_t saddr) {
     return d;
 }
 
-// Instruction descriptor of kind::f16 with bf16 A and B, fp32 D, both K-major.
+// The same for MN-major operands staged as boxes of 64 (M or N) x kBK (K): a K row
+// is 128 contiguous bytes; SBO = 1024 B between groups of 8 K rows, LBO = one
+// box (kBK * 128 B) between groups of 64 M or N.
+__device__ __forceinline__ uint64_t mnmajor_sw128_desc(uint32_t saddr) {
+    uint64_t d = 0;
+    d |= static_cast<uint64_t>((saddr >> 4) & 0x3FFFu);
+    d |= static_cast<uint64_t>((kBK * 128u) >> 4) << 16;
+    d |= static_cast<uint64_t>(1024u >> 4) << 32;
+    d |= static_cast<uint64_t>(1) << 46;
+    d |= static_cast<uint64_t>(2) << 61;
+    return d;
+}
+
+// Instruction descriptor of kind::f16 with bf16 A and B, fp32 D; both K-major, or
+// with MN both MN-major (bits 15 and 16).
+template <bool MN = false>
 __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) |
-           (static_cast<uint32_t>(m >> 4) << 24);
+    return (1u << 4) | (1u << 7) | (1u << 10) | (MN ? 3u << 15 : 0u) |
+           (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
@@ -149,6 +166,15 @@ __device__ __forceinline__ void tmem_load16(uint32_t taddr, float (&v)[16]) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// 32 bytes to a 32-byte aligned global address.
+__device__ __forceinline__ void store32(void* p, const uint32_t (&v)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(
+                     __cvta_generic_to_global(p)),
+                 "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]),
+                 "r"(v[7])
+                 : "memory");
+}
+
 // Stage one K-slice: 'rows' x 64 bf16 of a K-major matrix into the 128-byte
 // swizzled layout (16-byte chunk j of row r at r*128 + ((j ^ (r & 7)) * 16)).
 // Out-of-range rows or K chunks are zero-filled.
@@ -168,42 +194,72 @@ __device__ __forceinline__ void stage_tile(uint32_t sbase, const __nv_bfloat16* 
 
 // Epilogue: the four warps read their 32 accumulator lanes (rows) with
 // tcgen05.ld, 16 columns at a time, and apply alpha / bias / ReLU /
-// accumulate (or the split-K atomic sum) on the way to C.
+// accumulate (or the split-K atomic sum) on the way to C.  A lane's 16 columns
+// go out as 32-byte stores (whole sectors) where C's alignment allows it; one
+// element at a time every lane touched another row's sector 16 times over
+// (8192^3: 1087 -> 1428 TFLOP/s; the data-gradient products of the network at 180
+// views, 1.1 GB of fp32 output: 1.0 -> 0.36 ms with the short-K tiles below).
 template <int BN>
 __device__ __forceinline__ void gemm_epilogue(const GemmArgs& p, uint32_t tmem, int m0, int n0,
                                               bool has_k, bool split) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    {
-        const int row = m0 + warp * 32 + lane;
-        const uint32_t lane_addr = tmem + (static_cast<uint32_t>(warp * 32) << 16);
+    const int row = m0 + warp * 32 + lane;
+    const uint32_t lane_addr = tmem + (static_cast<uint32_t>(warp * 32) << 16);
+    const bool wide = (reinterpret_cast<uintptr_t>(p.C) & 31u) == 0 &&
+                      p.ldc % (p.c_bf16 ? 16 : 8) == 0;
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 16) {
-            float v[16];
-            tmem_load16(lane_addr + c0, v);
-            if (row < p.M) {
+    for (int c0 = 0; c0 < BN && n0 + c0 < p.N; c0 += 16) {
+        float v[16];
+        tmem_load16(lane_addr + c0, v);
+        if (row >= p.M) continue;
+        const int col0 = n0 + c0;
+        const bool add_bias = p.bias && (!split || blockIdx.z == 0);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const int col = n0 + c0 + j;
-                    if (col >= p.N) break;
-                    float x = has_k ? v[j] : 0.0f;
-                    x *= p.alpha;
-                    const long long off = (long long)row * p.ldc + col;
-                    if (split) {  // partial sum of a K range; bias from split 0
-                        if (p.bias && blockIdx.z == 0) x += p.bias[col];
-                        atomicAdd(static_cast<float*>(p.C) + off, x);
-                        continue;
-                    }
-                    if (p.bias) x += p.bias[col];
-                    if (p.relu) x = fmaxf(x, 0.0f);
-                    if (p.c_bf16) {
-                        __nv_bfloat16* C = static_cast<__nv_bfloat16*>(p.C);
-                        C[off] = __float2bfloat16(x);
-                    } else {
-                        float* C = static_cast<float*>(p.C);
-                        C[off] = p.accumulate ? C[off] + x : x;
-                    }
+        for (int j = 0; j < 16; ++j) {
+            float x = has_k ? v[j] : 0.0f;
+            x *= p.alpha;
+            if (add_bias && col0 + j < p.N) x += p.bias[col0 + j];
+            if (!split && p.relu) x = fmaxf(x, 0.0f);
+            v[j] = x;
+        }
+        const long long off = (long long)row * p.ldc + col0;
+        if (wide && col0 + 16 <= p.N) {
+            if (p.c_bf16) {
+                uint32_t h[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+                    h[j] = *reinterpret_cast<const uint32_t*>(&b);
                 }
+                store32(static_cast<__nv_bfloat16*>(p.C) + off, h);
+                continue;
             }
+            float* C = static_cast<float*>(p.C) + off;
+#pragma unroll
+            for (int j = 0; j < 16; j += 8) {
+                if (split) {  // partial sum of a K range; bias from split 0
+                    red_add4_global(C + j, v[j], v[j + 1], v[j + 2], v[j + 3]);
+                    red_add4_global(C + j + 4, v[j + 4], v[j + 5], v[j + 6], v[j + 7]);
+                    continue;
+                }
+                uint32_t x[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    x[k] = __float_as_uint(p.accumulate ? C[j + k] + v[j + k] : v[j + k]);
+                store32(C + j, x);
+            }
+            continue;
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            if (col0 + j >= p.N) break;
+            if (p.c_bf16) {
+                static_cast<__nv_bfloat16*>(p.C)[off + j] = __float2bfloat16(v[j]);
+                continue;
+            }
+            float* C = static_cast<float*>(p.C) + off + j;
+            if (split) atomicAdd(C, v[j]);
+            else *C = p.accumulate ? *C + v[j] : v[j];
         }
     }
 }
@@ -340,10 +396,14 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
 template <int BN, int MSUB = 1>
 struct TmaStages {
     static constexpr int kStageBytes = MSUB * kBM * kBK * 2 + BN * kBK * 2;
-    static constexpr int value = (196608 / kStageBytes) < 8 ? (196608 / kStageBytes) : 8;
+    // the narrow tiles' products are bound by memory: half the shared memory each,
+    // so that two CTAs per SM overlap their epilogues and loads
+    static constexpr int kBudget = BN <= 128 ? 98304 : 196608;
+    static constexpr int value = (kBudget / kStageBytes) < 8 ? (kBudget / kStageBytes) : 8;
 };
 
-template <int BN, int MSUB>
+// MN: MN-major operands, staged as boxes of 64 M or N x 64 K.
+template <int BN, int MSUB, bool MN>
 __global__ void __launch_bounds__(128) tc_gemm_tma_kernel(const __grid_constant__ CUtensorMap tmA,
                                                           const __grid_constant__ CUtensorMap tmB,
                                                           GemmArgs p) {
@@ -351,7 +411,8 @@ __global__ void __launch_bounds__(128) tc_gemm_tma_kernel(const __grid_constant_
     constexpr int kABytes = MSUB * kBM * kBK * 2;
     constexpr int kStageBytes = TmaStages<BN, MSUB>::kStageBytes;
     constexpr int kCols = MSUB * BN;  // tensor-memory columns of the accumulators
-    constexpr uint32_t kIdesc = idesc_bf16(kBM, BN);
+    constexpr uint32_t kIdesc = idesc_bf16<MN>(kBM, BN);
+    constexpr uint32_t kBox = 64 * kBK * 2;  // bytes of an MN-major box
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[S];
     __shared__ __align__(8) uint64_t empty[S];
@@ -402,8 +463,17 @@ __global__ void __launch_bounds__(128) tc_gemm_tma_kernel(const __grid_constant_
             const uint32_t sa = sbase + s * kStageBytes;
             const int kx = (kt0 + kt) * kBK;
             mbar_expect_tx(smem_u32(&full[s]), kStageBytes);
-            tma_load_2d(sa, &tmA, kx, m0, smem_u32(&full[s]));
-            tma_load_2d(sa + kABytes, &tmB, kx, n0, smem_u32(&full[s]));
+            if (MN) {
+#pragma unroll
+                for (int b = 0; b < MSUB * kBM / 64; ++b)
+                    tma_load_2d(sa + b * kBox, &tmA, m0 + b * 64, kx, smem_u32(&full[s]));
+#pragma unroll
+                for (int b = 0; b < BN / 64; ++b)
+                    tma_load_2d(sa + kABytes + b * kBox, &tmB, n0 + b * 64, kx, smem_u32(&full[s]));
+            } else {
+                tma_load_2d(sa, &tmA, kx, m0, smem_u32(&full[s]));
+                tma_load_2d(sa + kABytes, &tmB, kx, n0, smem_u32(&full[s]));
+            }
             ++issued;
         }
     } else if (warp == 1 && lane == 0) {
@@ -418,11 +488,15 @@ __global__ void __launch_bounds__(128) tc_gemm_tma_kernel(const __grid_constant_
             const uint32_t sa = sbase + s * kStageBytes;
 #pragma unroll
             for (int kk = 0; kk < kBK / 16; ++kk) {
-                const uint64_t bd = kmajor_sw128_desc(sa + kABytes + kk * 32);
+                // K = 16 per instruction: 32 bytes further into every row (K-major)
+                // or two groups of 8 K rows (MN-major)
+                const uint64_t bd = MN ? mnmajor_sw128_desc(sa + kABytes + kk * 2048)
+                                       : kmajor_sw128_desc(sa + kABytes + kk * 32);
 #pragma unroll
                 for (int m = 0; m < MSUB; ++m) {
-                    // sub-tile m: rows 128m.. of the staged A (128 B per row)
-                    const uint64_t ad = kmajor_sw128_desc(sa + m * kBM * 128 + kk * 32);
+                    // sub-tile m: rows 128m.. of the staged A (128 B per row), or its boxes
+                    const uint64_t ad = MN ? mnmajor_sw128_desc(sa + m * 2 * kBox + kk * 2048)
+                                           : kmajor_sw128_desc(sa + m * kBM * 128 + kk * 32);
                     umma_bf16(tmem + m * BN, ad, bd, kIdesc, (kt > 0 || kk > 0) ? 1u : 0u);
                 }
             }
@@ -458,9 +532,9 @@ __global__ void __launch_bounds__(128) tc_gemm_tma_kernel(const __grid_constant_
     }
 }
 
-// 2-D bf16 map of a row-major [rows][ld] matrix with K = cols valid columns:
-// boxes of 64 K elements (128 bytes) x box_rows rows, 128-byte swizzle,
-// zero fill outside.
+// 2-D bf16 map of a row-major [rows][ld] matrix with cols valid columns (K, or M
+// or N of an MN-major operand): boxes of 64 columns (128 bytes) x box_rows rows,
+// 128-byte swizzle, zero fill outside.
 bool make_kmajor_map(CUtensorMap* map, const void* base, int rows, int cols, int ld, int box_rows) {
     EncodeTiledFn fn = encode_tiled();
     if (!fn) return false;
@@ -473,26 +547,33 @@ bool make_kmajor_map(CUtensorMap* map, const void* base, int rows, int cols, int
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN, int MSUB>
+template <int BN, int MSUB, bool MN>
 int launch_gemm_tma(const GemmArgs& p, cudaStream_t s, bool* used) {
     *used = false;
     CUtensorMap ta, tb;
-    if (!make_kmajor_map(&ta, p.A, p.M, p.K, p.lda, kBM * MSUB) ||
-        !make_kmajor_map(&tb, p.B, p.N, p.K, p.ldb, BN))
+    if (MN ? !make_kmajor_map(&ta, p.A, p.K, p.M, p.lda, kBK) ||
+                 !make_kmajor_map(&tb, p.B, p.K, p.N, p.ldb, kBK)
+           : !make_kmajor_map(&ta, p.A, p.M, p.K, p.lda, kBM * MSUB) ||
+                 !make_kmajor_map(&tb, p.B, p.N, p.K, p.ldb, BN))
         return DGC_OK;
-    const int smem = TmaStages<BN, MSUB>::value * TmaStages<BN, MSUB>::kStageBytes + 1024;
+    constexpr int kMost = TmaStages<BN, MSUB>::value * TmaStages<BN, MSUB>::kStageBytes + 1024;
     static std::atomic<unsigned long long> configured{0};
-    const int rc = once_per_device(configured, [smem]() -> int {
-        DGC_CUDA(cudaFuncSetAttribute(tc_gemm_tma_kernel<BN, MSUB>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const int rc = once_per_device(configured, []() -> int {
+        DGC_CUDA(cudaFuncSetAttribute(tc_gemm_tma_kernel<BN, MSUB, MN>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
         return DGC_OK;
     });
     if (rc != DGC_OK) return rc;
-    const int splits = p.k_tiles_per_split > 0
-                           ? ceil_div(ceil_div(p.K, kBK), p.k_tiles_per_split) : 1;
+    const int ktiles = ceil_div(p.K, kBK);
+    const int splits = p.k_tiles_per_split > 0 ? ceil_div(ktiles, p.k_tiles_per_split) : 1;
+    // only the stages that the reduction fills: a short one leaves room for
+    // several CTAs per SM, whose epilogues then overlap
+    const int stages = std::min(TmaStages<BN, MSUB>::value,
+                                p.k_tiles_per_split > 0 ? p.k_tiles_per_split : ktiles);
+    const int smem = stages * TmaStages<BN, MSUB>::kStageBytes + 1024;
     const dim3 grid(ceil_div(p.N, BN), ceil_div(p.M, kBM * MSUB), splits);
     DGC_TRACE("tc_gemm_tma_kernel", s);
-    tc_gemm_tma_kernel<BN, MSUB><<<grid, 128, smem, s>>>(ta, tb, p);
+    tc_gemm_tma_kernel<BN, MSUB, MN><<<grid, 128, smem, s>>>(ta, tb, p);
     DGC_LAUNCH_CHECK("tc_gemm_tma_kernel");
     *used = true;
     return DGC_OK;
@@ -519,12 +600,25 @@ int launch_gemm(const GemmArgs& p, cudaStream_t s) {
 
 }  // namespace
 
+namespace {
+template <bool MN>
+int launch_gemm_tma_bn(const GemmArgs& p, int bn, bool two, cudaStream_t s, bool* used) {
+    return bn == 64    ? launch_gemm_tma<64, 1, MN>(p, s, used)
+           : two       ? launch_gemm_tma<256, 2, MN>(p, s, used)
+           : bn == 256 ? launch_gemm_tma<256, 1, MN>(p, s, used)
+                       : launch_gemm_tma<128, 1, MN>(p, s, used);
+}
+}  // namespace
+
 int tc_gemm(const GemmArgs& p, cudaStream_t s) {
     const int splits = p.k_tiles_per_split > 0 ? ceil_div(ceil_div(p.K, kBK), p.k_tiles_per_split) : 1;
+    // Short reductions (the data gradients' K = 32..256) are bound by their
+    // output: 128-column tiles leave tensor memory for four CTAs per SM.
+    const bool short_k = p.K <= 4 * kBK;
     // 256-column tiles halve the B traffic per FLOP; used when they still
     // give every SM a tile
     const int bn = p.N <= 64 ? 64
-                   : (p.N > 128 && (long long)ceil_div(p.M, kBM) * ceil_div(p.N, 256) * splits >= 148)
+                   : (!short_k && p.N > 128 && (long long)ceil_div(p.M, kBM) * ceil_div(p.N, 256) * splits >= 148)
                        ? 256
                        : 128;
     // DGC_GEMM=cpasync selects the cp.async pipeline (also the fallback when
@@ -535,11 +629,13 @@ int tc_gemm(const GemmArgs& p, cudaStream_t s) {
         const bool two = bn == 256 &&
                          (long long)ceil_div(p.M, 2 * kBM) * ceil_div(p.N, 256) * splits >= 148;
         bool used = false;
-        int rc = bn == 64    ? launch_gemm_tma<64, 1>(p, s, &used)
-                 : two       ? launch_gemm_tma<256, 2>(p, s, &used)
-                 : bn == 256 ? launch_gemm_tma<256, 1>(p, s, &used)
-                             : launch_gemm_tma<128, 1>(p, s, &used);
+        const int rc = p.mn_major ? launch_gemm_tma_bn<true>(p, bn, two, s, &used)
+                                  : launch_gemm_tma_bn<false>(p, bn, two, s, &used);
         if (rc != DGC_OK || used) return rc;
+    }
+    if (p.mn_major) {
+        set_error("MN-major operands need the TMA pipeline");
+        return DGC_ERR_UNSUPPORTED;
     }
     if (bn == 64) return launch_gemm<64>(p, s);
     if (bn == 256) return launch_gemm<256>(p, s);

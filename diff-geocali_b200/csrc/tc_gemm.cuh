@@ -19,6 +19,7 @@ struct GemmArgs {
     float alpha;     // result = alpha * A B^T (+ bias)
     int* error;      // device word set to 1 when a pipeline wait times out
     int k_tiles_per_split;  // > 0: split K over gridDim.z CTAs, fp32 atomic epilogue
+    int mn_major = 0;       // A is [K][lda], B [K][ldb] (M and N contiguous)
 };
 
 int tc_gemm(const GemmArgs& p, cudaStream_t s);

@@ -96,8 +96,12 @@ SIGNATURES = {
     "dgc_bp_clear_tile_rules": (_I, []),
     "dgc_bp_tiles": (_I, [_I, _I] + [ctypes.POINTER(ctypes.c_int)] * 4),
     "dgc_gemm_bf16": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _P, _P]),
+    "dgc_gemm_bf16_tn": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _P, _P]),
     "dgc_im2col_nhwc_bf16": (_I, [_P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P]),
     "dgc_col2im_nhwc_f32": (_I, [_P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P]),
+    "dgc_col2im_nhwc_bf16": (_I, [_P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P]),
+    "dgc_relu_grad_workspace_bytes": (_S, [_I, _I]),
+    "dgc_relu_grad_bf16": (_I, [_P, _P, _I, _I, _P, _P, _P, _S, _P]),
     "dgc_preprocess": (_I, [_P, _P, _P, _I, _I, _I, _I, _F, _P, _P]),
     "dgc_batch_workspace_bytes": (_S, [ctypes.POINTER(FpInstance), _I]),
     "dgc_batch_prepare": (_I, [ctypes.POINTER(FpInstance), _I, _P, _S, ctypes.POINTER(BatchPlan),
@@ -114,6 +118,8 @@ SIGNATURES = {
     "dgc_ceiling_gather": (_I, [_P, _S, _I, _I, _I, _I, _P, ctypes.POINTER(_D), _P]),
     "dgc_ceiling_issue": (_I, [_I, _I, _P, ctypes.POINTER(_D), _P]),
 }
+
+ERR_UNSUPPORTED = 4  # DGC_ERR_UNSUPPORTED
 
 _lib = None
 _lock = threading.Lock()

@@ -37,6 +37,7 @@ angle 0.3 deg, source 1 mm, detector centre 2 mm, sid/sod 0.5 %.
 from __future__ import annotations
 
 import math
+import os
 import time
 from dataclasses import dataclass, replace
 
@@ -159,8 +160,31 @@ def gemm(A, B, bias=None, relu=False, out_bf16=False, out=None, accumulate=False
     return out
 
 
+def gemm_tn(A, B):
+    """out[m, n] = sum_k A[k, m] * B[k, n] in fp32: the product of two bf16 matrices
+    over their rows (a weight gradient), as they lie."""
+    K, M = A.shape
+    N = B.shape[1]
+    lib = _native.lib()
+    if os.environ.get("DGC_GEMM") != "cpasync" and A.stride(0) % 8 == 0 and B.stride(0) % 8 == 0:
+        out = torch.empty((M, N), device=A.device, dtype=torch.float32)
+        rc = lib.dgc_gemm_bf16_tn(
+            A.data_ptr(), B.data_ptr(), out.data_ptr(), M, N, K, A.stride(0), B.stride(0),
+            out.stride(0), 0, 1.0, _Scratch.flag(A.device).data_ptr(),
+            torch.cuda.current_stream(A.device).cuda_stream)
+        if rc != _native.ERR_UNSUPPORTED:
+            _native.check(rc)
+            return out
+    # without tensor maps or with rows off 16 bytes: transposed copies for the
+    # K-major product
+    Kp = _round8(K)
+    return gemm(_padded_t(A, Kp), _padded_t(B, Kp))
+
+
 def _padded_t(x, cols):
     """x.T as a contiguous bf16 [x.shape[1], cols] with zero columns beyond x.shape[0]."""
+    if x.shape[0] == cols:
+        return x.t().contiguous()
     out = torch.zeros((x.shape[1], cols), dtype=torch.bfloat16, device=x.device)
     out[:, : x.shape[0]] = x.t()
     return out
@@ -176,10 +200,28 @@ def _im2col(x, k, stride, pad, Kp):
     return col, Ho, Wo
 
 
+def _relu_grad(gy, y, relu):
+    """``(g, db)``: g = gy * (y > 0) (gy without ``relu``) in bf16 and its column sums."""
+    if gy.dtype != torch.bfloat16 or gy.shape[1] % 8 or gy.shape[1] > 2048:
+        g = (gy * (y > 0) if relu else gy).to(torch.bfloat16).contiguous()
+        return g, g.float().sum(0)
+    gy = gy.contiguous()
+    M, C = gy.shape
+    g = torch.empty_like(gy) if relu else gy
+    db = torch.empty(C, dtype=torch.float32, device=gy.device)
+    lib = _native.lib()
+    n = lib.dgc_relu_grad_workspace_bytes(M, C)
+    ws = torch.empty(n, dtype=torch.uint8, device=gy.device)
+    _native.check(lib.dgc_relu_grad_bf16(
+        gy.data_ptr(), y.data_ptr() if relu else None, M, C, g.data_ptr() if relu else None,
+        db.data_ptr(), ws.data_ptr(), n, torch.cuda.current_stream(gy.device).cuda_stream))
+    return g, db
+
+
 def _col2im(dcol, shape, k, stride, pad, Kp):
     B, H, W, C = shape
-    dx = torch.empty(shape, dtype=torch.float32, device=dcol.device)
-    _native.check(_native.lib().dgc_col2im_nhwc_f32(
+    dx = torch.empty(shape, dtype=torch.bfloat16, device=dcol.device)
+    _native.check(_native.lib().dgc_col2im_nhwc_bf16(
         dcol.data_ptr(), B, H, W, C, k, k, stride, pad, Kp, dx.data_ptr(),
         torch.cuda.current_stream(dcol.device).cuda_stream))
     return dx
@@ -202,26 +244,20 @@ class _Conv2d(torch.autograd.Function):
     def backward(ctx, gy):
         col, wb, y = ctx.saved_tensors
         xshape, k, stride, pad, relu, need_dx = ctx.cfg
-        g = gy.reshape(y.shape)
-        if relu:
-            g = g * (y > 0)
-        g = g.to(torch.bfloat16).contiguous()
+        g, db = _relu_grad(gy.reshape(y.shape), y, relu)
         M = g.shape[0]
-        Mp = _round8(M)
-        dw = gemm(_padded_t(g, Mp), _padded_t(col, Mp))          # [Cout, Kp] fp32
-        db = g.float().sum(0)
+        dw = gemm_tn(g, col)                                       # [Cout, Kp] fp32
         dx = None
         if need_dx:
             Cout = g.shape[1]
-            wt = torch.zeros((wb.shape[1], _round8(Cout)), dtype=torch.bfloat16, device=g.device)
-            wt[:, :Cout] = wb.t()
+            wt = _padded_t(wb, _round8(Cout))
             if Cout % 8:
                 gp = torch.zeros((M, _round8(Cout)), dtype=torch.bfloat16, device=g.device)
                 gp[:, :Cout] = g
             else:
                 gp = g
             dcol = gemm(gp, wt)                                    # [M, Kp] fp32
-            dx = _col2im(dcol, xshape, k, stride, pad, wb.shape[1]).to(torch.bfloat16)
+            dx = _col2im(dcol, xshape, k, stride, pad, wb.shape[1])
         return dx, dw, db, None, None, None, None
 
 
@@ -246,8 +282,7 @@ class _ViewConv(torch.autograd.Function):
         g = gy * (y > 0) if relu else gy
         g = g.to(torch.bfloat16).contiguous()
         A, Cout = g.shape
-        Ap = _round8(A)
-        dw = gemm(_padded_t(g, Ap), _padded_t(col, Ap))
+        dw = gemm_tn(g, col.contiguous())
         db = g.float().sum(0)
         wt = torch.zeros((wb.shape[1], _round8(Cout)), dtype=torch.bfloat16, device=g.device)
         wt[:, :Cout] = wb.t()

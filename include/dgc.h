@@ -400,6 +400,14 @@ int dgc_gemm_bf16(const void* A, const void* B, void* C, const float* bias, int 
                   int lda, int ldb, int ldc, int c_bf16, int relu, int accumulate, float alpha,
                   int* error_flag, void* stream);
 
+/* C[m, n] (+)= alpha * sum_k A[k, m] * B[k, n] for bf16 A [K][lda] and B [K][ldb]
+ * (M and N contiguous: operands that a weight gradient reduces over their rows),
+ * fp32 C [M][ldc].  lda, ldb multiples of 8, A and B 16-byte aligned; needs the
+ * TMA pipeline (DGC_ERR_UNSUPPORTED without it).  No counterpart in the
+ * reference. */
+int dgc_gemm_bf16_tn(const void* A, const void* B, float* C, int M, int N, int K, int lda, int ldb,
+                     int ldc, int accumulate, float alpha, int* error_flag, void* stream);
+
 /* Scratch of dgc_project_mse_grad. */
 size_t dgc_project_mse_grad_workspace_bytes(int D, int H, int W, int A, int U, int V);
 
@@ -514,6 +522,19 @@ int dgc_im2col_nhwc_bf16(const void* x, int B, int H, int W, int C, int kh, int 
  * No counterpart in the reference. */
 int dgc_col2im_nhwc_f32(const float* col, int B, int H, int W, int C, int kh, int kw, int stride,
                         int pad, int Kp, float* dx, void* stream);
+
+/* The same, rounded to bf16 (dx: bf16 [B][H][W][C]). */
+int dgc_col2im_nhwc_bf16(const float* col, int B, int H, int W, int C, int kh, int kw, int stride,
+                         int pad, int Kp, void* dx, void* stream);
+
+/* Scratch of dgc_relu_grad_bf16. */
+size_t dgc_relu_grad_workspace_bytes(int M, int C);
+
+/* g = gy * (y > 0) for bf16 [M][C] (y NULL: g is gy and not written) and the fp32
+ * column sums db [C] of g; C a multiple of 8 up to 2048, 16-byte aligned arrays.
+ * No counterpart in the reference. */
+int dgc_relu_grad_bf16(const void* gy, const void* y, int M, int C, void* g, float* db,
+                       void* workspace, size_t workspace_bytes, void* stream);
 
 /* ---------------------------------------------------------------------- */
 /* Kernel timing (no counterpart in the reference; measurement support)     */

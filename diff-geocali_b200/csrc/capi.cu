@@ -208,7 +208,8 @@ static int project_impl(const float* volume, int D, int H, int W, const Geometry
     rc = arm.arm == 2 ? build_volume_pairs(volume, D, H, W, reinterpret_cast<float2*>(quads), s)
                       : build_volume_quads(volume, D, H, W, quads, s);
     if (rc != DGC_OK) return rc;
-    DGC_CUDA(cudaMemsetAsync(status, 0, sizeof(int), s));
+    // the status word belongs to the TMA arm's bounded waits
+    if (arm.arm == 1) DGC_CUDA(cudaMemsetAsync(status, 0, sizeof(int), s));
     return fp_launch_forward(p, kForwardTile, arm, s);
 }
 

@@ -74,7 +74,7 @@ def fp_forward(volume, angles, sid, sod, det_u0_arr, det_v0_arr, src_x_arr, src_
     geom = [t.contiguous() for t in geometry]
     D, H, W = vol.shape
     _require(D > 0 and H > 0 and W > 0, "every volume dimension must be positive")
-    out = torch.zeros((A, U, V), dtype=torch.float32, device=vol.device)
+    out = torch.empty((A, U, V), dtype=torch.float32, device=vol.device)
     lib = _native.lib()
     with torch.cuda.device(vol.device):
         ws = _workspace(lib.dgc_project_workspace_bytes(D, H, W, A, U, V), vol.device)
@@ -111,7 +111,7 @@ def fp_backward(grad_projection, volume, angles, sid, sod, det_u0_arr, det_v0_ar
     _require(D > 0 and H > 0 and W > 0, "every volume dimension must be positive")
     dev = vol.device
     compute = bool(compute_grad_volume)
-    grad_volume = torch.zeros_like(vol) if compute else torch.empty(0, dtype=vol.dtype, device=dev)
+    grad_volume = torch.empty_like(vol) if compute else torch.empty(0, dtype=vol.dtype, device=dev)
     lib = _native.lib()
     if compute and not compute_grad_geometry:
         with torch.cuda.device(dev):
@@ -121,7 +121,7 @@ def fp_backward(grad_projection, volume, angles, sid, sod, det_u0_arr, det_v0_ar
                 step_size, voxel_size, float(off_x), float(off_y), float(off_z),
                 grad_volume.data_ptr(), _p(ws), 0 if ws is None else ws.numel(), _stream(dev)))
         return [grad_volume, *[None] * 8]
-    grads = [torch.zeros_like(g) for g in geom]
+    grads = [torch.empty_like(g) for g in geom]
     with torch.cuda.device(dev):
         ws = _workspace(lib.dgc_project_backward_workspace_bytes(D, H, W, A, U, V, int(compute)), dev)
         _native.check(lib.dgc_project_backward(
@@ -217,7 +217,7 @@ def bp_forward(proj, angles, sid, sod, det_u0_arr, det_v0_arr, src_x_arr, src_y_
     geom = [t.contiguous() for t in geometry]
     A, U, V = p.shape
     dev = p.device
-    vol = torch.zeros((D, H, W), dtype=torch.float32, device=dev)
+    vol = torch.empty((D, H, W), dtype=torch.float32, device=dev)
     lib = _native.lib()
     with torch.cuda.device(dev):
         ws = _workspace(lib.dgc_backproject_workspace_bytes(A, U, V, D, H, W), dev)
@@ -262,7 +262,7 @@ def bp_backward(grad_vol, proj, angles, sid, sod, det_u0_arr, det_v0_arr, src_x_
                 voxel_size, off_x, off_y, off_z, grad_proj.data_ptr(), _p(ws),
                 0 if ws is None else ws.numel(), _stream(dev)))
         return [grad_proj, *[None] * 8]
-    grads = [torch.zeros_like(g) for g in geom]
+    grads = [torch.empty_like(g) for g in geom]
     with torch.cuda.device(dev):
         ws = _workspace(lib.dgc_backproject_backward_workspace_bytes(A, U, V, D, H, W), dev)
         _native.check(lib.dgc_backproject_backward(

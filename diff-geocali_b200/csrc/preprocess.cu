@@ -60,10 +60,55 @@ __global__ void preprocess_auv_kernel(const float* __restrict__ raw, const float
     }
 }
 
+// Bit i of *faults: array i holds a value that is not finite; bit 16 + i: one that
+// is <= 0.  One block: the arrays hold one value per view.
+struct ValueArrays {
+    const float* data[DGC_CHECK_MAX_ARRAYS];
+    int count[DGC_CHECK_MAX_ARRAYS];
+    int n;
+};
+
+__global__ void __launch_bounds__(256) check_values_kernel(ValueArrays v, int* __restrict__ faults) {
+    __shared__ int s_faults;
+    if (threadIdx.x == 0) s_faults = 0;
+    __syncthreads();
+    int mine = 0;
+    for (int k = 0; k < v.n; ++k) {
+        const float* __restrict__ x = v.data[k];
+        for (int i = threadIdx.x; i < v.count[k]; i += 256) {
+            if (!isfinite(x[i])) mine |= 1 << k;
+            if (x[i] <= 0.0f) mine |= 1 << (16 + k);
+        }
+    }
+    if (mine) atomicOr(&s_faults, mine);
+    __syncthreads();
+    if (threadIdx.x == 0) *faults = s_faults;
+}
+
 }  // namespace
 }  // namespace dgc
 
 using namespace dgc;
+
+extern "C" int dgc_check_values(const float* const* arrays, const int* counts, int n, int* faults,
+                                void* stream) {
+    clear_error();
+    DGC_REQUIRE(arrays && counts && faults, "arrays, counts and faults must be non-null");
+    DGC_REQUIRE(n >= 1 && n <= DGC_CHECK_MAX_ARRAYS, "one to sixteen arrays");
+    ValueArrays v;
+    memset(&v, 0, sizeof(v));
+    v.n = n;
+    for (int k = 0; k < n; ++k) {
+        DGC_REQUIRE(arrays[k] && counts[k] >= 1, "every array must be non-null and non-empty");
+        v.data[k] = arrays[k];
+        v.count[k] = counts[k];
+    }
+    cudaStream_t s = (cudaStream_t)stream;
+    DGC_TRACE("check_values", s);
+    check_values_kernel<<<1, 256, 0, s>>>(v, faults);
+    DGC_LAUNCH_CHECK("check_values");
+    return DGC_OK;
+}
 
 extern "C" int dgc_preprocess(const float* raw, const float* dark, const float* flat, int A, int U,
                               int V, int layout_avu, float min_ratio, float* out, void* stream) {

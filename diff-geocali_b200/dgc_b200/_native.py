@@ -102,6 +102,7 @@ SIGNATURES = {
     "dgc_col2im_nhwc_bf16": (_I, [_P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P]),
     "dgc_relu_grad_workspace_bytes": (_S, [_I, _I]),
     "dgc_relu_grad_bf16": (_I, [_P, _P, _I, _I, _P, _P, _P, _S, _P]),
+    "dgc_check_values": (_I, [ctypes.POINTER(_P), ctypes.POINTER(_I), _I, _P, _P]),
     "dgc_preprocess": (_I, [_P, _P, _P, _I, _I, _I, _I, _F, _P, _P]),
     "dgc_batch_workspace_bytes": (_S, [ctypes.POINTER(FpInstance), _I]),
     "dgc_batch_prepare": (_I, [ctypes.POINTER(FpInstance), _I, _P, _S, ctypes.POINTER(BatchPlan),

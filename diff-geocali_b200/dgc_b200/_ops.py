@@ -13,6 +13,7 @@ there is no other code path.
 
 from __future__ import annotations
 
+import ctypes
 import math
 
 import torch
@@ -273,6 +274,23 @@ def bp_backward(grad_vol, proj, angles, sid, sod, det_u0_arr, det_v0_arr, src_x_
 
 
 # ------------------------------------------------------------------------- FDK
+
+
+def value_faults(tensors):
+    """``[(has a value that is not finite, has one <= 0)]`` of up to sixteen float32
+    tensors on one device: on a GPU one launch and one read (dgc_check_values)."""
+    if not all(t.is_cuda and t.numel() for t in tensors):
+        return [(not bool(torch.isfinite(t).all()), bool((t <= 0).any())) for t in tensors]
+    tensors = [t.detach().contiguous() for t in tensors]
+    dev, n = tensors[0].device, len(tensors)
+    faults = torch.empty(1, dtype=torch.int32, device=dev)
+    arrays = (ctypes.c_void_p * n)(*[t.data_ptr() for t in tensors])
+    counts = (ctypes.c_int * n)(*[t.numel() for t in tensors])
+    with torch.cuda.device(dev):
+        _native.check(_native.lib().dgc_check_values(arrays, counts, n, faults.data_ptr(),
+                                                     _stream(dev)))
+    mask = faults.item()
+    return [(bool(mask >> i & 1), bool(mask >> (16 + i) & 1)) for i in range(n)]
 
 
 def fdk_filter(projections, pixel_size, sod, sid, alpha):

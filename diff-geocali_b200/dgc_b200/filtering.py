@@ -53,22 +53,9 @@ def _check_alpha(alpha):
     return alpha
 
 
-def _per_view_distance(name, value, projections):
-    """A scalar or one value per view, as a float32 [A] tensor on the projections' device."""
-    distance = torch.as_tensor(value, dtype=projections.dtype, device=projections.device)
-    distance = distance.reshape(-1)
-    views = projections.shape[0]
-    if distance.numel() == 1:
-        distance = distance.expand(views)
-    elif distance.numel() != views:
-        raise ValueError(f"{name} must be a scalar or have one value per view")
-    if not bool(torch.isfinite(distance).all()) or bool((distance <= 0).any()):
-        raise ValueError(f"{name} must contain finite positive distances")
-    return distance.contiguous()
-
-
-def _per_view_value(name, value, projections):
-    """A finite scalar or one value per view, as a float32 [A] tensor on the projections' device."""
+def _per_view(name, value, projections):
+    """A scalar or one value per view, as a contiguous float32 [A] tensor on the
+    projections' device."""
     values = torch.as_tensor(value, dtype=projections.dtype, device=projections.device)
     values = values.reshape(-1)
     views = projections.shape[0]
@@ -76,21 +63,48 @@ def _per_view_value(name, value, projections):
         values = values.expand(views)
     elif values.numel() != views:
         raise ValueError(f"{name} must be a scalar or have one value per view")
-    if not bool(torch.isfinite(values).all()):
-        raise ValueError(f"{name} must contain finite values")
     return values.contiguous()
 
 
-def _check_frame(frame, projections):
-    """``frame = (dist, u, v)`` with None entries as float32 [A] tensors (or None)."""
-    if frame is None:
-        return (None, None, None)
-    if not isinstance(frame, (tuple, list)) or len(frame) != 3:
-        raise TypeError("frame must be a (dist, u, v) triple")
-    dist, u, v = frame
-    return (None if dist is None else _per_view_distance("frame dist", dist, projections),
-            None if u is None else _per_view_value("frame u", u, projections),
-            None if v is None else _per_view_value("frame v", v, projections))
+def _check_per_view(checks):
+    """Raises for the first of ``[(name, values, positive)]`` that holds a value
+    that is not finite (or, where ``positive``, not above zero)."""
+    if not checks:
+        return
+    faults = _ops.value_faults([values for _, values, _ in checks])
+    for (name, _, positive), (not_finite, not_positive) in zip(checks, faults):
+        if positive and (not_finite or not_positive):
+            raise ValueError(f"{name} must contain finite positive distances")
+        if not_finite:
+            raise ValueError(f"{name} must contain finite values")
+
+
+def _distances_and_frame(projections, sod, sid, frame):
+    """The filter's per-view arguments as float32 [A] tensors (None frame entries
+    kept), their values checked together: one read for all of them."""
+    checks = []
+
+    def take(name, value, positive):
+        if value is None:
+            return None
+        values = _per_view(name, value, projections)
+        checks.append((name, values, positive))
+        return values
+
+    try:
+        sod, sid = take("sod", sod, True), take("sid", sid, True)
+        if frame is None:
+            frame = (None, None, None)
+        elif not isinstance(frame, (tuple, list)) or len(frame) != 3:
+            raise TypeError("frame must be a (dist, u, v) triple")
+        dist, u, v = frame
+        frame = (take("frame dist", dist, True), take("frame u", u, False),
+                 take("frame v", v, False))
+    except Exception:
+        _check_per_view(checks)  # a fault of an earlier argument comes first
+        raise
+    _check_per_view(checks)
+    return sod, sid, frame
 
 
 def preweight_frame(angles, sid, sod, det_u0, det_v0, src_x, src_y, src_z, pixel_size):
@@ -171,9 +185,7 @@ def fdk_filter(projections, pixel_size, sod, sid, alpha=0.8, *, frame=None):
     _check_projections(projections)
     pixel_size = _positive_scalar("pixel_size", pixel_size)
     alpha = _check_alpha(alpha)
-    sod = _per_view_distance("sod", sod, projections)
-    sid = _per_view_distance("sid", sid, projections)
-    frame = _check_frame(frame, projections)
+    sod, sid, frame = _distances_and_frame(projections, sod, sid, frame)
     if not projections.is_cuda:
         raise ValueError("fdk_filter requires CUDA projections (there is no CPU path)")
     framed = any(t is not None for t in frame)
@@ -191,7 +203,6 @@ def _fdk_arguments(projections, geometry, pixel_size, volume_shape, voxel_size, 
     (filtering.py:107-198) on one rank's views; returns (pixel_size,
     volume_shape, voxel_size, offset, alpha)."""
     _check_projections(projections)
-    sid, sod = geometry[1], geometry[2]
     if min(projections.shape[1:]) < 2:
         raise ValueError("reconstruct_fdk requires detector dimensions U and V >= 2")
     views = projections.shape[0]
@@ -203,9 +214,10 @@ def _fdk_arguments(projections, geometry, pixel_size, volume_shape, voxel_size, 
             raise ValueError(f"{name} must have shape [{views}]")
         if t.dtype != projections.dtype or t.device != projections.device:
             raise ValueError(f"{name} must match the projections' dtype and device")
-    if not bool(torch.isfinite(torch.stack(geometry)).all()):
+    faults = _ops.value_faults(geometry)
+    if any(not_finite for not_finite, _ in faults):
         raise ValueError("geometry must contain only finite values")
-    if bool((sid <= 0).any()) or bool((sod <= 0).any()):
+    if faults[1][1] or faults[2][1]:
         raise ValueError("sid and sod must contain positive distances")
     pixel_size = _positive_scalar("pixel_size", pixel_size)
     voxel_size = _positive_scalar("voxel_size", voxel_size)
@@ -279,25 +291,29 @@ def reconstruct_fdk(
         projections, geometry, pixel_size, volume_shape, voxel_size, volume_offset, alpha,
         angle_chunk_size)
     views = projections.shape[0]
-    frame = None
-    if offset_preweight:
-        frame = preweight_frame(*geometry, pixel_size)
-        if bool((frame[0] <= 0).any()):
-            raise ValueError("the source must lie in front of the detector plane")
+    frame = preweight_frame(*geometry, pixel_size) if offset_preweight else None
+    # what the host needs of the scan, in one read
+    wanted = [] if frame is None else [frame[0]]
+    if short_scan:
+        wanted += [angles, sid] if frame is None else [angles, frame[1]]
+    host = torch.stack(wanted).cpu() if wanted else None
+    if frame is not None and bool((host[0] <= 0).any()):
+        raise ValueError("the source must lie in front of the detector plane")
     U = projections.shape[1]
     if short_scan:
-        a0, a1 = float(angles[0]), float(angles[-1])
+        scan = host[-2]
+        a0, a1 = float(scan[0]), float(scan[-1])
         span = abs(a1 - a0)
         if frame is None:
-            fan = math.atan(((U - 1) / 2 * pixel_size) / float(sid.min()))
+            fan = math.atan(((U - 1) / 2 * pixel_size) / float(host[-1].min()))
         else:
-            reach = torch.maximum(frame[1], (U - 1) - frame[1]) * pixel_size
-            fan = float(torch.atan(reach / frame[0]).max())
+            reach = torch.maximum(host[-1], (U - 1) - host[-1]) * pixel_size
+            fan = float(torch.atan(reach / host[0]).max())
         if views < 2 or span < math.pi + 2 * fan - 1e-6:
             raise ValueError("a short scan must cover pi plus twice the largest fan angle "
                              f"({math.degrees(math.pi + 2 * fan):.2f} deg); got "
                              f"{math.degrees(span):.2f} deg")
-        steps = torch.diff(angles.double()) * (1.0 if a1 >= a0 else -1.0)
+        steps = torch.diff(scan.double()) * (1.0 if a1 >= a0 else -1.0)
         if bool((steps <= 0).any()):
             raise ValueError("short-scan angles must be strictly monotone")
         if frame is None:

@@ -436,6 +436,16 @@ int dgc_project_mse_grad(const float* volume, int D, int H, int W,
 /* Raw frames to line integrals                                             */
 /* ---------------------------------------------------------------------- */
 
+#define DGC_CHECK_MAX_ARRAYS 16
+
+/* Validity of up to DGC_CHECK_MAX_ARRAYS device arrays (host pointers to the array
+ * of device pointers and their counts) in one launch: bit i of *faults (a device
+ * word) is set if array i holds a value that is not finite, bit 16 + i if it
+ * holds one <= 0.  The checks of filtering.py:33-51 and 134-145, which the
+ * reference makes one torch reduction and host read at a time. */
+int dgc_check_values(const float* const* arrays, const int* counts, int n, int* faults,
+                     void* stream);
+
 /* out[a,u,v] = -log(max((raw - dark) / (flat - dark), min_ratio)), the
  * dark/flat-field correction and negative log the reference requires
  * upstream of its operators (README.md:108), fused with the transpose of

@@ -585,10 +585,19 @@ int dgc_fdk_filter_taps(int U, double pixel_size, double alpha, double* taps) {
 }
 
 size_t dgc_fdk_filter_workspace_bytes(int A, int U, int V) {
-    (void)A;
-    (void)V;
     if (U <= 0) return 0;
-    return Workspace::align(sizeof(float) * (size_t)U);
+    return Workspace::align(sizeof(float) * (size_t)U) + fdk_tc_bytes(A, U, V, false);
+}
+
+// The filter of every view: on the tensor cores where the sizes are theirs and
+// the workspace holds their scratch, else the FP32 product.
+static int run_filter(const FdkArgs& f, const Workspace& scratch, cudaStream_t s) {
+    if (f.A <= 65535) {
+        bool used = false;
+        const int rc = fdk_tc_filter(f, false, scratch, s, &used);
+        if (rc != DGC_OK || used) return rc;
+    }
+    return fdk_launch_filter(f, s);
 }
 
 static int check_fdk(int A, int U, int V, float pixel_size, float alpha) {
@@ -620,7 +629,7 @@ int dgc_fdk_filter_ex(const float* projections, int A, int U, int V, float pixel
     f.frame_dist = frame_dist;
     f.frame_u = frame_u;
     f.frame_v = frame_v;
-    return fdk_launch_filter(f, s);
+    return run_filter(f, ws, s);
 }
 
 int dgc_fdk_filter(const float* projections, int A, int U, int V, float pixel_size,
@@ -634,7 +643,8 @@ size_t dgc_fdk_filter_backward_workspace_bytes(int A, int U, int V) {
     if (A <= 0 || U <= 0 || V <= 0) return 0;
     return Workspace::align(sizeof(float) * (size_t)U) +
            Workspace::align(sizeof(double) * kFdkPartials * (size_t)A *
-                            (size_t)fdk_filter_tiles(U, V));
+                            (size_t)fdk_filter_tiles(U, V)) +
+           fdk_tc_bytes(A, U, V, true);
 }
 
 int dgc_fdk_filter_backward_ex(const float* grad_filtered, const float* projections,
@@ -675,7 +685,9 @@ int dgc_fdk_filter_backward_ex(const float* grad_filtered, const float* projecti
     f.frame_u = frame_u;
     f.frame_v = frame_v;
     f.frame_grads = (grad_frame_u || grad_frame_v) ? 1 : 0;
-    if ((rc = fdk_launch_filter_adjoint(f, s)) != DGC_OK) return rc;
+    bool used = false;
+    if (A <= 65535 && (rc = fdk_tc_filter(f, true, ws, s, &used)) != DGC_OK) return rc;
+    if (!used && (rc = fdk_launch_filter_adjoint(f, s)) != DGC_OK) return rc;
     if (!dist) return DGC_OK;
     const FdkGrads g{grad_sod, grad_sid, grad_frame_dist, grad_frame_u, grad_frame_v};
     return fdk_reduce_distance_grads(partials, A, tiles, f, g, s);
@@ -694,9 +706,13 @@ int dgc_fdk_filter_backward(const float* grad_filtered, const float* projections
 
 size_t dgc_reconstruct_fdk_workspace_bytes(int A, int U, int V, int D, int H, int W) {
     if (A <= 0 || U < 2 || V < 2) return 0;
-    return dgc_fdk_filter_workspace_bytes(A, U, V) +
-           Workspace::align(sizeof(float) * (size_t)A * U * V) +
-           dgc_backproject_workspace_bytes(A, U, V, D, H, W);
+    // the filter's scratch is done with before the quads are built in its place
+    (void)D;
+    (void)H;
+    (void)W;
+    return Workspace::align(sizeof(float) * (size_t)U) +
+           Workspace::align(sizeof(float) * (size_t)A * U * V) + bp_table_bytes(A) +
+           std::max(bp_quads_bytes(A, U, V), fdk_tc_bytes(A, U, V, false));
 }
 
 static int reconstruct_fdk_impl(const float* projections, int A, int U, int V,
@@ -721,6 +737,7 @@ static int reconstruct_fdk_impl(const float* projections, int A, int U, int V,
     float* taps = ws.take<float>((size_t)U);
     float* filtered = ws.take<float>((size_t)A * U * V);
     ViewRow* vt = ws.take<ViewRow>((size_t)A);
+    const Workspace filter_scratch = ws;  // shares its memory with the quads
     float4* pq = ws.take<float4>((size_t)A * (U - 1) * (V - 1));
     if (!taps || !filtered || !vt || !pq) {
         set_error("workspace too small: dgc_reconstruct_fdk needs " +
@@ -732,7 +749,7 @@ static int reconstruct_fdk_impl(const float* projections, int A, int U, int V,
     f.frame_dist = frame_dist;
     f.frame_u = frame_u;
     f.frame_v = frame_v;
-    if ((rc = fdk_launch_filter(f, s)) != DGC_OK) return rc;
+    if ((rc = run_filter(f, filter_scratch, s)) != DGC_OK) return rc;
     if ((rc = bp_view_table(g, A, vt, s)) != DGC_OK) return rc;
     if ((rc = build_proj_quads(filtered, A, U, V, pq, s)) != DGC_OK) return rc;
     BpArgs p = bp_args(vt, pq, A, U, V, D, H, W, pixel_size, voxel_size, off_x, off_y, off_z);

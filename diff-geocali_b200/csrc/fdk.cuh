@@ -34,6 +34,9 @@ struct FdkArgs {
     int frame_grads = 0;  // adjoint: also the sums for the frame-centre gradients
 };
 
+// The FP32 product's tiles; the adjoint's sums are kept per tile.
+constexpr int kFdkTileRows = 128, kFdkTileColumns = 128;
+
 // FP64 sums per (view, tile) of the adjoint: g*y, H(g) P dw/ddist,
 // H(g) P u_c/|r|^3, H(g) P v_c/|r|^3 (u_c, v_c in length units).
 constexpr int kFdkPartials = 4;
@@ -45,6 +48,12 @@ int fdk_launch_filter(const FdkArgs& p, cudaStream_t s);
 // g*y and H(g)*P*dw/dsid (partials), then dgc's distance gradients from them.
 long long fdk_filter_tiles(int U, int V);
 int fdk_launch_filter_adjoint(const FdkArgs& p, cudaStream_t s);
+// The filter's product on the tensor cores (fdk_tc.cu): views held at a time (0:
+// the sizes are not its), scratch, and the filter or the adjoint with its sums;
+// *used false: nothing was done.
+int fdk_tc_views(int A, int U, int V);
+size_t fdk_tc_bytes(int A, int U, int V, bool adjoint);
+int fdk_tc_filter(const FdkArgs& p, bool adjoint, Workspace ws, cudaStream_t s, bool* used);
 // Per-view gradients from the partials: sod, sid, and, where the frame was
 // given, its distance and centres (any output may be null).
 struct FdkGrads {

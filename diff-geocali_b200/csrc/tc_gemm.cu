@@ -33,6 +33,7 @@
 
 #include "common.cuh"
 #include "tc_gemm.cuh"
+#include "tcgen05.cuh"
 #include "tma.cuh"
 
 namespace dgc {
@@ -55,7 +56,6 @@ namespace {
 constexpr int kBM = 128;
 constexpr int kBK = 64;
 constexpr int kStages = 4;
-constexpr long long kWaitLimit = 1LL << 26;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -78,101 +78,17 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count) : "memory");
 }
 
-// Bounded wait for the phase with the given parity; false on timeout.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (long long i = 0; i < kWaitLimit; ++i) {
-        uint32_t done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            " selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-
-// Shared-memory matrix descriptor, K-major, 128-byte swizzle (sm_100 format:
-// start >> 4 in [0,14), LBO >> 4 in [16,30) (16 B, unused by swizzled
-// K-major), SBO >> 4 in [32,46) (1024 B between 8-row groups), version 1 at
-// bit 46, base offset 0 (atoms 1024-byte aligned), layout type 2 =
-// SWIZZLE_128B in [61,64)).
+// K-major operand with 128-byte swizzle: SBO = 1024 B between 8-row groups (LBO is
+// unused by swizzled K-major).
 __device__ __forceinline__ uint64_t kmajor_sw128_desc(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((saddr >> 4) & 0x3FFFu);
-    d |= static_cast<uint64_t>(16u >> 4) << 16;
-    d |= static_cast<uint64_t>(1024u >> 4) << 32;
-    d |= static_cast<uint64_t>(1) << 46;
-    d |= static_cast<uint64_t>(2) << 61;
-    return d;
+    return smem_desc(saddr, 16u, 1024u, 2u);
 }
 
 // The same for MN-major operands staged as boxes of 64 (M or N) x kBK (K): a K row
 // is 128 contiguous bytes; SBO = 1024 B between groups of 8 K rows, LBO = one
 // box (kBK * 128 B) between groups of 64 M or N.
 __device__ __forceinline__ uint64_t mnmajor_sw128_desc(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((saddr >> 4) & 0x3FFFu);
-    d |= static_cast<uint64_t>((kBK * 128u) >> 4) << 16;
-    d |= static_cast<uint64_t>(1024u >> 4) << 32;
-    d |= static_cast<uint64_t>(1) << 46;
-    d |= static_cast<uint64_t>(2) << 61;
-    return d;
-}
-
-// Instruction descriptor of kind::f16 with bf16 A and B, fp32 D; both K-major, or
-// with MN both MN-major (bits 15 and 16).
-template <bool MN = false>
-__host__ __device__ constexpr uint32_t idesc_bf16(int m, int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (MN ? 3u << 15 : 0u) |
-           (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
-}
-
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                          uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                     bar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() {
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_load16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
-        "[%16];\n"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-          "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// 32 bytes to a 32-byte aligned global address.
-__device__ __forceinline__ void store32(void* p, const uint32_t (&v)[8]) {
-    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(
-                     __cvta_generic_to_global(p)),
-                 "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]),
-                 "r"(v[7])
-                 : "memory");
+    return smem_desc(saddr, kBK * 128u, 1024u, 2u);
 }
 
 // Stage one K-slice: 'rows' x 64 bf16 of a K-major matrix into the 128-byte
@@ -285,13 +201,7 @@ __global__ void __launch_bounds__(128) tc_gemm_kernel(GemmArgs p) {
     const int nk = split ? max(0, min(p.k_tiles_per_split, nk_total - kt0)) : nk_total;
     const int k_base = kt0 * kBK;
 
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
-                         smem_u32(&tmem_slot)),
-                     "r"(BN)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-    }
+    if (warp == 0) tmem_alloc(smem_u32(&tmem_slot), BN);
     if (threadIdx.x == 0) {
         for (int s = 0; s <= kStages; ++s) mbar_init(smem_u32(&bars[s]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -358,8 +268,7 @@ __global__ void __launch_bounds__(128) tc_gemm_kernel(GemmArgs p) {
     __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(BN)
-                     : "memory");
+        tmem_free(tmem, BN);
     }
 }
 
@@ -411,7 +320,7 @@ __global__ void __launch_bounds__(128) tc_gemm_tma_kernel(const __grid_constant_
     constexpr int kABytes = MSUB * kBM * kBK * 2;
     constexpr int kStageBytes = TmaStages<BN, MSUB>::kStageBytes;
     constexpr int kCols = MSUB * BN;  // tensor-memory columns of the accumulators
-    constexpr uint32_t kIdesc = idesc_bf16<MN>(kBM, BN);
+    constexpr uint32_t kIdesc = idesc_bf16(kBM, BN, MN, MN);
     constexpr uint32_t kBox = 64 * kBK * 2;  // bytes of an MN-major box
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[S];
@@ -428,13 +337,7 @@ __global__ void __launch_bounds__(128) tc_gemm_tma_kernel(const __grid_constant_
     const int kt0 = split ? blockIdx.z * p.k_tiles_per_split : 0;
     const int nk = split ? max(0, min(p.k_tiles_per_split, nk_total - kt0)) : nk_total;
 
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
-                         smem_u32(&tmem_slot)),
-                     "r"(kCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-    }
+    if (warp == 0) tmem_alloc(smem_u32(&tmem_slot), kCols);
     if (threadIdx.x == 0) {
         for (int i = 0; i < S; ++i) {
             mbar_init(smem_u32(&full[i]), 1);
@@ -527,8 +430,7 @@ __global__ void __launch_bounds__(128) tc_gemm_tma_kernel(const __grid_constant_
     __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kCols)
-                     : "memory");
+        tmem_free(tmem, kCols);
     }
 }
 

@@ -1,0 +1,145 @@
+"""The FDK filter's product on the tensor cores against 64-bit arithmetic.
+
+Tolerances, with S = sum_k |h[|u-k|] w[k]|, the sum of magnitudes at an output, and
+e = 2^-24: rounded inputs 4 e S (weight and taps); the leading product, per 32 taps
+two matrix instructions that each truncate 17 aligned addends, at most 34 e S; U/32
+<= 64 FP32 additions, 64 e S; the other products, 2^-8 of it, in one truncating
+accumulator of 5 U/16 <= 640 instructions, 2 * 640 * 2^-8 e S; the products left out,
+3 e S.  Together below 128 e S at an output.  For white noise the errors of the terms
+are independent and the sums of magnitudes are not reached: relative L2 error 2^-20,
+below what the smallest product kept (2^-16 of the leading one) would leave.
+"""
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a GPU")]
+
+E = 2.0**-24
+
+
+def scan(A, U, V, seed):
+    g = torch.Generator().manual_seed(seed)
+    p = torch.randn((A, U, V), generator=g).cuda()
+    sid = (1000 + 5 * torch.randn(A, generator=g)).cuda()
+    sod = (600 + 5 * torch.randn(A, generator=g)).cuda()
+    return p, sid, sod
+
+
+def toeplitz(U, px, alpha):
+    from dgc_b200 import _ops
+
+    h = torch.tensor(np.asarray(_ops.fdk_filter_taps(U, px, alpha)), dtype=torch.float64).cuda()
+    i = torch.arange(U, device="cuda")
+    return h[(i[:, None] - i[None]).abs()]
+
+
+def weights(p, px, dist, cu, cv):
+    A, U, V = p.shape
+    u = (torch.arange(U, device="cuda", dtype=torch.float64)[None] - cu.double()[:, None]) * px
+    v = (torch.arange(V, device="cuda", dtype=torch.float64)[None] - cv.double()[:, None]) * px
+    d = dist.double()[:, None, None]
+    return d / (d * d + u[:, :, None] ** 2 + v[:, None, :] ** 2).sqrt()
+
+
+def close(got, want, magnitudes):
+    assert torch.isfinite(got).all()
+    assert float(((got.double() - want).abs() - 128 * E * magnitudes).max()) <= 0
+    assert float((got.double() - want).norm() / want.norm()) <= 2.0**-20
+
+
+# edges: 96 rows is the first size; a row tile (128) and one more or less; a column
+# tile (256), two, ragged ones; rows that are not 8-element multiples; 2048 rows the
+# last, 2049 the FP32 product's
+SIZES = [(2, 96, 16), (1, 97, 17), (3, 127, 255), (2, 128, 256), (2, 129, 257), (5, 192, 40),
+         (1, 187, 521), (2, 768, 100), (1, 2048, 24), (1, 2049, 24)]
+
+
+@pytest.mark.parametrize("A,U,V", SIZES)
+def test_filter_and_adjoint_match_64_bits(A, U, V):
+    from dgc_b200 import _ops
+
+    px, alpha = 0.9, 0.8
+    p, sid, sod = scan(A, U, V, U + V)
+    H = toeplitz(U, px, alpha)
+    w = weights(p, px, sid, torch.full_like(sid, (U - 1) / 2), torch.full_like(sid, (V - 1) / 2))
+    c = px * (sid / sod).double()[:, None, None]
+    y = _ops.fdk_filter(p, px, sod, sid, alpha)
+    close(y, c * (H @ (w * p.double())), c * (H.abs() @ (w * p.double()).abs()))
+    g = torch.randn(p.shape, generator=torch.Generator().manual_seed(1)).cuda()
+    gp, gsod, gsid = _ops.fdk_filter_backward(g, p, y, px, sod, sid, alpha)
+    z = H @ g.double()
+    close(gp, c * w * z, c * w * (H.abs() @ g.double().abs()))
+    # y = c H(w P): dy/dsod = -y/sod; dy/dsid = y/sid + c H(P dw/dsid), dw/dsid = w r2/(sid dist^2)
+    s, o = sid.double(), sod.double()
+    gy = (g.double() * y.double()).flatten(1)
+    dw = w * (1 - w * w) / s[:, None, None]
+    zp = (c * z * p.double() * dw).flatten(1)
+    # magnitudes of the summed terms; each carries the error of its y or z, by the L2 bound
+    scale = gy.abs().sum(1) / o
+    assert float(((gsod.double() + gy.sum(1) / o).abs() - 2.0**-20 * scale).max()) <= 0
+    scale = gy.abs().sum(1) / s + zp.abs().sum(1)
+    assert float(((gsid.double() - gy.sum(1) / s - zp.sum(1)).abs() - 2.0**-20 * scale).max()) <= 0
+
+
+def test_frames():
+    from dgc_b200 import _ops
+
+    A, U, V, px, alpha = 3, 160, 130, 1.1, 0.9
+    p, sid, sod = scan(A, U, V, 3)
+    dist, cu, cv = sid * 0.98, torch.tensor([70.0, 79.5, 90.0]).cuda(), torch.tensor([60.0, 64.5, 71.0]).cuda()
+    y = _ops.fdk_filter_framed(p, px, sod, sid, alpha, (dist, cu, cv))
+    H = toeplitz(U, px, alpha)
+    w = weights(p, px, dist, cu, cv)
+    c = px * (sid / sod).double()[:, None, None]
+    close(y, c * (H @ (w * p.double())), c * (H.abs() @ (w * p.double()).abs()))
+
+
+def small_workspace(p, px, sod, sid, alpha):
+    """The filter with room for its taps alone: the FP32 product."""
+    from dgc_b200 import _native
+
+    lib, (A, U, V) = _native.lib(), p.shape
+    out = torch.empty_like(p)
+    n = (4 * U + 255) // 256 * 256
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    _native.check(lib.dgc_fdk_filter(p.data_ptr(), A, U, V, px, sod.data_ptr(), sid.data_ptr(), alpha,
+                                     out.data_ptr(), ws.data_ptr(), n,
+                                     torch.cuda.current_stream().cuda_stream))
+    return out
+
+
+def test_values_outside_the_split_take_the_fp32_product():
+    """NaN, infinities, values at either end of FP32's range: view by view as the FP32
+    product gives them, the other views untouched."""
+    from dgc_b200 import _ops
+
+    A, U, V = 7, 130, 70
+    p, sid, sod = scan(A, U, V, 4)
+    p[1, 5, 6] = float("nan")
+    p[2, 129, 69] = float("inf")
+    p[3] *= 1e-30
+    p[4, 7, 8] = 3e38
+    p[5] = 0
+    y = _ops.fdk_filter(p, 1.0, sod, sid, 0.8)
+    f = small_workspace(p, 1.0, sod, sid, 0.8)
+    for a in (1, 2, 3, 4, 5):
+        assert torch.equal(torch.nan_to_num(y[a], 7.0, 8.0, 9.0), torch.nan_to_num(f[a], 7.0, 8.0, 9.0))
+    assert not torch.isfinite(y[1]).all() and not torch.isfinite(y[2]).all()
+    for a in (0, 6):
+        one = _ops.fdk_filter(p[a:a + 1].contiguous(), 1.0, sod[a:a + 1], sid[a:a + 1], 0.8)
+        assert torch.equal(y[a], one[0])
+        assert float((y[a] - f[a]).norm() / f[a].norm()) <= 2.0**-19  # both sides' bounds
+
+
+def test_chunks_of_views():
+    """More views than the split holds at a time: each as in a call of its own."""
+    from dgc_b200 import _ops
+
+    A, U, V = 12, 2048, 2000
+    p, sid, sod = scan(A, U, V, 5)
+    y = _ops.fdk_filter(p, 1.0, sod, sid, 0.8)
+    for a in (0, 5, 6, 11):
+        one = _ops.fdk_filter(p[a:a + 1].contiguous(), 1.0, sod[a:a + 1], sid[a:a + 1], 0.8)
+        assert torch.equal(y[a], one[0])

@@ -27,6 +27,8 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include <climits>
+
 #include "backprojector.cuh"
 
 namespace dgc {
@@ -173,15 +175,34 @@ __host__ __device__ __forceinline__ int bp_super(int cta) { return cta >= 64 ? 1
 // A CTA owns a cta_x x cta_y patch of (x, y) columns, one warp per column
 // (at most kBpMaxWarps warps), and 32*KZ voxels of each along z.
 //
-// Register caps by z depth (in place of launch bounds, which cannot express
-// "five 256-thread CTAs per SM"): at KZ = 2 the compiler's own choice (49
-// registers) leaves four CTAs per SM and runs 1.5x slower than 48 registers
-// and five CTAs.  Any CTA of up to kBpMaxWarps warps fits under each cap.
+// What bounds it is the L1 pipe: the 32 quads of a warp's load, 16 bytes each and
+// 1.67 quads apart at magnification 1.67, take 8.5 of its cycles (4 if they were
+// contiguous), and two of three come from L2.  So the six values of a (column, view)
+// are read from shared memory (two broadcasts; six shuffles were a quarter of that
+// pipe's work at KZ = 2), and the loads of four taps (one view's at KZ = 4, two
+// views' at KZ = 2, four views' at KZ = 1) are issued before the first of them is
+// used.  KZ = 4 now runs at 9.2 L1 cycles per load.
+//
+// Register caps by z depth (launch bounds cannot express "seven 128-thread CTAs per
+// SM"): 72 leave 28 warps per SM, and the four loads in flight with them; 64 (KZ = 4:
+// 256^3 7.2 ms for 6.5, 512^3 26.3 for 24.3) serialise the loads, 80 leave 24 warps
+// (6.6, 25.2).  KZ = 3 holds three loads in 64.  CTAs of 2 x 2 columns: of 4 x 2, 72
+// registers leave only 24 warps (6.7, 25.6).
+//
+// Before (KZ = 2 above 32 slices, shuffles, one tap at a time, 8 x 1 columns) -> now:
+// 256^3 / 360 x 384^2 7.40 -> 6.48 ms; 512^3 / 180 x 768^2 28.1 -> 24.3; 128^3 / 180 x
+// 256^2 0.640 -> 0.521; 90 x 133 x 121 / 200 x 187 x 161 0.527 -> 0.372; 64^3 / 90 x
+// 128^2 0.070 -> 0.056; 24 x 40 x 40 / 30 x 48^2 0.028 -> 0.020.
 template <int KZ, bool PIXDIV, bool FDK>
-__global__ void __maxnreg__(KZ == 1 ? 40 : KZ == 2 ? 48 : KZ == 4 ? 64 : 96) bp_forward_kernel(BpArgs p) {
-    __shared__ float s_out[32 * KZ][kBpMaxWarps + 1];
+__global__ void __maxnreg__(KZ == 3 ? 64 : KZ == 8 ? 96 : 72) bp_forward_kernel(BpArgs p) {
+    constexpr int kViews = KZ == 1 ? 4 : KZ == 2 ? 2 : 1;
+    constexpr int kDepth = KZ >= 4 ? 4 : KZ;
+    extern __shared__ __align__(16) unsigned char bp_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int cx = p.cta_x, cy = p.cta_y, nw = cx * cy;
+    float4* s_line = reinterpret_cast<float4*>(bp_smem) + 32 * warp;
+    float2* s_rest = reinterpret_cast<float2*>(bp_smem + 512 * nw) + 32 * warp;
+    float (*s_out)[kBpMaxWarps + 1] = reinterpret_cast<float (*)[kBpMaxWarps + 1]>(bp_smem);
     const int tiles_x = (p.W + cx - 1) / cx, tiles_y = (p.H + cy - 1) / cy;
     const BpTile tile = bp_tile((long long)blockIdx.y * gridDim.x + blockIdx.x, tiles_x, tiles_y,
                                 bp_super(cx), bp_super(cy));
@@ -212,9 +233,10 @@ __global__ void __maxnreg__(KZ == 1 ? 40 : KZ == 2 ? 48 : KZ == 4 ? 64 : 96) bp_
         // magic-number split, which maps NaN, infinities and values beyond
         // 2^22 outside [0, V-2]) as an unsigned index is below V-1
         const uint32_t vcount = (uint32_t)max(p.V - 1, 0);
-        f32x2 pz2[KZ / 2 > 0 ? KZ / 2 : 1];
+        constexpr int kPairs = (KZ + 1) / 2;
+        f32x2 pz2[kPairs];
 #pragma unroll
-        for (int k = 0; k + 1 < KZ; k += 2) pz2[k / 2] = pack2(pz[k], pz[k + 1]);
+        for (int k = 0; k < kPairs; ++k) pz2[k] = pack2(pz[2 * k], pz[2 * k + 1 < KZ ? 2 * k + 1 : 2 * k]);
         const f32x2 ip2 = pack2(p.inv_pixel, p.inv_pixel);
         const f32x2 npix2 = pack2(-p.pixel_size, -p.pixel_size);
         const f32x2 magic2 = pack2(kFloorMagic, kFloorMagic);
@@ -224,53 +246,65 @@ __global__ void __maxnreg__(KZ == 1 ? 40 : KZ == 2 ? 48 : KZ == 4 ? 64 : 96) bp_
             if (a0 + lane < p.A) mine = column_view<PIXDIV>(p.vt[a0 + lane], a0 + lane, vx, vy, p);
             const unsigned valid_mask = __ballot_sync(FULL, mine.valid);
             const int nv = min(32, p.A - a0);
+            __syncwarp();  // the last 32 views' have been read
+            if (mine.valid) {
+                s_line[lane] = make_float4(mine.t, mine.ds_v, mine.v0, mine.w);
+                s_rest[lane] = make_float2(mine.fu, __int_as_float(mine.row));
+            }
+            __syncwarp();
             // views in chunks of 8, each chunk's FP32 partial sums added into
             // the FP64 totals after it
             for (int jb = 0; jb < nv; jb += 8) {
                 const int je = min(jb + 8, nv);
-                for (int j = jb; j < je; ++j) {
-                    if (!((valid_mask >> j) & 1u)) continue;
-                    const float t = __shfl_sync(FULL, mine.t, j);
-                    const float dsv = __shfl_sync(FULL, mine.ds_v, j);
-                    const float v0 = __shfl_sync(FULL, mine.v0, j);
-                    const float w = __shfl_sync(FULL, mine.w, j);
-                    const float fu = __shfl_sync(FULL, mine.fu, j);
-                    const int row = __shfl_sync(FULL, mine.row, j);
-                    const ulonglong2* __restrict__ rq =
-                        reinterpret_cast<const ulonglong2*>(p.pquads) + row;
-                    // one tap: v_idx's floor split -> validity, column pair lerp
-                    // along v (packed: rows u and u+1), then along u
-                    auto tap = [&](int k, uint32_t biased, float fv) {
-                        const uint32_t vi = biased - kFloorMagicBits;
-                        if (32 * k < zlimit && vi < vcount) {
-                            const ulonglong2 q = __ldg(rq + vi);
-                            const float2 e = unpack2(lerp2(q.x, q.y, pack2(fv, fv)));
-                            part[k] = fmaf(w, lerpf(e.x, e.y, fu), part[k]);
-                        }
-                    };
-                    if constexpr (KZ % 2 == 0) {
-                        const f32x2 t2 = pack2(t, t), d2 = pack2(dsv, dsv), o2 = pack2(v0, v0);
+                for (int j = jb; j < je; j += kViews) {
+                    if (!((valid_mask >> j) & ((1u << kViews) - 1u))) continue;
+                    // the taps of kViews views and kDepth steps of z: all positions and
+                    // loads first, then the interpolations
 #pragma unroll
-                        for (int k = 0; k < KZ; k += 2) {
-                            const f32x2 vp = fma2(t2, sub2(pz2[k / 2], d2), d2);
-                            const f32x2 vx2 = PIXDIV ? add2(div_by2(vp, npix2, ip2), o2)
-                                                     : fma2(vp, ip2, o2);
-                            const f32x2 f2 = add2_rd(vx2, magic2);
-                            const float2 fr = unpack2(sub2(vx2, sub2(f2, magic2)));
-                            const uint2 bits = unpack2_bits(f2);
-                            tap(k, bits.x, fr.x);
-                            tap(k + 1, bits.y, fr.y);
-                        }
-                    } else {
+                    for (int kb = 0; kb < KZ; kb += kDepth) {
+                        ulonglong2 q[kViews][kDepth];
+                        float fv[kViews][kDepth], fu[kViews], w[kViews];
+                        bool in[kViews][kDepth];
 #pragma unroll
-                        for (int k = 0; k < KZ; ++k) {
-                            const float v_phys = dsv + t * (pz[k] - dsv);
-                            const float v_idx =
-                                PIXDIV ? div_by(v_phys, p.pixel_size, p.inv_pixel) + v0
-                                       : fmaf(v_phys, p.inv_pixel, v0);
-                            const FloorSplit fs = floor_split(v_idx);
-                            tap(k, fs.biased, fs.frac);
+                        for (int i = 0; i < kViews; ++i) {
+                            const float4 line = s_line[j + i];
+                            const float2 rest = s_rest[j + i];
+                            const bool valid = kViews == 1 || (valid_mask >> (j + i)) & 1u;
+                            const f32x2 t2 = pack2(line.x, line.x), d2 = pack2(line.y, line.y);
+                            const f32x2 o2 = pack2(line.z, line.z);
+                            w[i] = line.w;
+                            fu[i] = rest.x;
+                            const ulonglong2* __restrict__ rq =
+                                reinterpret_cast<const ulonglong2*>(p.pquads) + __float_as_int(rest.y);
+#pragma unroll
+                            for (int k = 0; k < kDepth; k += 2) {
+                                const f32x2 vp = fma2(t2, sub2(pz2[(kb + k) / 2], d2), d2);
+                                const f32x2 vx2 = PIXDIV ? add2(div_by2(vp, npix2, ip2), o2)
+                                                         : fma2(vp, ip2, o2);
+                                const f32x2 f2 = add2_rd(vx2, magic2);
+                                const float2 f = unpack2(sub2(vx2, sub2(f2, magic2)));
+                                const uint2 bits = unpack2_bits(f2);
+#pragma unroll
+                                for (int h = 0; h < 2; ++h) {
+                                    if (k + h >= kDepth) break;
+                                    const uint32_t vi = (h ? bits.y : bits.x) - kFloorMagicBits;
+                                    const bool ok = valid && 32 * (kb + k + h) < zlimit && vi < vcount;
+                                    in[i][k + h] = ok;
+                                    fv[i][k + h] = h ? f.y : f.x;
+                                    q[i][k + h] = make_ulonglong2(0, 0);
+                                    if (ok) q[i][k + h] = __ldg(rq + vi);
+                                }
+                            }
                         }
+#pragma unroll
+                        for (int i = 0; i < kViews; ++i)
+#pragma unroll
+                            for (int k = 0; k < kDepth; ++k) {
+                                const float2 e = unpack2(lerp2(q[i][k].x, q[i][k].y,
+                                                               pack2(fv[i][k], fv[i][k])));
+                                if (in[i][k])
+                                    part[kb + k] = fmaf(w[i], lerpf(e.x, e.y, fu[i]), part[kb + k]);
+                            }
                     }
                 }
 #pragma unroll
@@ -281,7 +315,9 @@ __global__ void __maxnreg__(KZ == 1 ? 40 : KZ == 2 ? 48 : KZ == 4 ? 64 : 96) bp_
             }
         }
     }
-    // Transpose through shared memory; write rows along X.
+    // Transpose through shared memory (the views' values are done with); write rows
+    // along X.
+    __syncthreads();
 #pragma unroll
     for (int k = 0; k < KZ; ++k) {
         float val = FDK ? (float)(acc[k] * (double)p.out_scale) : (float)acc[k];
@@ -1017,12 +1053,16 @@ namespace {
 template <int KZ>
 int launch_bp_forward_kz(const BpArgs& p, bool pixdiv, bool fdk, dim3 grid, cudaStream_t s) {
     const unsigned threads = 32u * (unsigned)(p.cta_x * p.cta_y);
+    // a column's values of 32 views, then the transposed tile in their place
+    const size_t smem = std::max<size_t>(
+        threads * (sizeof(float4) + sizeof(float2)),
+        sizeof(float) * 32 * KZ * (kBpMaxWarps + 1));
     if (fdk) {
-        if (pixdiv) bp_forward_kernel<KZ, true, true><<<grid, threads, 0, s>>>(p);
-        else bp_forward_kernel<KZ, false, true><<<grid, threads, 0, s>>>(p);
+        if (pixdiv) bp_forward_kernel<KZ, true, true><<<grid, threads, smem, s>>>(p);
+        else bp_forward_kernel<KZ, false, true><<<grid, threads, smem, s>>>(p);
     } else {
-        if (pixdiv) bp_forward_kernel<KZ, true, false><<<grid, threads, 0, s>>>(p);
-        else bp_forward_kernel<KZ, false, false><<<grid, threads, 0, s>>>(p);
+        if (pixdiv) bp_forward_kernel<KZ, true, false><<<grid, threads, smem, s>>>(p);
+        else bp_forward_kernel<KZ, false, false><<<grid, threads, smem, s>>>(p);
     }
     DGC_LAUNCH_CHECK("bp_forward_kernel");
     return DGC_OK;
@@ -1043,12 +1083,24 @@ int bp_launch_forward(const BpArgs& args, bool fdk, cudaStream_t s) {
     BpArgs p = args;
     bp_forward_cta(p.D, p.A, p.cta_x, p.cta_y);
     const bool pixdiv = !is_pow2_float(p.pixel_size);
-    const int kz = bp_kz_forward(p.D, p.A);
+    int kz = bp_kz_forward(p.D, p.A);
+    const long long blocks = (long long)ceil_div(p.W, 2) * ceil_div(p.H, 2);
+    if (p.cta_x == 8 && p.cta_y == 1 && kz == (p.D <= 32 ? 1 : 2) && blocks <= INT_MAX) {
+        // The built-in tile, from a rule or without one, stands for the kernel's own
+        // choice: 2 x 2 columns and the fewest blocks of up to 128 slices, each no
+        // deeper than it needs to be (KZ = 2 / 3 / 4, ms: 70 x 256^2, 180 views 1.62 /
+        // 1.21 / -, 96 x 128^2, 180 views 0.50 / 0.45 / -, 128^3 0.54 / 0.70 / 0.52,
+        // 160^3, 200 views 1.12 / 1.08 / 1.29, 192^3, 360 views 3.37 / 3.45 / 3.85,
+        // 256^3 6.65 / 7.08 / 6.48)
+        p.cta_x = p.cta_y = 2;
+        kz = ceil_div(p.D, 32 * (long long)ceil_div(p.D, 128));
+    }
     const dim3 grid((unsigned)(ceil_div(p.W, p.cta_x) * (long long)ceil_div(p.H, p.cta_y)),
                     (unsigned)ceil_div(p.D, 32 * kz));
     switch (kz) {
         case 1: return launch_bp_forward_kz<1>(p, pixdiv, fdk, grid, s);
         case 2: return launch_bp_forward_kz<2>(p, pixdiv, fdk, grid, s);
+        case 3: return launch_bp_forward_kz<3>(p, pixdiv, fdk, grid, s);
         case 4: return launch_bp_forward_kz<4>(p, pixdiv, fdk, grid, s);
         default: return launch_bp_forward_kz<8>(p, pixdiv, fdk, grid, s);
     }

@@ -423,12 +423,24 @@ __device__ __forceinline__ float quad_value(const ulonglong2& q0, const ulonglon
     return fmaf(c.fy, e.y, e.x);
 }
 
+// Samples whose loads fp_forward_kernel has in flight at once.  One at a time, the march
+// waited for its loads (9 of 18 warp-cycles per instruction) with issue and FMA pipe at
+// 65 %; four at a time load also where samples share their cell, and fill the L1 pipe
+// instead: 256^3 / 360 x 384^2 35.2 -> 34.1 ms, 512^3 / 96 x 768^2 86.0 -> 82.8, 128^3 of
+// 4.0 / 180 x 256^2 at step 2 4.48 -> 4.09, 32^3 / 24 x 48^2 28 -> 24 us.  The other
+// forms tried took 34-37 ms, 88-92 and 4.2-4.5: two, three or five in flight, three CTAs
+// per SM instead of four, whole groups without predicates, and the cell's index computed
+// under the predicate (which makes a branch of it, and the loads wait again).  The
+// persistent batch kernel, six CTAs per SM, has no registers for it (10.07 -> 10.18 ms).
+constexpr int kMarchGroup = 4;
+
 // Sum of the trilinear samples along the ray (fp.cu:321-335).  The
 // interpolation runs on packed (value, y difference) pairs: along x at z0 and
 // z1, along z, then along y.
 // UNROLL: the march loop unrolled by the compiler (1 or 2; the same samples
-// and sums either way, a tuned dimension of the forward).
-template <bool CLAMP, bool DIV, bool OFF, bool GUARD = true, int UNROLL = 1>
+// and sums either way, a tuned dimension of the forward).  GROUP: samples in flight
+// where the steps advance, the same samples and sums again.
+template <bool CLAMP, bool DIV, bool OFF, bool GUARD = true, int UNROLL = 1, int GROUP = 1>
 __device__ __forceinline__ float march_sum(const RaySetup& r, const ViewGeo& vg, const FpArgs& p) {
     const ulonglong2* __restrict__ Q = reinterpret_cast<const ulonglong2*>(p.quads);
     const XYPacks k = make_xy_packs<DIV>(r, vg, p);
@@ -436,6 +448,32 @@ __device__ __forceinline__ float march_sum(const RaySetup& r, const ViewGeo& vg,
     float acc = 0.0f;
     float t = r.tmin;
     int n = 0;
+    if constexpr (!GUARD && GROUP > 1) {
+#pragma unroll 1
+        while (t <= r.tmax) {
+            ulonglong2 q0[GROUP], q1[GROUP];
+            Cell c[GROUP];
+            bool in[GROUP];
+#pragma unroll
+            for (int i = 0; i < GROUP; ++i) {
+                c[i] = sample_cell<CLAMP, DIV, OFF, true>(t, r, vg, p, k);
+                const uint32_t qi = quad_index(c[i], p);
+                in[i] = i == 0 || t <= r.tmax;
+                q0[i] = q1[i] = make_ulonglong2(0, 0);
+                if (in[i]) {
+                    q0[i] = __ldg(Q + qi);
+                    q1[i] = __ldg(Q + qi + 1);
+                }
+                t += p.step_size;
+            }
+#pragma unroll
+            for (int i = 0; i < GROUP; ++i) {
+                const float v = quad_value(q0[i], q1[i], c[i]);
+                if (in[i]) acc += v;
+            }
+        }
+        return acc;
+    }
     CellQuads cq;
 #pragma unroll UNROLL
     for (; t <= r.tmax && (!GUARD || n < nmax); t += p.step_size, n += GUARD ? 1 : 0) {
@@ -508,7 +546,7 @@ __device__ __forceinline__ void tile_ray(const TileCoord& tc, int& u, int& v) {
 }
 
 // Line integral of one ray, written to p.projections.
-template <bool DIV, bool OFF, int UNROLL = 1>
+template <bool DIV, bool OFF, int UNROLL = 1, int GROUP = 1>
 __device__ __forceinline__ void forward_ray(const FpArgs& p, const ViewGeo& vg, int a, int u,
                                             int v) {
     const RaySetup r = setup_ray(vg, u, v, p);
@@ -516,8 +554,8 @@ __device__ __forceinline__ void forward_ray(const FpArgs& p, const ViewGeo& vg, 
     if (r.ok && r.hit) {
         const bool inside = ray_inside_pad<DIV>(r, vg, p);
         if (steps_advance(r, p.step_size))
-            integral = inside ? march_sum<false, DIV, OFF, false, UNROLL>(r, vg, p)
-                              : march_sum<true, DIV, OFF, false, UNROLL>(r, vg, p);
+            integral = inside ? march_sum<false, DIV, OFF, false, UNROLL, GROUP>(r, vg, p)
+                              : march_sum<true, DIV, OFF, false, UNROLL, GROUP>(r, vg, p);
         else
             integral = inside ? march_sum<false, DIV, OFF, true, UNROLL>(r, vg, p)
                               : march_sum<true, DIV, OFF, true, UNROLL>(r, vg, p);
@@ -528,7 +566,7 @@ __device__ __forceinline__ void forward_ray(const FpArgs& p, const ViewGeo& vg, 
 
 // A CTA owns TU detector columns x (256/TU) rows of one view.
 template <int TU, bool DIV, bool OFF, int UNROLL = 1>
-__global__ void __launch_bounds__(256) fp_forward_kernel(FpArgs p) {
+__global__ void __launch_bounds__(256, 4) fp_forward_kernel(FpArgs p) {
     __shared__ ViewGeo s_view;
     const int tiles_u = (p.U + TU - 1) / TU;
     const TileCoord tc = tile_coord(p, tiles_u);
@@ -544,7 +582,7 @@ __global__ void __launch_bounds__(256) fp_forward_kernel(FpArgs p) {
     if (TU % 4 == 0 && p.view_block > 0) tile_ray<TU, (TU % 4 == 0 ? 4 : 1)>(tc, u, v);
     else tile_ray<TU>(tc, u, v);
     if (u >= p.U || v >= p.V) return;
-    forward_ray<DIV, OFF, UNROLL>(p, vg, tc.a, u, v);
+    forward_ray<DIV, OFF, UNROLL, UNROLL == 1 ? kMarchGroup : 1>(p, vg, tc.a, u, v);
 }
 
 // ---------------------------------------------------------------------------

@@ -13,7 +13,8 @@
 //     positions (coalesced).
 //   * Per-view trig and source terms are tabulated once per call; within a
 //     warp, lane j evaluates the column geometry of view a0+j and the warp
-//     broadcasts it with shuffles, so no lane recomputes it.
+//     broadcasts it (the forward through shared memory, the backward with
+//     shuffles), so no lane recomputes it.
 //   * Projections are re-laid out as quads PQ[a][u][v] = float4(P[u][v],
 //     P[u+1][v], P[u][v+1], P[u+1][v+1]) -- two column pairs, so the lerp
 //     along v runs as one packed f32x2 lerp over rows u and u+1: one 16-byte
@@ -23,12 +24,11 @@
 //   * The backward sums the per-voxel terms over Z in four accumulators and
 //     applies the (column, view) chain-rule coefficients once per warp; the
 //     eight per-view gradients are reduced in FP64 in a fixed order.
+#include <climits>
 #include <mutex>
 #include <type_traits>
 
 #include "common.cuh"
-#include <climits>
-
 #include "backprojector.cuh"
 
 namespace dgc {

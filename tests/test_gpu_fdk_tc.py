@@ -51,9 +51,9 @@ def close(got, want, magnitudes):
 
 # edges: 96 rows is the first size; a row tile (128) and one more or less; a column
 # tile (256), two, ragged ones; rows that are not 8-element multiples; 2048 rows the
-# last, 2049 the FP32 product's
+# last (300 columns: no room to turn the rows), 2049 the FP32 product's
 SIZES = [(2, 96, 16), (1, 97, 17), (3, 127, 255), (2, 128, 256), (2, 129, 257), (5, 192, 40),
-         (1, 187, 521), (2, 768, 100), (1, 2048, 24), (1, 2049, 24)]
+         (1, 187, 521), (2, 768, 100), (1, 2048, 24), (1, 2048, 300), (1, 2049, 24)]
 
 
 @pytest.mark.parametrize("A,U,V", SIZES)

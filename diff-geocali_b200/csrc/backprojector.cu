@@ -65,26 +65,42 @@ int bp_view_table(const Geometry& g, int A, ViewRow* vt, cudaStream_t s) {
     return DGC_OK;
 }
 
-__global__ void build_proj_quads_kernel(const float* __restrict__ P, int A, int U, int V,
-                                        float4* __restrict__ PQ) {
+// Bound by the quads' stores.  A block (32, 8) fills 32 columns x 32 rows of a view,
+// kQuadRows rows a thread with the row shared by two quads read once and all loads
+// issued first; the only divisions are the block's.  720 x 768^2 1.77 -> 1.29 ms (1.31
+// at the copy bandwidth), 360 x 384^2 220 -> 163 us, 200 x 187 x 161 26 -> 17 us against
+// one quad a thread with 64-bit divisions for its place.
+constexpr int kQuadRows = 4;
+
+__global__ void __launch_bounds__(256) build_proj_quads_kernel(const float* __restrict__ P, int U,
+                                                               int V, int tiles_v, int tiles_u,
+                                                               float4* __restrict__ PQ) {
     const int QU = U - 1, QV = V - 1;
-    const long long total = (long long)A * QU * QV;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int v = (int)(i % QV);
-        const long long r = i / QV;
-        const int u = (int)(r % QU);
-        const int a = (int)(r / QU);
-        const float* row = P + ((long long)a * U + u) * V + v;
-        PQ[i] = make_float4(__ldg(row), __ldg(row + V), __ldg(row + 1), __ldg(row + V + 1));
+    int b = (int)blockIdx.x;
+    const int v = (b % tiles_v) * 32 + (int)threadIdx.x;
+    b /= tiles_v;
+    const int u = (b % tiles_u) * 8 * kQuadRows + (int)threadIdx.y * kQuadRows;
+    const int a = b / tiles_u;
+    if (v >= QV || u >= QU) return;
+    const float* __restrict__ row = P + ((long long)a * U + u) * V + v;
+    float4* __restrict__ to = PQ + ((long long)a * QU + u) * QV + v;
+    const int n = min(kQuadRows, QU - u);
+    float x[kQuadRows + 1], y[kQuadRows + 1];
+#pragma unroll
+    for (int r = 0; r <= kQuadRows; ++r) {
+        x[r] = r <= n ? __ldg(row + (long long)r * V) : 0.0f;
+        y[r] = r <= n ? __ldg(row + (long long)r * V + 1) : 0.0f;
     }
+#pragma unroll
+    for (int r = 0; r < kQuadRows; ++r)
+        if (r < n) to[(long long)r * QV] = make_float4(x[r], x[r + 1], y[r], y[r + 1]);
 }
 
 int build_proj_quads(const float* P, int A, int U, int V, float4* PQ, cudaStream_t s) {
     DGC_TRACE("build_proj_quads", s);
-    const long long total = (long long)A * (U - 1) * (V - 1);
-    const int blocks = (int)std::min<long long>((total + 255) / 256, 148LL * 16);
-    build_proj_quads_kernel<<<blocks, 256, 0, s>>>(P, A, U, V, PQ);
+    const int tiles_v = ceil_div(V - 1, 32), tiles_u = ceil_div(U - 1, 8 * kQuadRows);
+    const unsigned blocks = (unsigned)((long long)tiles_v * tiles_u * A);
+    build_proj_quads_kernel<<<blocks, dim3(32, 8), 0, s>>>(P, U, V, tiles_v, tiles_u, PQ);
     DGC_LAUNCH_CHECK("build_proj_quads");
     return DGC_OK;
 }

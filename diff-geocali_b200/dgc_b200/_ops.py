@@ -35,6 +35,17 @@ def _workspace(nbytes: int, device) -> torch.Tensor | None:
     return torch.empty(int(nbytes), dtype=torch.uint8, device=device)
 
 
+def _filter_workspace(nbytes: int, A: int, U: int, V: int, adjoint: bool, device):
+    """Workspace of the FDK filter: what the library asks for or, where the device has no
+    room for the split operands of the tensor cores, the taps (and the adjoint's sums,
+    four doubles per view and 128 x 128 tile) that its FP32 product needs."""
+    try:
+        return _workspace(nbytes, device)
+    except torch.cuda.OutOfMemoryError:
+        sums = 32 * A * (-(-U // 128)) * (-(-V // 128)) if adjoint else 0
+        return _workspace(-(-4 * U // 256) * 256 + -(-sums // 256) * 256, device)
+
+
 def _p(t):
     return None if t is None else t.data_ptr()
 
@@ -301,7 +312,7 @@ def fdk_filter(projections, pixel_size, sod, sid, alpha):
     out = torch.empty_like(p)
     lib = _native.lib()
     with torch.cuda.device(dev):
-        ws = _workspace(lib.dgc_fdk_filter_workspace_bytes(A, U, V), dev)
+        ws = _filter_workspace(lib.dgc_fdk_filter_workspace_bytes(A, U, V), A, U, V, False, dev)
         _native.check(lib.dgc_fdk_filter(
             p.data_ptr(), A, U, V, float(pixel_size), sod.data_ptr(), sid.data_ptr(), float(alpha),
             out.data_ptr(), _p(ws), 0 if ws is None else ws.numel(), _stream(dev)))
@@ -322,7 +333,8 @@ def fdk_filter_backward(grad_filtered, projections, filtered, pixel_size, sod, s
     y = filtered.contiguous() if need_distances else None
     lib = _native.lib()
     with torch.cuda.device(dev):
-        ws = _workspace(lib.dgc_fdk_filter_backward_workspace_bytes(A, U, V), dev)
+        ws = _filter_workspace(lib.dgc_fdk_filter_backward_workspace_bytes(A, U, V), A, U, V,
+                               True, dev)
         _native.check(lib.dgc_fdk_filter_backward(
             g.data_ptr(), _p(p), _p(y), A, U, V, float(pixel_size), sod.data_ptr(),
             sid.data_ptr(), float(alpha), _p(gp), _p(gsod), _p(gsid), _p(ws),
@@ -349,7 +361,7 @@ def fdk_filter_framed(projections, pixel_size, sod, sid, alpha, frame):
     out = torch.empty_like(p)
     lib = _native.lib()
     with torch.cuda.device(dev):
-        ws = _workspace(lib.dgc_fdk_filter_workspace_bytes(A, U, V), dev)
+        ws = _filter_workspace(lib.dgc_fdk_filter_workspace_bytes(A, U, V), A, U, V, False, dev)
         _native.check(lib.dgc_fdk_filter_ex(
             p.data_ptr(), A, U, V, float(pixel_size), sod.data_ptr(), sid.data_ptr(), *ptrs,
             float(alpha), out.data_ptr(), _p(ws), 0 if ws is None else ws.numel(),
@@ -379,7 +391,8 @@ def fdk_filter_backward_framed(grad_filtered, projections, filtered, pixel_size,
     y = filtered.contiguous() if dist else None
     lib = _native.lib()
     with torch.cuda.device(dev):
-        ws = _workspace(lib.dgc_fdk_filter_backward_workspace_bytes(A, U, V), dev)
+        ws = _filter_workspace(lib.dgc_fdk_filter_backward_workspace_bytes(A, U, V), A, U, V,
+                               True, dev)
         _native.check(lib.dgc_fdk_filter_backward_ex(
             g.data_ptr(), _p(p), _p(y), A, U, V, float(pixel_size), sod.data_ptr(),
             sid.data_ptr(), *ptrs, float(alpha), _p(gp), _p(gsod), _p(gsid),

@@ -143,3 +143,29 @@ def test_chunks_of_views():
     for a in (0, 5, 6, 11):
         one = _ops.fdk_filter(p[a:a + 1].contiguous(), 1.0, sod[a:a + 1], sid[a:a + 1], 0.8)
         assert torch.equal(y[a], one[0])
+
+
+def test_without_room_for_the_scratch(monkeypatch):
+    """No device memory for the split operands: the FP32 product's values and gradients."""
+    from dgc_b200 import _ops
+
+    A, U, V = 3, 200, 150
+    p, sid, sod = scan(A, U, V, 6)
+    g = torch.randn(p.shape, generator=torch.Generator().manual_seed(2)).cuda()
+    want = _ops.fdk_filter(p, 1.0, sod, sid, 0.8)
+    grads = _ops.fdk_filter_backward(g, p, want, 1.0, sod, sid, 0.8)
+    room = _ops._workspace
+
+    def tight(nbytes, device):
+        if nbytes > 2048:
+            raise torch.cuda.OutOfMemoryError("no room")
+        return room(nbytes, device)
+
+    monkeypatch.setattr(_ops, "_workspace", tight)
+    y = _ops.fdk_filter(p, 1.0, sod, sid, 0.8)
+    assert torch.equal(y, small_workspace(p, 1.0, sod, sid, 0.8))
+    assert not torch.equal(y, want)  # the other route
+    for got, ref in zip(_ops.fdk_filter_backward(g, p, y, 1.0, sod, sid, 0.8), grads):
+        # both sides within 2^-20 of the magnitudes summed; sums of random signs lose
+        # at most the square root of their 30000 terms, 2^8, of that
+        assert float((got - ref).abs().max()) <= 2.0**-19 * 2.0**8 * float(ref.abs().max())

@@ -395,8 +395,8 @@ __device__ __forceinline__ uint32_t quad_index(const Cell& c, const FpArgs& p) {
 // stay in one cell (about half of them at step 0.5 voxel along an axis), and
 // then read the same 32 bytes: those keep the previous sample's registers and
 // issue no load.  Bitwise the same values as loading every sample.  Used by
-// the value march only: it takes the forward at 256^3 / 360 x 384^2 from
-// 40.1 to 38.7 ms and the batched forward of that instance plus its half
+// the value march where it goes sample by sample (the batch kernel, the unrolled
+// arm): the batched forward of that instance plus its half went
 // from 50.9 to 48.1 ms, while the gradient marches, which hold more live
 // values, slowed by 2-17 % with it.
 struct CellQuads {

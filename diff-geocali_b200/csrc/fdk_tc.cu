@@ -87,13 +87,13 @@ __device__ __forceinline__ Split3 split3(float x) {
 }
 
 // split[view][part][U-1-k][v] = part of the staged value of fdk_filter_kernel: the
-// cosine-weighted projection, or (ADJ) the upstream gradient; peaks[view][k / 8] = the
-// bits of its largest magnitude.  grid: x = groups of 8 rows, y = view; the blocks
+// cosine-weighted projection, or (ADJ) the upstream gradient; ranges[view][k / 8] =
+// the range of its magnitudes.  grid: x = groups of 8 rows, y = view; the blocks
 // of the row after the last view fill strip[part][q][8r + c] = part of f[8q + r + c].
 template <bool ADJ>
 __global__ void __launch_bounds__(256) fdk_split_kernel(FdkArgs p, int stride,
                                                         __nv_bfloat16* __restrict__ split,
-                                                        int* __restrict__ peaks, int cores,
+                                                        FdkRange* __restrict__ ranges, int cores,
                                                         __nv_bfloat16* __restrict__ strip) {
     if (blockIdx.y == p.A) {
         for (int i = blockIdx.x * 256 + threadIdx.x; i < cores * 64; i += gridDim.x * 256) {
@@ -115,9 +115,16 @@ __global__ void __launch_bounds__(256) fdk_split_kernel(FdkArgs p, int stride,
         (ADJ ? p.grad_filtered : p.projections) + (long long)a * p.U * p.V;
     const int groups = stride / 4;
     const bool wide = (p.V & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
-    int peak = 0;  // bits of the largest magnitude: a NaN is above the infinities
-    __shared__ int s_peak;
-    if (threadIdx.x == 0) s_peak = 0;
+    // as bits, which order as the magnitudes do: a NaN is above the infinities, and a
+    // zero, less one as unsigned, above all
+    int high = 0;
+    unsigned low = 0x7fffffffu;
+    __shared__ int s_high;
+    __shared__ unsigned s_low;
+    if (threadIdx.x == 0) {
+        s_high = 0;
+        s_low = 0x7fffffffu;
+    }
     __syncthreads();
     for (int i = threadIdx.x; i < 8 * groups; i += 256) {
         const int row = i / groups, v0 = (i - row * groups) * 4;
@@ -148,7 +155,11 @@ __global__ void __launch_bounds__(256) fdk_split_kernel(FdkArgs p, int stride,
         __align__(8) __nv_bfloat16 h[3][4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            if (v0 + j < p.V) peak = max(peak, __float_as_int(x[j]) & 0x7fffffff);
+            if (v0 + j < p.V) {
+                const int bits = __float_as_int(x[j]) & 0x7fffffff;
+                high = max(high, bits);
+                low = min(low, (unsigned)bits - 1u);
+            }
             const Split3 s = split3(x[j]);
             h[0][j] = s.part[0];
             h[1][j] = s.part[1];
@@ -160,10 +171,16 @@ __global__ void __launch_bounds__(256) fdk_split_kernel(FdkArgs p, int stride,
                 split + (((size_t)a * 3 + s) * p.U + (p.U - 1 - k)) * stride + v0) =
                 *reinterpret_cast<const uint2*>(h[s]);
     }
-    peak = __reduce_max_sync(0xffffffffu, peak);
-    if ((threadIdx.x & 31) == 0) atomicMax(&s_peak, peak);
+    high = __reduce_max_sync(0xffffffffu, high);
+    low = __reduce_min_sync(0xffffffffu, low);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&s_high, high);
+        atomicMin(&s_low, low);
+    }
     __syncthreads();
-    if (threadIdx.x == 0) peaks[(long long)a * gridDim.x + blockIdx.x] = s_peak;
+    if (threadIdx.x == 0)
+        ranges[(long long)a * gridDim.x + blockIdx.x] =
+            FdkRange{s_low == 0x7fffffffu ? INT_MAX : (int)s_low + 1, s_high};
 }
 
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes,
@@ -184,7 +201,7 @@ struct TcArgs {
     const float* sid;  // null: out = the plain product (the adjoint's z)
     const float* sod;
     float pixel_size;
-    int* peaks;  // [views][ceil(U/8)]
+    FdkRange* ranges;  // [views][ceil(U/8)]
     bool wide, staged;  // stores: 32 bytes a lane; rows by way of shared memory
 };
 
@@ -408,7 +425,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) fdk_filter_tc_kernel(
         for (int g = s_consumed; g < issued; ++g)
             mbar_wait(tma_smem_u32(&full[g % S]), (g / S) & 1);
         for (int tile = first; tile < p.columns; tile += step)
-            p.peaks[(long long)(tile / p.col_tiles) * ((p.U + 7) / 8)] = 0x7fffffff;
+            p.ranges[(long long)(tile / p.col_tiles) * ((p.U + 7) / 8)].high = INT_MAX;
     }
     tc_fence_before();
     __syncthreads();
@@ -435,7 +452,7 @@ bool split_map(CUtensorMap* map, const __nv_bfloat16* split, int views, int U, i
 
 // The product of `views` split views into out (scaled where f is given).
 int launch_tc(const FdkArgs* f, const __nv_bfloat16* strip, const __nv_bfloat16* split, int views,
-              int U, int V, float* out, int* peaks, cudaStream_t s, bool* used) {
+              int U, int V, float* out, FdkRange* ranges, cudaStream_t s, bool* used) {
     *used = false;
     CUtensorMap map;
     if (!split_map(&map, split, views, U, V)) return DGC_OK;
@@ -463,7 +480,7 @@ int launch_tc(const FdkArgs* f, const __nv_bfloat16* strip, const __nv_bfloat16*
     p.sid = f ? f->sid : nullptr;
     p.sod = f ? f->sod : nullptr;
     p.pixel_size = f ? f->pixel_size : 1.0f;
-    p.peaks = peaks;
+    p.ranges = ranges;
     static std::atomic<unsigned long long> configured{0};
     const int rc = once_per_device(configured, []() -> int {
         DGC_CUDA(cudaFuncSetAttribute(fdk_filter_tc_kernel,
@@ -493,11 +510,11 @@ int launch_tc(const FdkArgs* f, const __nv_bfloat16* strip, const __nv_bfloat16*
 }
 
 template <bool ADJ>
-int launch_split(const FdkArgs& p, __nv_bfloat16* split, int* peaks, __nv_bfloat16* strip,
+int launch_split(const FdkArgs& p, __nv_bfloat16* split, FdkRange* ranges, __nv_bfloat16* strip,
                  cudaStream_t s) {
     DGC_TRACE("fdk_split_kernel", s);
     const dim3 grid((unsigned)ceil_div(p.U, 8), (unsigned)p.A + (strip ? 1 : 0));
-    fdk_split_kernel<ADJ><<<grid, 256, 0, s>>>(p, tc_row_stride(p.V), split, peaks, tc_cores(p.U),
+    fdk_split_kernel<ADJ><<<grid, 256, 0, s>>>(p, tc_row_stride(p.V), split, ranges, tc_cores(p.U),
                                                strip);
     DGC_LAUNCH_CHECK("fdk_split_kernel");
     return DGC_OK;
@@ -660,7 +677,7 @@ size_t fdk_tc_bytes(int A, int U, int V, bool adjoint) {
     const int views = fdk_tc_views(A, U, V);
     if (!views) return 0;
     return Workspace::align(3 * 128 * (size_t)tc_cores(U)) +
-           Workspace::align(sizeof(int) * (size_t)views * (size_t)ceil_div(U, 8)) +
+           Workspace::align(sizeof(FdkRange) * (size_t)views * (size_t)ceil_div(U, 8)) +
            Workspace::align(tc_split_bytes(U, V) * (size_t)views) +
            (adjoint ? Workspace::align(sizeof(float) * (size_t)U * V * (size_t)views) : 0);
 }
@@ -670,27 +687,27 @@ int fdk_tc_filter(const FdkArgs& p, bool adjoint, Workspace ws, cudaStream_t s, 
     const int views = fdk_tc_views(p.A, p.U, p.V);
     if (!views) return DGC_OK;
     __nv_bfloat16* strip = ws.take<__nv_bfloat16>((size_t)3 * 64 * (size_t)tc_cores(p.U));
-    int* peaks = ws.take<int>((size_t)views * (size_t)ceil_div(p.U, 8));
+    FdkRange* ranges = ws.take<FdkRange>((size_t)views * (size_t)ceil_div(p.U, 8));
     __nv_bfloat16* split = reinterpret_cast<__nv_bfloat16*>(
         ws.take<char>(tc_split_bytes(p.U, p.V) * (size_t)views));
     float* z = adjoint ? ws.take<float>((size_t)p.U * p.V * (size_t)views) : nullptr;
-    if (!strip || !peaks || !split || (adjoint && !z)) return DGC_OK;
+    if (!strip || !ranges || !split || (adjoint && !z)) return DGC_OK;
     for (int a0 = 0; a0 < p.A; a0 += views) {
         FdkArgs q = views_of(p, a0, std::min(views, p.A - a0));
         __nv_bfloat16* fill = a0 == 0 ? strip : nullptr;  // the taps serve every chunk
-        int rc = adjoint ? launch_split<true>(q, split, peaks, fill, s)
-                         : launch_split<false>(q, split, peaks, fill, s);
+        int rc = adjoint ? launch_split<true>(q, split, ranges, fill, s)
+                         : launch_split<false>(q, split, ranges, fill, s);
         if (rc != DGC_OK) return rc;
         bool launched = false;
         rc = launch_tc(adjoint ? nullptr : &q, strip, split, q.A, q.U, q.V,
-                       adjoint ? z : q.filtered, peaks, s, &launched);
+                       adjoint ? z : q.filtered, ranges, s, &launched);
         if (rc != DGC_OK) return rc;
         if (!launched) {
             if (a0 == 0) return DGC_OK;  // nothing written yet: the SIMT product takes the call
             set_error("fdk filter: no tensor map for a later chunk of views");
             return DGC_ERR_CUDA;
         }
-        const FdkLeft left(q, peaks);
+        const FdkLeft left(q, ranges);
         if (adjoint) {
             if ((rc = launch_epilogue(left, z, s)) != DGC_OK) return rc;
         }

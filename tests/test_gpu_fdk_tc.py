@@ -169,3 +169,29 @@ def test_without_room_for_the_scratch(monkeypatch):
         # both sides within 2^-20 of the magnitudes summed; sums of random signs lose
         # at most the square root of their 30000 terms, 2^8, of that
         assert float((got - ref).abs().max()) <= 2.0**-19 * 2.0**8 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("U,px", [(96, 1.0), (187, 1.0), (768, 3.0), (130, 0.05)])
+def test_columns_of_small_values_keep_their_precision(U, px):
+    """Every detector column to its own magnitudes, down to the subnormals, beside one of
+    ordinary values.  Below FP32's smallest normal number a rounding is 2^-149 at most
+    whatever the value: two for a weighted value, one for each of the U products, two
+    for the scale."""
+    from dgc_b200 import _ops
+
+    A, V, alpha = 2, 64, 0.8
+    p, sid, sod = scan(A, U, V, U)
+    scale = torch.tensor([1.0] + [2.0 ** -(72 + j) for j in range(1, V)]).cuda()
+    H = toeplitz(U, px, alpha)
+    w = weights(p, px, sid, torch.full_like(sid, (U - 1) / 2), torch.full_like(sid, (V - 1) / 2))
+    c = px * (sid / sod).double()[:, None, None]
+    tiny = c * (2 * float(H.abs().sum(1).max()) + U) * 2.0**-149 + 2.0**-148
+
+    def held(got, want, magnitudes):
+        assert float(((got.double() - want).abs() - 128 * E * magnitudes - tiny).max()) <= 0
+
+    x = p * scale
+    y = _ops.fdk_filter(x, px, sod, sid, alpha)
+    held(y, c * (H @ (w * x.double())), c * (H.abs() @ (w * x.double()).abs()))
+    gp, _, _ = _ops.fdk_filter_backward(x, x, y, px, sod, sid, alpha)
+    held(gp, c * w * (H @ x.double()), c * w * (H.abs() @ x.double().abs()))

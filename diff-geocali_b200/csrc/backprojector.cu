@@ -37,9 +37,7 @@ namespace dgc {
 // Per-view table and projection re-layout
 // ---------------------------------------------------------------------------
 
-__global__ void bp_view_table_kernel(Geometry g, int A, ViewRow* __restrict__ vt) {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= A) return;
+__device__ __forceinline__ ViewRow view_row(const Geometry& g, int a) {
     const float beta = g.angles[a];
     const float c = cosf(beta);
     const float s = sinf(beta);
@@ -54,8 +52,14 @@ __global__ void bp_view_table_kernel(Geometry g, int A, ViewRow* __restrict__ vt
     r.sid = g.sid[a];
     r.u0 = g.det_u0[a];
     r.v0 = g.det_v0[a];
-    r.pad0 = r.pad1 = r.pad2 = 0.0f;
-    vt[a] = r;
+    r.gather = 0;
+    r.pad1 = r.pad2 = 0.0f;
+    return r;
+}
+
+__global__ void bp_view_table_kernel(Geometry g, int A, ViewRow* __restrict__ vt) {
+    const int a = blockIdx.x * blockDim.x + threadIdx.x;
+    if (a < A) vt[a] = view_row(g, a);
 }
 
 int bp_view_table(const Geometry& g, int A, ViewRow* vt, cudaStream_t s) {
@@ -474,6 +478,7 @@ template <int KZ, int GP, bool GEO>
 __global__ void __launch_bounds__(256) bp_backward_kernel(BpArgs p) {
     constexpr int G = kBpGroup;
     __shared__ double s_terms[GEO ? 8 : 1][32][8];
+    if (p.only_if >= 0 && p.vt[0].gather != p.only_if) return;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int cols_x = (p.W + 7) >> 3;
@@ -685,8 +690,10 @@ __global__ void __launch_bounds__(256) bp_reduce_partials_kernel(const double* _
 // G[(y*W + x)*(D+3) + z + 1], z in [-1, D+1].
 // grid: x = ceil(W/32) * H, y = ceil((D+3)/32); block (32, 8)
 __global__ void __launch_bounds__(256) bp_columns_kernel(const float* __restrict__ g, int D, int H,
-                                                         int W, float* __restrict__ G) {
+                                                         int W, const ViewRow* __restrict__ vt,
+                                                         float* __restrict__ G) {
     __shared__ float tile[32][33];
+    if (!vt[0].gather) return;
     const int xtiles = (W + 31) / 32;
     const int y = blockIdx.x / xtiles;
     const int x0 = (blockIdx.x - y * xtiles) * 32, z0 = blockIdx.y * 32 - 1;
@@ -736,17 +743,22 @@ __device__ __forceinline__ AdjLine adj_line(const ViewRow& r, float q, bool alon
     return l;
 }
 
+// The volume's corner columns: distance of one along the view's normal.
+__device__ __forceinline__ float corner_distance(const ViewRow& r, const BpArgs& p, int c) {
+    const float x = ((c & 1 ? p.W - 1 : 0) - p.W * 0.5f) * p.voxel_size + p.off_x;
+    const float y = ((c & 2 ? p.H - 1 : 0) - p.H * 0.5f) * p.voxel_size + p.off_y;
+    return r.sod + r.ds_n + x * r.s - y * r.c;
+}
+
 // First and last detector row that the volume can reach, with a margin, from its
 // four corners' magnifications (all rows if a corner is not in front of the source).
 __device__ __forceinline__ float2 adj_reach(const ViewRow& r, const BpArgs& p) {
-    const float sdn = r.sid + r.ds_n, m = r.sod + r.ds_n;
+    const float sdn = r.sid + r.ds_n;
     float tlo = FLT_MAX, thi = -FLT_MAX;
     bool front = true;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-        const float x = ((c & 1 ? p.W - 1 : 0) - p.W * 0.5f) * p.voxel_size + p.off_x;
-        const float y = ((c & 2 ? p.H - 1 : 0) - p.H * 0.5f) * p.voxel_size + p.off_y;
-        const float denom = m + x * r.s - y * r.c;
+        const float denom = corner_distance(r, p, c);
         front = front && denom > 1e-3f * fabsf(r.sod);
         tlo = fminf(tlo, sdn / denom);
         thi = fmaxf(thi, sdn / denom);
@@ -757,6 +769,35 @@ __device__ __forceinline__ float2 adj_reach(const ViewRow& r, const BpArgs& p) {
     return front ? make_float2((r.ds_v + lo) * p.inv_pixel + r.v0 - 2.0f,
                                (r.ds_v + hi) * p.inv_pixel + r.v0 + 2.0f)
                  : make_float2(-FLT_MAX, FLT_MAX);
+}
+
+// The view table, and in its rows whether every view is one for the gather.  With s a
+// voxel's height in pixels: 1 or more in the farthest corner (below, a pixel has more
+// than two voxels and the general sum runs: 1.6-3 times the scatter's time at
+// 1.1-fold magnification), at most 5 in the middle (a column's pixels are mostly
+// between two voxels: 1.1-1.8 times at 6-8), and a detector that the volume's shadow
+// fills to `fill` (else the pixels beside it idle).  bp_may_gather has the
+// measurements.  One block: a scan has hundreds of views.
+__global__ void __launch_bounds__(256) bp_view_choice_kernel(Geometry g, BpArgs p, float fill,
+                                                             ViewRow* __restrict__ vt) {
+    bool ok = true;
+    for (int a = threadIdx.x; a < p.A; a += 256) {
+        const ViewRow r = view_row(g, a);
+        vt[a] = r;
+        float lo = FLT_MAX, hi = -FLT_MAX;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float d = corner_distance(r, p, c);
+            lo = fminf(lo, d);
+            hi = fmaxf(hi, d);
+        }
+        const float height = (r.sid + r.ds_n) * (p.voxel_size * p.inv_pixel);
+        const float middle = 2.0f * height / (lo + hi);
+        ok = ok && lo > 1e-3f * fabsf(r.sod) && height / hi >= 1.0001f && middle <= 5.0f &&
+             p.D * middle >= fill * p.V;
+    }
+    ok = __syncthreads_and(ok);
+    for (int a = threadIdx.x; a < p.A; a += 256) vt[a].gather = ok;
 }
 
 // Work item: `bins` bins of one view, one tile of V; NV pixels a thread, a warp's
@@ -773,7 +814,9 @@ __global__ void __launch_bounds__(32 * kAdjMaxWarps, NV < 3 ? 4 : 3)
     const int block = blockIdx.x / tiles;
     const int a = block / bin_blocks;
     const int b0 = (block - a * bin_blocks) * bins;
-    const int b1 = min(b0 + bins, p.U - 1);
+    // no bins where the views chose the scatter (returning here instead took 7 % of the
+    // kernel's time: the compiler then allocates the loop's registers otherwise)
+    const int b1 = p.vt[a].gather ? min(b0 + bins, p.U - 1) : b0;
     const ViewRow r = p.vt[a];
     const float vox = p.voxel_size;
 
@@ -1129,9 +1172,9 @@ int bp_launch_backward(const BpArgs& p, cudaStream_t s) {
     const int kz = p.kz_backward ? p.kz_backward : bp_kz_backward(p.D, p.A);
     unsigned gx, gy;
     bp_grid(p.D, p.H, p.W, kz, gx, gy);
-    const dim3 grid(gx, gy);
     const int gp = p.grad_projections ? 1 : 0;
     const bool geo = p.partials != nullptr;
+    const dim3 grid(gx, gy);
     switch (kz) {
         case 1: return launch_bp_backward_kz<1>(p, gp, geo, grid, s);
         case 2: return launch_bp_backward_kz<2>(p, gp, geo, grid, s);
@@ -1142,39 +1185,52 @@ int bp_launch_backward(const BpArgs& p, cudaStream_t s) {
 
 size_t bp_column_floats(int D, int H, int W) { return (size_t)(D + 3) * H * W; }
 
-// Detector rows that the volume spans, at about twofold magnification.
-static float bp_shadow(const BpArgs& p) { return 2.2f * p.D * p.voxel_size * p.inv_pixel; }
-
-// Gather or scatter?  The gather's work is a column times the detector's rows
-// (those in the volume's shadow), whatever the number of voxels along z, and its
-// columns come in bins that must feed whole CTAs.  Measured gather / scatter,
-// the projection gradient alone: 10.0 / 18.5 ms (256^3 / 360 x 384^2), 3.4 / 5.1
-// (200 x 180 x 150 / 300 x 260 x 290), 1.07 / 1.63 (128^3 / 180 x 256^2), 0.26 /
-// 0.35 (96^3), 0.11 / 0.15 (64^3 / 90 x 128^2), 0.14 / 0.18 (48^3), but 0.028 /
-// 0.017 ms (16 x 20 x 24), 4.0 / 1.3 ms for a slab of 32 slices under 384 rows
-// 1.3 / 0.18 ms for voxels below a pixel (0.64; more than two candidates) and
-// 0.47 / 0.44 ms for voxels of 6.7 pixels (most pixels of a column wasted; 1.1 /
-// 1.5 ms at 3.3).
-// With the geometry gradients the scatter shares its march with theirs: 20.4 /
-// 24.4 ms at 256^3, 1.89 / 2.06 at 128^3, but 0.48 / 0.44 at 96^3.
-bool bp_gathers(const BpArgs& p, bool with_geometry) {
+// Gather or scatter?  The scatter's work is the voxels; the gather's the columns
+// times the detector's rows and, beside them, its lists: per (bin, row of the volume)
+// whatever there is to find.  So it wants deep columns, many of them in a bin and
+// views enough to fill the chip; what it wants of the magnification the views know
+// (bp_view_choice_kernel).  Measured over 506 random scans and cubes (20 to 300 voxels a
+// side, 1 to 400 views, 1.1- to 6-fold magnification, voxels of 0.5 to 4 pixels, a
+// shadow of half to twice the detector), the projection gradient alone: the scans
+// that this takes to the gather need 0.58 to 1.5 times the scatter's time, 1.9 below
+// 20000 columns x views (30 us, half of them launches; the sums are reproducible
+// there too) and 1.2 at most above 0.1 ms.  A rule by sizes and voxel / pixel alone took 181 of
+// them, of which 123 were slower, up to 12 times.  Gather / scatter: 10.0 / 18.5 ms
+// (256^3 / 360 x 384^2), 1.07 / 1.63 (128^3 / 180 x 256^2), 0.103 / 0.142 (64^3 / 90 x
+// 117^2); with 4 views 0.78 to 2.1 times.
+// With the geometry gradients the scatter shares its march with theirs, and the gather
+// gains only on large volumes: 20.4 / 24.4 ms at 256^3 / 360 x 384^2, 1.81 / 1.98 at
+// 128^3 / 180 x 234^2, but 1.1 to 1.9 times slower below the line drawn here.  What a
+// launch that was not taken costs: 10-30 us.
+bool bp_may_gather(const BpArgs& p, bool with_geometry) {
     const long long area = (long long)p.H * p.W;
-    return p.voxel_size >= 0.75f * p.pixel_size && p.voxel_size <= 3.0f * p.pixel_size &&
-           bp_shadow(p) >= 0.6f * p.V && area >= (with_geometry ? 128 * 128 : 32 * 32);
+    if (with_geometry)
+        return p.D >= 100 && p.V >= 48 && area >= 25LL * (p.U - 1) && area * p.A >= 1600000;
+    return p.A >= 6 && p.D >= 48 && p.V >= 48 && area >= 15LL * (p.U - 1);
+}
+
+int bp_view_choice(const Geometry& g, const BpArgs& p, bool with_geometry, ViewRow* vt,
+                   cudaStream_t s) {
+    DGC_TRACE("bp_view_choice", s);
+    bp_view_choice_kernel<<<1, 256, 0, s>>>(g, p, with_geometry ? 0.9f : 0.75f, vt);
+    DGC_LAUNCH_CHECK("bp_view_choice");
+    return DGC_OK;
 }
 
 int bp_launch_gather(const BpArgs& p, float* columns, cudaStream_t s) {
     {
         DGC_TRACE("bp_columns", s);
         const dim3 grid((unsigned)(ceil_div(p.W, 32) * (long long)p.H), (unsigned)ceil_div(p.D + 3, 32));
-        bp_columns_kernel<<<grid, dim3(32, 8), 0, s>>>(p.grad_volume, p.D, p.H, p.W, columns);
+        bp_columns_kernel<<<grid, dim3(32, 8), 0, s>>>(p.grad_volume, p.D, p.H, p.W, p.vt,
+                                                     columns);
         DGC_LAUNCH_CHECK("bp_columns");
     }
     DGC_TRACE("bp_adjoint_kernel", s);
     // pixels a thread and warps a CTA: the fewest idle slots, a column's own
     // instructions (about 10) against 25 a pixel; a warp that the volume's shadow
-    // does not reach costs little
-    const float shadow = bp_shadow(p);
+    // does not reach costs little (its rows at about twofold magnification: the host
+    // does not know the views')
+    const float shadow = 2.2f * p.D * p.voxel_size * p.inv_pixel;
     int nv = 1, warps = 1, tiles = 1;
     float best = FLT_MAX;
     for (int n = 1; n <= 3; ++n) {
@@ -1189,9 +1245,10 @@ int bp_launch_gather(const BpArgs& p, float* columns, cudaStream_t s) {
             tiles = t;
         }
     }
-    // bins per CTA: up to 16, as many as leave every SM some 32 CTAs
+    // bins per CTA: up to 16, as many as leave every SM some 32 CTAs (one instead of
+    // two where even these leave fewer: 0.6-0.9 of the time with 1 to 16 views)
     int bins = 16;
-    while (bins > 2 && (long long)p.A * ceil_div(p.U - 1, bins) * tiles < 148LL * 32) bins >>= 1;
+    while (bins > 1 && (long long)p.A * ceil_div(p.U - 1, bins) * tiles < 148LL * 32) bins >>= 1;
     const int bin_blocks = ceil_div(p.U - 1, bins);
     const unsigned grid = (unsigned)((long long)p.A * bin_blocks * tiles);
     const size_t smem = (size_t)warps * kAdjList * (sizeof(AdjColumn) + sizeof(unsigned));

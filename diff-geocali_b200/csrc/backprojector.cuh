@@ -15,7 +15,8 @@ struct ViewRow {
     float ds_u, ds_n;    // source offset in the rotating detector frame
     float ds_v;          // src_z
     float sod, sid, u0, v0;
-    float pad0, pad1, pad2;
+    int gather;          // of all rows: the projection gradient is gathered (bp_view_choice)
+    float pad1, pad2;
 };
 
 struct BpArgs {
@@ -34,16 +35,22 @@ struct BpArgs {
     const float* grad_volume;  // [D][H][W]
     float* grad_projections;   // [A][U][V], zeroed by the caller; null: not computed
     double* partials;          // [A][8][blocks]; null: no geometry gradients
+    int only_if;               // 0 or 1: the kernels run only where the rows' `gather` is that; -1
 };
 
 int bp_view_table(const Geometry& g, int A, ViewRow* vt, cudaStream_t s);
 int build_proj_quads(const float* P, int A, int U, int V, float4* PQ, cudaStream_t s);
 int bp_launch_forward(const BpArgs& p, bool fdk, cudaStream_t s);
 int bp_launch_backward(const BpArgs& p, cudaStream_t s);
-// Projection gradient as a gather (where bp_gathers says so): the upstream volume
-// as z-fastest columns (scratch of bp_column_floats), then every pixel of
-// p.grad_projections (zeroed).
-bool bp_gathers(const BpArgs& p, bool with_geometry);
+// Projection gradient as a gather: where the sizes allow it (bp_may_gather) the
+// views decide on the device, into their table (bp_view_choice, in place of
+// bp_view_table), and if they do, the upstream volume is laid out as z-fastest columns
+// (scratch of bp_column_floats) and every pixel of p.grad_projections (zeroed)
+// gathered.  If they do not, bp_launch_gather's kernels return at once; launch
+// bp_launch_backward with only_if = 0 for that.
+bool bp_may_gather(const BpArgs& p, bool with_geometry);
+int bp_view_choice(const Geometry& g, const BpArgs& p, bool with_geometry, ViewRow* vt,
+                   cudaStream_t s);
 size_t bp_column_floats(int D, int H, int W);
 int bp_launch_gather(const BpArgs& p, float* columns, cudaStream_t s);
 int bp_clamp_volume(float* volume, long long n, cudaStream_t s);

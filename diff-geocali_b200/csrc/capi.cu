@@ -110,6 +110,7 @@ BpArgs bp_args(const ViewRow* vt, const float4* pq, int A, int U, int V, int D, 
     p.W = W;
     p.pixel_size = pixel_size;
     p.inv_pixel = 1.0f / pixel_size;
+    p.only_if = -1;
     p.voxel_size = voxel_size;
     p.off_x = ox;
     p.off_y = oy;
@@ -515,21 +516,27 @@ int dgc_backproject_backward(const float* grad_volume, const float* projections,
                   " bytes");
         return DGC_ERR_WORKSPACE;
     }
-    if ((rc = bp_view_table(g, A, vt, s)) != DGC_OK) return rc;
     BpArgs p = bp_args(vt, pq, A, U, V, D, H, W, pixel_size, voxel_size, off_x, off_y, off_z);
+    const bool gather = grad_projections && bp_may_gather(p, true);
+    rc = gather ? bp_view_choice(g, p, true, vt, s) : bp_view_table(g, A, vt, s);
+    if (rc != DGC_OK) return rc;
     if (grad_projections) {
         p.grad_volume = grad_volume;
         p.grad_projections = grad_projections;
         DGC_CUDA(cudaMemsetAsync(grad_projections, 0, sizeof(float) * (size_t)A * U * V, s));
-        if (bp_gathers(p, true)) {
-            if ((rc = bp_launch_gather(p, columns, s)) != DGC_OK) return rc;
-            p.grad_projections = nullptr;  // done: the geometry gradients alone remain
-        }
+        if (gather && (rc = bp_launch_gather(p, columns, s)) != DGC_OK) return rc;
     }
     if ((rc = build_proj_quads(projections, A, U, V, pq, s)) != DGC_OK) return rc;
     p.grad_volume = grad_volume;
     p.partials = partials;
     p.kz_backward = kz;
+    if (gather) {
+        BpArgs rest = p;  // gathered: the geometry gradients alone remain
+        rest.grad_projections = nullptr;
+        rest.only_if = 1;
+        if ((rc = bp_launch_backward(rest, s)) != DGC_OK) return rc;
+        p.only_if = 0;
+    }
     if ((rc = bp_launch_backward(p, s)) != DGC_OK) return rc;
     return bp_reduce_partials(partials, A, nblocks, out, s);
 }
@@ -562,12 +569,18 @@ int dgc_backproject_adjoint(const float* grad_volume, int A, int U, int V, const
                   std::to_string(dgc_backproject_adjoint_workspace_bytes(A, D, H, W)) + " bytes");
         return DGC_ERR_WORKSPACE;
     }
-    if ((rc = bp_view_table(g, A, vt, s)) != DGC_OK) return rc;
     BpArgs p = bp_args(vt, nullptr, A, U, V, D, H, W, pixel_size, voxel_size, off_x, off_y, off_z);
+    const bool gather = bp_may_gather(p, false);
+    rc = gather ? bp_view_choice(g, p, false, vt, s) : bp_view_table(g, A, vt, s);
+    if (rc != DGC_OK) return rc;
     p.grad_volume = grad_volume;
     p.grad_projections = grad_projections;
     DGC_CUDA(cudaMemsetAsync(grad_projections, 0, sizeof(float) * (size_t)A * U * V, s));
-    return bp_gathers(p, false) ? bp_launch_gather(p, columns, s) : bp_launch_backward(p, s);
+    if (gather) {
+        if ((rc = bp_launch_gather(p, columns, s)) != DGC_OK) return rc;
+        p.only_if = 0;
+    }
+    return bp_launch_backward(p, s);
 }
 
 // --------------------------------------------------------------------- FDK

@@ -1202,11 +1202,10 @@ size_t bp_column_floats(int D, int H, int W) { return (size_t)(D + 3) * H * W; }
 // gains only on large volumes: 20.4 / 24.4 ms at 256^3 / 360 x 384^2, 1.81 / 1.98 at
 // 128^3 / 180 x 234^2, but 1.1 to 1.9 times slower below the line drawn here.  What a
 // launch that was not taken costs: 10-30 us.
-bool bp_may_gather(const BpArgs& p, bool with_geometry) {
-    const long long area = (long long)p.H * p.W;
-    if (with_geometry)
-        return p.D >= 100 && p.V >= 48 && area >= 25LL * (p.U - 1) && area * p.A >= 1600000;
-    return p.A >= 6 && p.D >= 48 && p.V >= 48 && area >= 15LL * (p.U - 1);
+bool bp_may_gather(int A, int U, int V, int D, int H, int W, bool with_geometry) {
+    const long long area = (long long)H * W;
+    if (with_geometry) return D >= 100 && V >= 48 && area >= 25LL * (U - 1) && area * A >= 1600000;
+    return A >= 6 && D >= 48 && V >= 48 && area >= 15LL * (U - 1);
 }
 
 int bp_view_choice(const Geometry& g, const BpArgs& p, bool with_geometry, ViewRow* vt,

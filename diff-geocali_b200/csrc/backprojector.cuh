@@ -48,7 +48,7 @@ int bp_launch_backward(const BpArgs& p, cudaStream_t s);
 // (scratch of bp_column_floats) and every pixel of p.grad_projections (zeroed)
 // gathered.  If they do not, bp_launch_gather's kernels return at once; launch
 // bp_launch_backward with only_if = 0 for that.
-bool bp_may_gather(const BpArgs& p, bool with_geometry);
+bool bp_may_gather(int A, int U, int V, int D, int H, int W, bool with_geometry);
 int bp_view_choice(const Geometry& g, const BpArgs& p, bool with_geometry, ViewRow* vt,
                    cudaStream_t s);
 size_t bp_column_floats(int D, int H, int W);

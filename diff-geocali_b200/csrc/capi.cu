@@ -471,16 +471,20 @@ int dgc_backproject(const float* projections, int A, int U, int V, const float* 
     return bp_launch_forward(p, false, s);
 }
 
-size_t dgc_backproject_backward_workspace_bytes(int A, int U, int V, int D, int H, int W) {
+size_t dgc_backproject_backward_least_workspace_bytes(int A, int U, int V, int D, int H, int W) {
     if (A <= 0 || U < 2 || V < 2 || D <= 0 || H <= 0 || W <= 0) return 0;
+    return bp_table_bytes(A) + bp_quads_bytes(A, U, V) +
+           Workspace::align(sizeof(double) * 8 * (size_t)A *
+                            (size_t)bp_backward_blocks(D, H, W, bp_kz_backward(D, A)));
+}
+
+size_t dgc_backproject_backward_workspace_bytes(int A, int U, int V, int D, int H, int W) {
+    const size_t least = dgc_backproject_backward_least_workspace_bytes(A, U, V, D, H, W);
+    if (!least || !bp_may_gather(A, U, V, D, H, W, true)) return least;
     // the projection gradient as a gather is done with its columns before the
     // quads and partials of the geometry gradients are written in their place
     const size_t columns = Workspace::align(sizeof(float) * bp_column_floats(D, H, W));
-    const size_t geometry =
-        bp_quads_bytes(A, U, V) +
-        Workspace::align(sizeof(double) * 8 * (size_t)A *
-                         (size_t)bp_backward_blocks(D, H, W, bp_kz_backward(D, A)));
-    return bp_table_bytes(A) + std::max(columns, geometry);
+    return std::max(least, bp_table_bytes(A) + columns);
 }
 
 int dgc_backproject_backward(const float* grad_volume, const float* projections, int A, int U,
@@ -507,17 +511,19 @@ int dgc_backproject_backward(const float* grad_volume, const float* projections,
     Workspace ws(workspace, workspace_bytes);
     ViewRow* vt = ws.take<ViewRow>((size_t)A);
     Workspace ws_columns = ws;  // shares its memory with the quads and partials
-    float* columns = grad_projections ? ws_columns.take<float>(bp_column_floats(D, H, W)) : nullptr;
+    float* columns = grad_projections && bp_may_gather(A, U, V, D, H, W, true)
+                         ? ws_columns.take<float>(bp_column_floats(D, H, W))
+                         : nullptr;
     float4* pq = ws.take<float4>((size_t)A * (U - 1) * (V - 1));
     double* partials = ws.take<double>((size_t)8 * A * nblocks);
-    if (!vt || !pq || !partials || (grad_projections && !columns)) {
+    if (!vt || !pq || !partials) {
         set_error("workspace too small: dgc_backproject_backward needs " +
-                  std::to_string(dgc_backproject_backward_workspace_bytes(A, U, V, D, H, W)) +
+                  std::to_string(dgc_backproject_backward_least_workspace_bytes(A, U, V, D, H, W)) +
                   " bytes");
         return DGC_ERR_WORKSPACE;
     }
     BpArgs p = bp_args(vt, pq, A, U, V, D, H, W, pixel_size, voxel_size, off_x, off_y, off_z);
-    const bool gather = grad_projections && bp_may_gather(p, true);
+    const bool gather = columns != nullptr;
     rc = gather ? bp_view_choice(g, p, true, vt, s) : bp_view_table(g, A, vt, s);
     if (rc != DGC_OK) return rc;
     if (grad_projections) {
@@ -543,9 +549,16 @@ int dgc_backproject_backward(const float* grad_volume, const float* projections,
 
 // --------------------------------------------- projection gradient alone
 
+size_t dgc_backproject_adjoint_least_workspace_bytes(int A) {
+    return A > 0 ? bp_table_bytes(A) : 0;
+}
+
 size_t dgc_backproject_adjoint_workspace_bytes(int A, int D, int H, int W) {
     if (A <= 0 || D <= 0 || H <= 0 || W <= 0) return 0;
-    return bp_table_bytes(A) + Workspace::align(sizeof(float) * bp_column_floats(D, H, W));
+    // for the smallest detector that a gather takes: the most columns that may be needed
+    return bp_table_bytes(A) + (bp_may_gather(A, 2, 1 << 30, D, H, W, false)
+                                    ? Workspace::align(sizeof(float) * bp_column_floats(D, H, W))
+                                    : 0);
 }
 
 int dgc_backproject_adjoint(const float* grad_volume, int A, int U, int V, const float* angles,
@@ -563,14 +576,16 @@ int dgc_backproject_adjoint(const float* grad_volume, int A, int U, int V, const
     DGC_REQUIRE(grad_volume && grad_projections, "grad_vol and grad_proj must be non-null");
     Workspace ws(workspace, workspace_bytes);
     ViewRow* vt = ws.take<ViewRow>((size_t)A);
-    float* columns = ws.take<float>(bp_column_floats(D, H, W));
-    if (!vt || !columns) {
+    float* columns = bp_may_gather(A, U, V, D, H, W, false)
+                         ? ws.take<float>(bp_column_floats(D, H, W))
+                         : nullptr;
+    if (!vt) {
         set_error("workspace too small: dgc_backproject_adjoint needs " +
-                  std::to_string(dgc_backproject_adjoint_workspace_bytes(A, D, H, W)) + " bytes");
+                  std::to_string(dgc_backproject_adjoint_least_workspace_bytes(A)) + " bytes");
         return DGC_ERR_WORKSPACE;
     }
     BpArgs p = bp_args(vt, nullptr, A, U, V, D, H, W, pixel_size, voxel_size, off_x, off_y, off_z);
-    const bool gather = bp_may_gather(p, false);
+    const bool gather = columns != nullptr;
     rc = gather ? bp_view_choice(g, p, false, vt, s) : bp_view_table(g, A, vt, s);
     if (rc != DGC_OK) return rc;
     p.grad_volume = grad_volume;

@@ -65,9 +65,11 @@ SIGNATURES = {
     "dgc_backproject_workspace_bytes": (_S, [_I] * 6),
     "dgc_backproject": (_I, [_P, _I, _I, _I, *_GEOM, _F, _I, _I, _I, _F, _F, _F, _F, _P, _P, _S, _P]),
     "dgc_backproject_backward_workspace_bytes": (_S, [_I] * 6),
+    "dgc_backproject_backward_least_workspace_bytes": (_S, [_I] * 6),
     "dgc_backproject_backward": (_I, [_P, _P, _I, _I, _I, *_GEOM, _F, _I, _I, _I, _F, _F, _F, _F,
                                       *([_P] * 9), _P, _S, _P]),
     "dgc_backproject_adjoint_workspace_bytes": (_S, [_I] * 4),
+    "dgc_backproject_adjoint_least_workspace_bytes": (_S, [_I]),
     "dgc_backproject_adjoint": (_I, [_P, _I, _I, _I, *_GEOM, _F, _I, _I, _I, _F, _F, _F, _F, _P, _P,
                                      _S, _P]),
     "dgc_fdk_filter_taps": (_I, [_I, _D, _D, ctypes.POINTER(_D)]),

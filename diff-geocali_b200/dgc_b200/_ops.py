@@ -35,6 +35,15 @@ def _workspace(nbytes: int, device) -> torch.Tensor | None:
     return torch.empty(int(nbytes), dtype=torch.uint8, device=device)
 
 
+def _workspace_or_least(nbytes: int, least: int, device):
+    """Workspace of ``nbytes`` or, where the device has no room for it, of the ``least``
+    that the call takes."""
+    try:
+        return _workspace(nbytes, device)
+    except torch.cuda.OutOfMemoryError:
+        return _workspace(least, device)
+
+
 def _filter_workspace(nbytes: int, A: int, U: int, V: int, adjoint: bool, device):
     """Workspace of the FDK filter: what the library asks for or, where the device has no
     room for the split operands of the tensor cores, the taps (and the adjoint's sums,
@@ -268,7 +277,8 @@ def bp_backward(grad_vol, proj, angles, sid, sod, det_u0_arr, det_v0_arr, src_x_
     lib = _native.lib()
     if compute_grad_proj and not compute_grad_geometry:
         with torch.cuda.device(dev):
-            ws = _workspace(lib.dgc_backproject_adjoint_workspace_bytes(A, D, H, W), dev)
+            ws = _workspace_or_least(lib.dgc_backproject_adjoint_workspace_bytes(A, D, H, W),
+                                     lib.dgc_backproject_adjoint_least_workspace_bytes(A), dev)
             _native.check(lib.dgc_backproject_adjoint(
                 gv.data_ptr(), A, U, V, *[g.data_ptr() for g in geom], pixel_size, D, H, W,
                 voxel_size, off_x, off_y, off_z, grad_proj.data_ptr(), _p(ws),
@@ -276,7 +286,9 @@ def bp_backward(grad_vol, proj, angles, sid, sod, det_u0_arr, det_v0_arr, src_x_
         return [grad_proj, *[None] * 8]
     grads = [torch.empty_like(g) for g in geom]
     with torch.cuda.device(dev):
-        ws = _workspace(lib.dgc_backproject_backward_workspace_bytes(A, U, V, D, H, W), dev)
+        ws = _workspace_or_least(
+            lib.dgc_backproject_backward_workspace_bytes(A, U, V, D, H, W),
+            lib.dgc_backproject_backward_least_workspace_bytes(A, U, V, D, H, W), dev)
         _native.check(lib.dgc_backproject_backward(
             gv.data_ptr(), p.data_ptr(), A, U, V, *[g.data_ptr() for g in geom], pixel_size, D, H,
             W, voxel_size, off_x, off_y, off_z, _p(grad_proj),

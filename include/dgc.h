@@ -133,8 +133,12 @@ int dgc_backproject(const float* projections, int A, int U, int V,
                     float* volume,
                     void* workspace, size_t workspace_bytes, void* stream);
 
-/* Scratch of dgc_backproject_backward. */
+/* Scratch of dgc_backproject_backward: what it uses best, and the least that it takes.
+ * Where the two differ (deep volumes under few views), the larger one holds a copy
+ * of the volume for the projection gradient as a gather; with less, it is a scatter:
+ * the same products, added in another order. */
 size_t dgc_backproject_backward_workspace_bytes(int A, int U, int V, int D, int H, int W);
+size_t dgc_backproject_backward_least_workspace_bytes(int A, int U, int V, int D, int H, int W);
 
 /* Replaces src_cbct_backprojector_cuda.backward
  * (csrc/src_cbct_backprojector_cuda.cu:423-522, kernel 101-295).
@@ -154,8 +158,10 @@ int dgc_backproject_backward(const float* grad_volume, const float* projections,
                              float* grad_src_x, float* grad_src_y, float* grad_src_z,
                              void* workspace, size_t workspace_bytes, void* stream);
 
-/* Scratch of dgc_backproject_adjoint. */
+/* Scratch of dgc_backproject_adjoint: what it uses best, and the least that it takes
+ * (without the gather's copy of the volume, as for dgc_backproject_backward). */
 size_t dgc_backproject_adjoint_workspace_bytes(int A, int D, int H, int W);
+size_t dgc_backproject_adjoint_least_workspace_bytes(int A);
 
 /* The projection gradient of dgc_backproject alone (dgc_backproject_backward
  * without the geometry gradients, which an autograd call with fixed geometry

@@ -211,3 +211,60 @@ def test_a_view_without_numbers_contributes_nothing():
     want, gathered = chosen(proj, geom, up, case)
     assert gathered == 1
     assert rel_l2(got[4:].cpu(), want[4:].cpu()) < SAME_RTOL
+
+
+@pytest.mark.parametrize("geometry", [False, True])
+def test_without_room_for_the_columns(geometry, monkeypatch):
+    """No device memory for the gather's copy of the volume: the scatter, in the room
+    that the view table (and the quads and sums of the geometry gradients) takes."""
+    from dgc_b200 import _native, _ops
+
+    case = ((100, 283, 284), 12, 100, 1.0, 1.0, 900.0, 600.0, (0.0, 0.0, 0.0))
+    (D, H, W), U, V = case[:3]
+    A = 20
+    proj, geom, up = make(case, A=A)
+    want = gradients(proj, geom, up, case, geometry)
+    lib = _native.lib()
+    most, least = ((lib.dgc_backproject_backward_workspace_bytes(A, U, V, D, H, W),
+                    lib.dgc_backproject_backward_least_workspace_bytes(A, U, V, D, H, W)) if geometry else
+                   (lib.dgc_backproject_adjoint_workspace_bytes(A, D, H, W),
+                    lib.dgc_backproject_adjoint_least_workspace_bytes(A)))
+    assert most >= 4 * D * H * W > least
+    asked, room = [], _ops._workspace
+
+    def tight(nbytes, device):
+        if nbytes == most:
+            asked.append(nbytes)
+            raise torch.cuda.OutOfMemoryError("no room")
+        return room(nbytes, device)
+
+    monkeypatch.setattr(_ops, "_workspace", tight)
+    got = gradients(proj, geom, up, case, geometry)
+    assert asked == [most]
+    assert rel_l2(got[0].cpu(), want[0].cpu()) < SAME_RTOL
+    assert all(torch.equal(a, b) for a, b in zip(got[1:], want[1:]))
+
+
+def test_least_workspace():
+    """dgc_backproject_adjoint in the least workspace, and refused below it."""
+    from dgc_b200 import _native
+
+    case = GATHERED[1]
+    (D, H, W), U, V, px, vs, sid, sod, off = case
+    proj, geom, up = make(case)
+    want, gathered = chosen(proj, geom, up, case)
+    assert gathered == 1
+    lib, A = _native.lib(), proj.shape[0]
+    n = lib.dgc_backproject_adjoint_least_workspace_bytes(A)
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    out = torch.empty_like(want)
+    g, u = [cuda(x) for x in geom], cuda(up)
+
+    def call(nbytes):
+        return lib.dgc_backproject_adjoint(
+            u.data_ptr(), A, U, V, *[x.data_ptr() for x in g], px, D, H, W, vs, *off, out.data_ptr(),
+            ws.data_ptr(), nbytes, torch.cuda.current_stream().cuda_stream)
+
+    assert call(n) == 0
+    assert rel_l2(out.cpu(), want.cpu()) < SAME_RTOL
+    assert call(n - 256) == 3

@@ -612,9 +612,24 @@ int dgc_fdk_filter_taps(int U, double pixel_size, double alpha, double* taps) {
     return DGC_OK;
 }
 
+// The taps and, of the adjoint, its sums: what the FP32 product takes.
+static size_t filter_base_bytes(int A, int U, int V, bool adjoint) {
+    return Workspace::align(sizeof(float) * (size_t)U) +
+           (adjoint ? Workspace::align(sizeof(double) * kFdkPartials * (size_t)A *
+                                       (size_t)fdk_filter_tiles(U, V))
+                    : 0);
+}
+
 size_t dgc_fdk_filter_workspace_bytes(int A, int U, int V) {
     if (U <= 0) return 0;
-    return Workspace::align(sizeof(float) * (size_t)U) + fdk_tc_bytes(A, U, V, false);
+    return filter_base_bytes(A, U, V, false) + fdk_tc_bytes(A, U, V, false);
+}
+
+size_t dgc_fdk_filter_workspace_bytes_at_a_time(int A, int U, int V, int adjoint, int views) {
+    if (A <= 0 || U <= 0 || V <= 0 || views < 0) return 0;
+    const int most = fdk_tc_views(A, U, V);
+    return filter_base_bytes(A, U, V, adjoint != 0) +
+           (views && most ? fdk_tc_scratch(U, V, adjoint != 0, std::min(views, most)) : 0);
 }
 
 // The filter of every view: on the tensor cores where the sizes are theirs and
@@ -669,10 +684,7 @@ int dgc_fdk_filter(const float* projections, int A, int U, int V, float pixel_si
 
 size_t dgc_fdk_filter_backward_workspace_bytes(int A, int U, int V) {
     if (A <= 0 || U <= 0 || V <= 0) return 0;
-    return Workspace::align(sizeof(float) * (size_t)U) +
-           Workspace::align(sizeof(double) * kFdkPartials * (size_t)A *
-                            (size_t)fdk_filter_tiles(U, V)) +
-           fdk_tc_bytes(A, U, V, true);
+    return filter_base_bytes(A, U, V, true) + fdk_tc_bytes(A, U, V, true);
 }
 
 int dgc_fdk_filter_backward_ex(const float* grad_filtered, const float* projections,

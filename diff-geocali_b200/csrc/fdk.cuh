@@ -49,10 +49,12 @@ int fdk_launch_filter(const FdkArgs& p, cudaStream_t s);
 long long fdk_filter_tiles(int U, int V);
 int fdk_launch_filter_adjoint(const FdkArgs& p, cudaStream_t s);
 // The filter's product on the tensor cores (fdk_tc.cu): views held at a time (0:
-// the sizes are not its), scratch, and the filter or the adjoint with its sums;
-// *used false: nothing was done.
+// the sizes are not its), scratch for these or for some, and the filter or the
+// adjoint with its sums, with as many views at a time as ws holds; *used false:
+// nothing was done.
 int fdk_tc_views(int A, int U, int V);
 size_t fdk_tc_bytes(int A, int U, int V, bool adjoint);
+size_t fdk_tc_scratch(int U, int V, bool adjoint, int views);
 int fdk_tc_filter(const FdkArgs& p, bool adjoint, Workspace ws, cudaStream_t s, bool* used);
 // Per-view gradients from the partials: sod, sid, and, where the frame was
 // given, its distance and centres (any output may be null).

@@ -673,18 +673,34 @@ int fdk_tc_views(int A, int U, int V) {
     return ceil_div(A, ceil_div(A, most));  // equal chunks
 }
 
-size_t fdk_tc_bytes(int A, int U, int V, bool adjoint) {
-    const int views = fdk_tc_views(A, U, V);
-    if (!views) return 0;
+size_t fdk_tc_scratch(int U, int V, bool adjoint, int views) {
     return Workspace::align(3 * 128 * (size_t)tc_cores(U)) +
            Workspace::align(sizeof(FdkRange) * (size_t)views * (size_t)ceil_div(U, 8)) +
            Workspace::align(tc_split_bytes(U, V) * (size_t)views) +
            (adjoint ? Workspace::align(sizeof(float) * (size_t)U * V * (size_t)views) : 0);
 }
 
+size_t fdk_tc_bytes(int A, int U, int V, bool adjoint) {
+    const int views = fdk_tc_views(A, U, V);
+    return views ? fdk_tc_scratch(U, V, adjoint, views) : 0;
+}
+
+// Views at a time: those of the rule or, in less room, as many as it holds (a view's
+// result is the same whatever their number).
+static int views_that_fit(const FdkArgs& p, bool adjoint, const Workspace& ws) {
+    const size_t room = ws.base ? ws.size - ws.used : 0;
+    int low = 0, high = fdk_tc_views(p.A, p.U, p.V);
+    if (!high || fdk_tc_scratch(p.U, p.V, adjoint, high) <= room) return high;
+    while (low + 1 < high) {
+        const int mid = (low + high) / 2;
+        (fdk_tc_scratch(p.U, p.V, adjoint, mid) <= room ? low : high) = mid;
+    }
+    return low;
+}
+
 int fdk_tc_filter(const FdkArgs& p, bool adjoint, Workspace ws, cudaStream_t s, bool* used) {
     *used = false;
-    const int views = fdk_tc_views(p.A, p.U, p.V);
+    const int views = views_that_fit(p, adjoint, ws);
     if (!views) return DGC_OK;
     __nv_bfloat16* strip = ws.take<__nv_bfloat16>((size_t)3 * 64 * (size_t)tc_cores(p.U));
     FdkRange* ranges = ws.take<FdkRange>((size_t)views * (size_t)ceil_div(p.U, 8));

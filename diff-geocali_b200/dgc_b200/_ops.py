@@ -46,13 +46,15 @@ def _workspace_or_least(nbytes: int, least: int, device):
 
 def _filter_workspace(nbytes: int, A: int, U: int, V: int, adjoint: bool, device):
     """Workspace of the FDK filter: what the library asks for or, where the device has no
-    room for the split operands of the tensor cores, the taps (and the adjoint's sums,
-    four doubles per view and 128 x 128 tile) that its FP32 product needs."""
-    try:
-        return _workspace(nbytes, device)
-    except torch.cuda.OutOfMemoryError:
-        sums = 32 * A * (-(-U // 128)) * (-(-V // 128)) if adjoint else 0
-        return _workspace(-(-4 * U // 256) * 256 + -(-sums // 256) * 256, device)
+    room for it, for one view at a time on the tensor cores (the same results) and
+    at last for the FP32 product (the same but for rounding)."""
+    for views in (1, 0):
+        try:
+            return _workspace(nbytes, device)
+        except torch.cuda.OutOfMemoryError:
+            nbytes = _native.lib().dgc_fdk_filter_workspace_bytes_at_a_time(A, U, V, int(adjoint),
+                                                                            views)
+    return _workspace(nbytes, device)
 
 
 def _p(t):

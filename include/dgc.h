@@ -184,8 +184,15 @@ int dgc_backproject_adjoint(const float* grad_volume, int A, int U, int V,
  * filter (filtering.py:87-103) as a symmetric Toeplitz kernel, FP64. */
 int dgc_fdk_filter_taps(int U, double pixel_size, double alpha, double* taps);
 
-/* Scratch of dgc_fdk_filter. */
+/* Scratch of dgc_fdk_filter.  For U from 96 to 2048 (and V >= 16) the filter runs on
+ * the tensor cores, and the workspace holds the split operands of up to 256 MB of
+ * views; a smaller one is taken too.  ..._at_a_time is what the filter (adjoint 1:
+ * dgc_fdk_filter_backward) takes with `views` views at a time there: the results are
+ * the same bit for bit, whatever their number.  With room for none (views 0) the
+ * filter is an FP32 product, whose results differ by both products' rounding
+ * (relative L2 1e-7 to 4e-6, growing with U). */
 size_t dgc_fdk_filter_workspace_bytes(int A, int U, int V);
+size_t dgc_fdk_filter_workspace_bytes_at_a_time(int A, int U, int V, int adjoint, int views);
 
 /* Replaces cbct_backprojector.filtering.fdk_filter (filtering.py:54-104):
  * centred cosine preweight, ramp x Hann filter along U, pixel*sid/sod scale.
@@ -239,7 +246,8 @@ int dgc_fdk_filter_noalloc(const float* projections, int A, int U, int V, float 
                            const float* sod, const float* sid, float alpha,
                            float* filtered, void* stream);
 
-/* Scratch of dgc_fdk_filter_backward. */
+/* Scratch of dgc_fdk_filter_backward; a smaller workspace is taken as by
+ * dgc_fdk_filter. */
 size_t dgc_fdk_filter_backward_workspace_bytes(int A, int U, int V);
 
 /* Gradients of dgc_fdk_filter, which the reference's torch implementation of

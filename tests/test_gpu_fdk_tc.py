@@ -195,3 +195,69 @@ def test_columns_of_small_values_keep_their_precision(U, px):
     held(y, c * (H @ (w * x.double())), c * (H.abs() @ (w * x.double()).abs()))
     gp, _, _ = _ops.fdk_filter_backward(x, x, y, px, sod, sid, alpha)
     held(gp, c * w * (H @ x.double()), c * w * (H.abs() @ x.double().abs()))
+
+
+def in_room(p, g, y, sod, sid, dist, views):
+    """Filter and adjoint (its distance gradients too) of ``views`` views at a time."""
+    from dgc_b200 import _native
+
+    lib, (A, U, V) = _native.lib(), p.shape
+    out, gp = torch.empty_like(p), torch.empty_like(p)
+    gs = [torch.empty_like(sod) for _ in range(3)]
+    s = torch.cuda.current_stream().cuda_stream
+    n = lib.dgc_fdk_filter_workspace_bytes_at_a_time(A, U, V, 0, views)
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    _native.check(lib.dgc_fdk_filter_ex(
+        p.data_ptr(), A, U, V, 1.0, sod.data_ptr(), sid.data_ptr(), dist.data_ptr(), None, None, 0.8,
+        out.data_ptr(), ws.data_ptr(), n, s))
+    n = lib.dgc_fdk_filter_workspace_bytes_at_a_time(A, U, V, 1, views)
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    _native.check(lib.dgc_fdk_filter_backward_ex(
+        g.data_ptr(), p.data_ptr(), y.data_ptr(), A, U, V, 1.0, sod.data_ptr(), sid.data_ptr(),
+        dist.data_ptr(), None, None, 0.8, gp.data_ptr(), *[t.data_ptr() for t in gs], None, None,
+        ws.data_ptr(), n, s))
+    return [out, gp, *gs]
+
+
+@pytest.mark.parametrize("U,V", [(97, 17), (300, 203)])
+def test_fewer_views_at_a_time_give_the_same_bits(U, V):
+    from dgc_b200 import _native, _ops
+
+    A = 7
+    p, sid, sod = scan(A, U, V, 8)
+    g = torch.randn(p.shape, generator=torch.Generator().manual_seed(3)).cuda()
+    dist = sid * 0.97
+    y = _ops.fdk_filter_framed(p, 1.0, sod, sid, 0.8, (dist, None, None))
+    most = in_room(p, g, y, sod, sid, dist, A)
+    assert torch.equal(most[0], y)
+    for views in (1, 3, 6):
+        assert all(torch.equal(a, b) for a, b in zip(in_room(p, g, y, sod, sid, dist, views), most)), views
+    none = in_room(p, g, y, sod, sid, dist, 0)
+    assert not torch.equal(none[0], y)
+    lib = _native.lib()
+    sizes = [lib.dgc_fdk_filter_workspace_bytes_at_a_time(A, U, V, 0, v) for v in (0, 1, 3, A, A + 1)]
+    assert sizes == sorted(sizes) and sizes[-1] == sizes[-2] == lib.dgc_fdk_filter_workspace_bytes(A, U, V)
+
+
+def test_room_for_one_view(monkeypatch):
+    """The device has room for one view's split operands: the same bits."""
+    from dgc_b200 import _native, _ops
+
+    A, U, V = 5, 200, 150
+    p, sid, sod = scan(A, U, V, 6)
+    g = torch.randn(p.shape, generator=torch.Generator().manual_seed(2)).cuda()
+    want = _ops.fdk_filter(p, 1.0, sod, sid, 0.8)
+    grads = _ops.fdk_filter_backward(g, p, want, 1.0, sod, sid, 0.8)
+    lib, room = _native.lib(), _ops._workspace
+    limit = [lib.dgc_fdk_filter_workspace_bytes_at_a_time(A, U, V, 0, 1)]
+
+    def tight(nbytes, device):
+        if nbytes > limit[0]:
+            raise torch.cuda.OutOfMemoryError("no room")
+        return room(nbytes, device)
+
+    monkeypatch.setattr(_ops, "_workspace", tight)
+    assert torch.equal(_ops.fdk_filter(p, 1.0, sod, sid, 0.8), want)
+    limit[0] = lib.dgc_fdk_filter_workspace_bytes_at_a_time(A, U, V, 1, 1)
+    for a, b in zip(_ops.fdk_filter_backward(g, p, want, 1.0, sod, sid, 0.8), grads):
+        assert torch.equal(a, b)

@@ -241,7 +241,10 @@ int dgc_fdk_filter_ex(const float* projections, int A, int U, int V, float pixel
  * before its filter reads them, so nothing needs to start at zero, but all
  * calls share the one array: calls that overlap on the GPU (different
  * streams, no ordering between them) race on it.  Same inputs and outputs as
- * dgc_fdk_filter; results equal its within the taps' FP64 rounding. */
+ * dgc_fdk_filter.  Its product is the FP32 one at every U: the results equal those
+ * of dgc_fdk_filter with views 0 at a time within the taps' FP64 rounding, and where
+ * dgc_fdk_filter runs on the tensor cores they differ by both products' rounding and
+ * take longer (720 x 768 x 768: 15.8 against 3.8 ms). */
 int dgc_fdk_filter_noalloc(const float* projections, int A, int U, int V, float pixel_size,
                            const float* sod, const float* sid, float alpha,
                            float* filtered, void* stream);

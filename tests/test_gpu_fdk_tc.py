@@ -261,3 +261,27 @@ def test_room_for_one_view(monkeypatch):
     limit[0] = lib.dgc_fdk_filter_workspace_bytes_at_a_time(A, U, V, 1, 1)
     for a, b in zip(_ops.fdk_filter_backward(g, p, want, 1.0, sod, sid, 0.8), grads):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("U,px", [(96, 1.0), (384, 0.9), (2048, 1.3)])
+def test_noalloc_is_the_fp32_product(U, px):
+    """An impulse gives the taps, one product each: dgc_fdk_filter_noalloc's are those of the
+    FP32 product within a rounding of the FP64 taps to FP32 (2^-23 of a tap; an FP64
+    error of the DFT, 2^-50 of the largest)."""
+    from dgc_b200 import _native
+
+    lib, A, V = _native.lib(), 1, 16
+    p = torch.zeros((A, U, V), device="cuda")
+    p[0, U // 3] = 1.0
+    sid, sod = torch.full((A,), 1000.0, device="cuda"), torch.full((A,), 600.0, device="cuda")
+    got, want = torch.empty_like(p), torch.empty_like(p)
+    s = torch.cuda.current_stream().cuda_stream
+    _native.check(lib.dgc_fdk_filter_noalloc(p.data_ptr(), A, U, V, px, sod.data_ptr(), sid.data_ptr(),
+                                             0.8, got.data_ptr(), s))
+    n = lib.dgc_fdk_filter_workspace_bytes_at_a_time(A, U, V, 0, 0)
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    _native.check(lib.dgc_fdk_filter(p.data_ptr(), A, U, V, px, sod.data_ptr(), sid.data_ptr(), 0.8,
+                                     want.data_ptr(), ws.data_ptr(), n, s))
+    a, b = got.double(), want.double()
+    assert float(b.abs().max()) > 0
+    assert float(((a - b).abs() - 2.0**-22 * b.abs() - 2.0**-49 * b.abs().max()).max()) <= 0

@@ -1073,10 +1073,12 @@ void bp_clear_tile_rules() {
     g_rule_count = 0;
 }
 
+static int bp_nominal_kz(int D) { return D <= 32 ? 1 : 2; }
+
 int bp_kz_forward(int D, int A) {
     BpTileRule r;
     if (bp_rule(D, A, r) && r.kz_forward) return r.kz_forward;
-    return D <= 32 ? 1 : 2;
+    return bp_nominal_kz(D);
 }
 
 int bp_kz_backward(int D, int A) {
@@ -1137,23 +1139,30 @@ int launch_bp_backward_kz(const BpArgs& p, int gp, bool geo, dim3 grid, cudaStre
 }
 }  // namespace
 
+void bp_forward_tile(int D, int H, int W, int A, int& kz, int& cx, int& cy) {
+    BpTileRule r;
+    const bool asked = bp_rule(D, A, r) && (r.kz_forward || r.cta_x);
+    if (asked || (long long)ceil_div(W, 2) * ceil_div(H, 2) > INT_MAX) {
+        kz = asked && r.kz_forward ? r.kz_forward : bp_nominal_kz(D);
+        cx = asked && r.cta_x ? r.cta_x : 8;
+        cy = asked && r.cta_x ? r.cta_y : 1;
+        return;
+    }
+    // The kernel's own choice: 2 x 2 columns and the fewest blocks of up to 128 slices,
+    // each no deeper than it needs to be (KZ = 2 / 3 / 4, ms: 70 x 256^2, 180 views 1.62 /
+    // 1.21 / -, 96 x 128^2, 180 views 0.50 / 0.45 / -, 128^3 0.54 / 0.70 / 0.52, 160^3, 200
+    // views 1.12 / 1.08 / 1.29, 192^3, 360 views 3.37 / 3.45 / 3.85, 256^3 6.65 / 7.08 /
+    // 6.48)
+    cx = cy = 2;
+    kz = ceil_div(D, 32 * (long long)ceil_div(D, 128));
+}
+
 int bp_launch_forward(const BpArgs& args, bool fdk, cudaStream_t s) {
     DGC_TRACE(fdk ? "bp_forward_kernel<fdk>" : "bp_forward_kernel", s);
     BpArgs p = args;
-    bp_forward_cta(p.D, p.A, p.cta_x, p.cta_y);
+    int kz = 0;
+    bp_forward_tile(p.D, p.H, p.W, p.A, kz, p.cta_x, p.cta_y);
     const bool pixdiv = !is_pow2_float(p.pixel_size);
-    int kz = bp_kz_forward(p.D, p.A);
-    const long long blocks = (long long)ceil_div(p.W, 2) * ceil_div(p.H, 2);
-    if (p.cta_x == 8 && p.cta_y == 1 && kz == (p.D <= 32 ? 1 : 2) && blocks <= INT_MAX) {
-        // The built-in tile, from a rule or without one, stands for the kernel's own
-        // choice: 2 x 2 columns and the fewest blocks of up to 128 slices, each no
-        // deeper than it needs to be (KZ = 2 / 3 / 4, ms: 70 x 256^2, 180 views 1.62 /
-        // 1.21 / -, 96 x 128^2, 180 views 0.50 / 0.45 / -, 128^3 0.54 / 0.70 / 0.52,
-        // 160^3, 200 views 1.12 / 1.08 / 1.29, 192^3, 360 views 3.37 / 3.45 / 3.85,
-        // 256^3 6.65 / 7.08 / 6.48)
-        p.cta_x = p.cta_y = 2;
-        kz = ceil_div(p.D, 32 * (long long)ceil_div(p.D, 128));
-    }
     const dim3 grid((unsigned)(ceil_div(p.W, p.cta_x) * (long long)ceil_div(p.H, p.cta_y)),
                     (unsigned)ceil_div(p.D, 32 * kz));
     switch (kz) {

@@ -61,6 +61,9 @@ long long bp_backward_blocks(int D, int H, int W, int kz);
 int bp_kz_forward(int D, int A);
 int bp_kz_backward(int D, int A);
 void bp_forward_cta(int D, int A, int& cx, int& cy);
+// The forward tile that a call runs: the rule's or, without one, the kernel's own
+// choice (for which the two above report 8 x 1 columns and 32 or 64 slices).
+void bp_forward_tile(int D, int H, int W, int A, int& kz, int& cx, int& cy);
 int bp_add_tile_rule(int d_max, int a_max, int kz_forward, int kz_backward, int cta_x, int cta_y);
 void bp_clear_tile_rules();
 int bp_reduce_partials(const double* partials, int A, long long nblocks, const GeometryGrad& out,

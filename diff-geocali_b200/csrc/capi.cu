@@ -892,6 +892,14 @@ int dgc_bp_tiles(int D, int A, int* kz_forward, int* kz_backward, int* cta_x, in
     return DGC_OK;
 }
 
+int dgc_bp_forward_tile(int D, int H, int W, int A, int* kz, int* cta_x, int* cta_y) {
+    clear_error();
+    DGC_REQUIRE(D >= 1 && H >= 1 && W >= 1 && A >= 1, "D, H, W and A must be positive");
+    DGC_REQUIRE(kz && cta_x && cta_y, "output pointers must be non-null");
+    bp_forward_tile(D, H, W, A, *kz, *cta_x, *cta_y);
+    return DGC_OK;
+}
+
 int dgc_fp_add_arm_rule(long long voxels_max, int arm, int slab_cells, int unroll,
                         int view_block) {
     using namespace dgc;

@@ -97,6 +97,7 @@ SIGNATURES = {
     "dgc_clamp_volume": (_I, [_P, ctypes.c_longlong, _P]),
     "dgc_bp_add_tile_rule": (_I, [_I] * 6),
     "dgc_bp_clear_tile_rules": (_I, []),
+    "dgc_bp_forward_tile": (_I, [_I] * 4 + [ctypes.POINTER(ctypes.c_int)] * 3),
     "dgc_bp_tiles": (_I, [_I, _I] + [ctypes.POINTER(ctypes.c_int)] * 4),
     "dgc_gemm_bf16": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _P, _P]),
     "dgc_gemm_bf16_tn": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _P, _P]),

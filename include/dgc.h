@@ -366,18 +366,20 @@ int dgc_reconstruct_fdk_ex(const float* projections, int A, int U, int V,
  * call with volume depth D <= d_max and A <= a_max views uses Z blocking
  * kz_forward / kz_backward (32*kz voxels of a column per warp; 1, 2, 4 or 8,
  * 0 = built-in choice) and a cta_x x cta_y patch of columns per CTA in the
- * forward (both 0 = built-in 8 x 1; cta_x*cta_y <= 16).  The built-in forward
- * tile, kz_forward 1 up to depth 32 and 2 above with 8 x 1 columns, is nominal:
- * for it the kernel blocks the volume as suits its depth.  Rules are tried in
- * the order they were added (at most 16).  Results do not depend on the tiles
- * beyond float-summation order (the forward's not at all).  No counterpart in
+ * forward (both 0 = built-in 8 x 1; cta_x*cta_y <= 16).  The forward runs the tile
+ * that a rule asks for; without a rule, and with one whose three forward fields are
+ * zero, it blocks the volume as suits its sizes (dgc_bp_forward_tile).  Rules are
+ * tried in the order they were added (at most 16).  Results do not depend on the
+ * tiles beyond float-summation order (the forward's not at all).  No counterpart in
  * the reference. */
 int dgc_bp_add_tile_rule(int d_max, int a_max, int kz_forward, int kz_backward, int cta_x,
                          int cta_y);
 int dgc_bp_clear_tile_rules(void);
-/* The tiles a call with depth D and A views uses (the forward's built-in tile
- * nominally, see above). */
+/* The tiles a call with depth D and A views uses, from its rule; the forward's own
+ * choice is reported as 8 x 1 columns with kz_forward 1 up to depth 32 and 2 above. */
 int dgc_bp_tiles(int D, int A, int* kz_forward, int* kz_backward, int* cta_x, int* cta_y);
+/* The forward tile that a call on a [D][H][W] volume with A views runs. */
+int dgc_bp_forward_tile(int D, int H, int W, int A, int* kz, int* cta_x, int* cta_y);
 
 /* Forward-projector arm rules (what the autotuner chose per volume size): a
  * dgc_project of D*H*W <= voxels_max voxels runs arm 0 (quad loads through

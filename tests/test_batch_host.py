@@ -151,6 +151,36 @@ def test_backprojector_tile_rules(clean_bp_rules):
         _native.check(lib.dgc_bp_add_tile_rule(1024, 1024, 2, 4, 0, 0))
 
 
+def forward_tile(lib, D, H, W, A):
+    import ctypes
+
+    out = [ctypes.c_int() for _ in range(3)]
+    assert lib.dgc_bp_forward_tile(D, H, W, A, *[ctypes.byref(x) for x in out]) == 0
+    return out[0].value, (out[1].value, out[2].value)
+
+
+def test_backprojector_runs_the_tile_a_rule_asks_for(clean_bp_rules):
+    """Every tile, 8 x 1 columns of 32 or 64 slices among them, is the one that runs;
+    without a rule for the forward the kernel takes its own -- host only."""
+    lib = clean_bp_rules
+    own = forward_tile(lib, 256, 256, 256, 360)
+    assert own == (4, (2, 2))
+    asked = [(2, 8, 1), (1, 8, 1), (4, 8, 1), (2, 2, 2), (8, 16, 1), (4, 0, 0), (0, 4, 2), (0, 8, 1),
+             (2, 0, 0)]
+    for kz, cx, cy in asked:
+        lib.dgc_bp_clear_tile_rules()
+        assert lib.dgc_bp_add_tile_rule(256, 360, kz, 0, cx, cy) == 0
+        want = kz or 2, (cx, cy) if cx else (8, 1)
+        assert forward_tile(lib, 256, 256, 256, 360) == want
+        assert forward_tile(lib, 257, 256, 256, 360)[1] == (2, 2)  # beyond the rule
+    lib.dgc_bp_clear_tile_rules()
+    assert lib.dgc_bp_add_tile_rule(256, 360, 0, 8, 0, 0) == 0  # a rule for the backward alone
+    assert forward_tile(lib, 256, 256, 256, 360) == own
+    lib.dgc_bp_clear_tile_rules()
+    assert lib.dgc_bp_add_tile_rule(32, 10, 1, 0, 8, 1) == 0
+    assert forward_tile(lib, 20, 64, 64, 10) == (1, (8, 1))
+
+
 def test_autotuner_tunes_backprojector(clean_bp_rules, tmp_path):
     """Fastest forward (KZ, patch) and backward KZ per (depth, views) bucket,
     cached as JSON and registered as a library rule."""

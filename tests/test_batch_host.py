@@ -181,6 +181,16 @@ def test_backprojector_runs_the_tile_a_rule_asks_for(clean_bp_rules):
     assert forward_tile(lib, 20, 64, 64, 10) == (1, (8, 1))
 
 
+@pytest.mark.parametrize("D,H,W,kz", [
+    (353, 16, 7, 1), (91, 26, 31, 1), (228, 40, 22, 2), (128, 64, 64, 4), (64, 64, 64, 2),
+    (128, 37, 28, 1), (128, 37, 29, 2), (128, 37, 56, 2), (128, 37, 57, 4), (96, 45, 46, 2),
+    (96, 45, 47, 3), (32, 5, 5, 1), (256, 256, 256, 4), (160, 200, 200, 3)])
+def test_backprojector_fills_the_chip(clean_bp_rules, D, H, W, kz):
+    """Few columns: the shallowest blocks of a column that one wave of 148 x 28 warps
+    holds; otherwise the fewest blocks of up to 128 slices -- host only."""
+    assert forward_tile(clean_bp_rules, D, H, W, 100) == (kz, (2, 2))
+
+
 def test_autotuner_tunes_backprojector(clean_bp_rules, tmp_path):
     """Fastest forward (KZ, patch) and backward KZ per (depth, views) bucket,
     cached as JSON and registered as a library rule."""

@@ -26,9 +26,10 @@ rule (``dgc_fp_add_arm_rule``).
 
 The backprojector is tuned the same way (``tune_backprojector``): the Z
 blocking of its forward and backward (32*KZ voxels of a column per warp) and
-the forward's patch of columns per CTA, per bucket of volume depth and view
-count (each rounded up to a power of two), registered in the library as tile
-rules (``dgc_bp_add_tile_rule``).  No counterpart in the reference.
+the forward's patch of columns per CTA, or the forward's own choice of both, per
+bucket of volume depth and view count (each rounded up to a power of two),
+registered in the library as tile rules (``dgc_bp_add_tile_rule``).  No
+counterpart in the reference.
 """
 
 from __future__ import annotations
@@ -41,9 +42,12 @@ from pathlib import Path
 FORWARD_TILES = (8, 4, 2)
 BACKWARD_TILES = (8, 4)
 TUNE_VIEWS = 48
-BP_KZ_FORWARD = (1, 2, 4, 8)
 BP_KZ_BACKWARD = (2, 4, 8)
-BP_CTAS = ((8, 1), (4, 2))
+# (KZ, column patch) of the backprojector's forward; BUILT_IN leaves both to the kernel,
+# which blocks a volume as suits its sizes
+BUILT_IN = (0, (0, 0))
+BP_FORWARD = (BUILT_IN, (1, (4, 2)), (2, (4, 2)), (4, (4, 2)), (1, (2, 2)), (2, (2, 2)), (4, (2, 2)),
+              (2, (8, 1)))
 BP_TUNE_VIEWS = 360
 # (arm, slab cells, march unroll, view block): L1 quads unrolled once or twice,
 # CTAs in view blocks of 0 (every u tile of a view first), 8, 16, 32 or 64; TMA
@@ -254,16 +258,19 @@ class Autotuner:
         if key not in self.table:
             args = (projections, geometry, pixel_size, volume_shape, voxel_size,
                     tuple(float(x) for x in volume_offset))
-            fwd = {f"{kz}/{cx}x{cy}": float(self.measure_bp(*args, "forward", kz, (cx, cy)))
-                   for kz in BP_KZ_FORWARD for cx, cy in BP_CTAS}
+            label = {c: "built-in" if c == BUILT_IN else f"{c[0]}/{c[1][0]}x{c[1][1]}"
+                     for c in BP_FORWARD}
+            fwd = {c: float(self.measure_bp(*args, "forward", *c)) for c in BP_FORWARD}
             bwd = {str(kz): float(self.measure_bp(*args, "backward", kz, (8, 1)))
                    for kz in BP_KZ_BACKWARD}
             best = min(fwd, key=fwd.get)
-            kz_f, patch = best.split("/")
-            cx, cy = (int(x) for x in patch.split("x"))
-            self.table[key] = {"d_max": d_max, "a_max": a_max, "kz_forward": int(kz_f),
-                               "kz_backward": int(min(bwd, key=bwd.get)), "cta": [cx, cy],
-                               "forward_ms": fwd, "backward_ms": bwd}
+            # the kernel's own choice goes by the tile that the library reports for it
+            kz_f, cta = best if best != BUILT_IN else (1 if d_max <= 32 else 2, (8, 1))
+            self.table[key] = {"d_max": d_max, "a_max": a_max, "forward": label[best],
+                               "kz_forward": kz_f, "cta": list(cta),
+                               "kz_backward": int(min(bwd, key=bwd.get)),
+                               "forward_ms": {label[c]: ms for c, ms in fwd.items()},
+                               "backward_ms": bwd}
             self.measured.append(key)
             self._save()
         self.apply_backprojector_rules()
@@ -313,9 +320,9 @@ class Autotuner:
         rules = sorted((e for k, e in self.table.items() if k.startswith("bp:")),
                        key=lambda e: (e["d_max"], e["a_max"]))
         for e in rules[:16]:
-            _native.check(lib.dgc_bp_add_tile_rule(int(e["d_max"]), int(e["a_max"]),
-                                                   int(e["kz_forward"]), int(e["kz_backward"]),
-                                                   int(e["cta"][0]), int(e["cta"][1])))
+            kz, cta = (e["kz_forward"], e["cta"]) if e.get("forward") != "built-in" else BUILT_IN
+            _native.check(lib.dgc_bp_add_tile_rule(int(e["d_max"]), int(e["a_max"]), int(kz),
+                                                   int(e["kz_backward"]), int(cta[0]), int(cta[1])))
         return len(rules[:16])
 
     def choose(self, problems):
@@ -330,7 +337,8 @@ class Autotuner:
 
 def backprojector_tiles(D, A):
     """(kz_forward, kz_backward, (cta_x, cta_y)) a backprojection of depth D
-    over A views uses (dgc_bp_tiles)."""
+    over A views uses (dgc_bp_tiles, which reports the forward's own choice as 8 x 1
+    columns with KZ 1 up to depth 32 and 2 above)."""
     import ctypes
 
     from . import _native

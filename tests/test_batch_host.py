@@ -219,6 +219,35 @@ def test_autotuner_tunes_backprojector(clean_bp_rules, tmp_path):
     assert backprojector_tiles(256, 360) == (4, 8, (4, 2))
 
 
+def test_autotuner_offers_what_the_forward_runs(clean_bp_rules, tmp_path):
+    """Every candidate is a tile that its measurement really runs, the kernel's own choice
+    and its 2 x 2 columns among them; the own choice, chosen, leaves the forward
+    without a rule -- host only."""
+    from dgc_b200.autotune import BP_FORWARD, BUILT_IN, Autotuner, backprojector_tiles
+
+    lib = clean_bp_rules
+    own = forward_tile(lib, 256, 256, 256, 360)
+    ran = []
+
+    def fake(proj, geom, px, shape, vs, off, direction, kz, cta):
+        if direction == "forward":
+            lib.dgc_bp_clear_tile_rules()
+            assert lib.dgc_bp_add_tile_rule(1 << 30, 1 << 30, kz, kz, *cta) == 0
+            ran.append(forward_tile(lib, *shape, 360))
+            assert ran[-1] == (own if (kz, cta) == BUILT_IN else (kz, cta))
+            return 1.0 if ran[-1] == own and kz == 0 else 2.0
+        return float(kz)
+
+    geom = [SimpleNamespace(numel=lambda: 360)]
+    tuner = Autotuner(cache_path=tmp_path / "tiles.json", measure_bp=fake)
+    e = tuner.tune_backprojector(None, geom, 1.0, (256, 256, 256), 1.0)
+    assert len(ran) == len(BP_FORWARD) and {(2, (2, 2)), (4, (2, 2)), (2, (8, 1))} < set(ran)
+    assert e["forward"] == "built-in" and len(e["forward_ms"]) == len(BP_FORWARD)
+    assert forward_tile(lib, 256, 256, 256, 360) == own
+    assert backprojector_tiles(256, 360) == (e["kz_forward"], e["kz_backward"], tuple(e["cta"]))
+    assert e["kz_backward"] == 2
+
+
 def test_autotuner_tunes_forward_arm(tmp_path):
     """Fastest forward arm (L1 quads or TMA bricks, slab 2 or 4) per
     volume-size bucket, cached as JSON and registered as a library arm rule;

@@ -6,7 +6,8 @@ detector and volume shape: narrow tiles keep more rows of one column together
 (better z-locality of the volume reads), wide tiles share more of a view's
 volume slab across columns.  The tuner times every candidate on a
 representative problem of each shape bucket, with CUDA events, and keeps the
-choice in a JSON cache so that a bucket is measured once per machine.
+choice in a JSON cache so that a bucket is measured once per machine and build of
+the library.
 
 Buckets: volume size class (log2 of the voxel count, rounded), detector U and
 V rounded up to a multiple of 128, and whether the voxel size is a power of
@@ -34,6 +35,7 @@ counterpart in the reference.
 
 from __future__ import annotations
 
+import hashlib
 import json
 import math
 import os
@@ -76,6 +78,18 @@ def default_cache_path() -> Path:
     if env:
         return Path(env)
     return Path.home() / ".cache" / "dgc_b200" / "tiles.json"
+
+
+def measured_on() -> str:
+    """What a measurement depends on beside the problem: the library's build (a digest of
+    the file) and the device.  Choices cached for another are measured again."""
+    import torch
+
+    from . import _native
+
+    path = Path(os.environ.get("DGC_LIBRARY", _native.LIB_PATH))
+    build = hashlib.sha256(path.read_bytes()).hexdigest()[:16] if path.exists() else "none"
+    return f"{build} {torch.cuda.get_device_name() if torch.cuda.is_available() else 'no GPU'}"
 
 
 def time_problem(problem, direction: str, tile: int, grad_volume=True, warmup=1, repeats=3):
@@ -217,17 +231,21 @@ class Autotuner:
         self.measure_bp = measure_bp or time_backprojector
         self.measure_arm = measure_arm or time_forward_arm
         self.table = {}
+        self.measured_on = measured_on()
         if self.cache_path.exists():
             try:
-                self.table = json.loads(self.cache_path.read_text())
-            except (OSError, ValueError):
-                self.table = {}
+                cached = json.loads(self.cache_path.read_text())
+                if cached.get("measured_on") == self.measured_on:
+                    self.table = dict(cached["table"])
+            except (OSError, ValueError, TypeError, KeyError, AttributeError):
+                pass
         self.measured = []  # buckets measured by this tuner
 
     def _save(self):
         self.cache_path.parent.mkdir(parents=True, exist_ok=True)
         tmp = self.cache_path.with_suffix(".tmp")
-        tmp.write_text(json.dumps(self.table, indent=1, sort_keys=True))
+        tmp.write_text(json.dumps({"measured_on": self.measured_on, "table": self.table}, indent=1,
+                                  sort_keys=True))
         tmp.replace(self.cache_path)
 
     def tune_bucket(self, problem):

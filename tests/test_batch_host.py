@@ -248,6 +248,47 @@ def test_autotuner_offers_what_the_forward_runs(clean_bp_rules, tmp_path):
     assert e["kz_backward"] == 2
 
 
+def test_autotuner_measures_again_for_another_build(clean_bp_rules, tmp_path, monkeypatch):
+    """A choice holds for the library build and the device that it was measured on; a file
+    without either, or that is no table, counts as none -- host only."""
+    import json
+
+    from dgc_b200 import autotune
+    from dgc_b200.autotune import Autotuner
+
+    calls = []
+
+    def fake(*args):
+        calls.append(args[-2:])
+        return 1.0
+
+    geom = [SimpleNamespace(numel=lambda: 360)]
+    path = tmp_path / "tiles.json"
+
+    def tune():
+        calls.clear()
+        tuner = Autotuner(cache_path=path, measure_bp=fake)
+        tuner.tune_backprojector(None, geom, 1.0, (256, 256, 256), 1.0)
+        return len(calls)
+
+    assert tune() > 0 and tune() == 0
+    monkeypatch.setattr(autotune, "measured_on", lambda: "another build")
+    assert tune() > 0 and tune() == 0
+    entry = json.loads(path.read_text())["table"]
+    for text in (json.dumps(entry), "[]", "{", json.dumps({"measured_on": "another build"}),
+                 json.dumps({"measured_on": "another build", "table": 3})):
+        path.write_text(text)
+        assert tune() > 0 and tune() == 0
+    monkeypatch.undo()
+    assert tune() > 0
+    library = tmp_path / "lib.so"
+    library.write_bytes(b"one")
+    monkeypatch.setenv("DGC_LIBRARY", str(library))
+    one = autotune.measured_on()
+    library.write_bytes(b"two")
+    assert autotune.measured_on() != one
+
+
 def test_autotuner_tunes_forward_arm(tmp_path):
     """Fastest forward arm (L1 quads or TMA bricks, slab 2 or 4) per
     volume-size bucket, cached as JSON and registered as a library arm rule;

@@ -627,7 +627,7 @@ size_t dgc_fdk_filter_workspace_bytes(int A, int U, int V) {
 
 size_t dgc_fdk_filter_workspace_bytes_at_a_time(int A, int U, int V, int adjoint, int views) {
     if (A <= 0 || U <= 0 || V <= 0 || views < 0) return 0;
-    const int most = fdk_tc_views(A, U, V);
+    const int most = fdk_tc_views(A, U, V, adjoint != 0);
     return filter_base_bytes(A, U, V, adjoint != 0) +
            (views && most ? fdk_tc_scratch(U, V, adjoint != 0, std::min(views, most)) : 0);
 }

@@ -52,7 +52,7 @@ int fdk_launch_filter_adjoint(const FdkArgs& p, cudaStream_t s);
 // the sizes are not its), scratch for these or for some, and the filter or the
 // adjoint with its sums, with as many views at a time as ws holds; *used false:
 // nothing was done.
-int fdk_tc_views(int A, int U, int V);
+int fdk_tc_views(int A, int U, int V, bool adjoint);
 size_t fdk_tc_bytes(int A, int U, int V, bool adjoint);
 size_t fdk_tc_scratch(int U, int V, bool adjoint, int views);
 int fdk_tc_filter(const FdkArgs& p, bool adjoint, Workspace ws, cudaStream_t s, bool* used);

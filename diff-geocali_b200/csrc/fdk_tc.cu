@@ -661,14 +661,17 @@ FdkArgs views_of(const FdkArgs& p, int a0, int n) {
 
 }  // namespace
 
-int fdk_tc_views(int A, int U, int V) {
-    // U from 96: the FP32 product's time there is that of its chain over U, the tensor
-    // cores' that of their launches (FP32 / tensor cores, us: U = 64, 1 to 90 views
-    // 22.5 / 23.3-24.6; 96, 64 views x 80 28.6 / 27.6; 128, 1 view x 128 34.8 / 27.5;
-    // 200, 120 views x 160 121 / 53; adjoint at 96 52.1 / 50.2, at 64 37.9 / 42.0).  To
-    // 2048: the strip and two stages fill the shared memory.  The rule has no number
-    // of views in it, so that a view's result does not depend on its neighbours.
-    if (A < 1 || U < 96 || U > 2048 || V < 16 || tc_split_bytes(U, V) > kTcChunkBytes) return 0;
+int fdk_tc_views(int A, int U, int V, bool adjoint) {
+    // Below, the FP32 product's time is that of its chain over U, the tensor cores' that of
+    // their launches and of rows that the tile of 128 pads.  Tensor cores / FP32, over
+    // 1 to 512 views of 16 to 600 columns: the filter 0.68-1.14 at U = 96, 0.66-1.09 at
+    // 112, 0.63-0.98 at 128, 0.40-0.66 at 256; the adjoint, whose epilogue is a launch of
+    // its own, 0.77-1.25 at 96, 0.82-1.20 at 128, 0.56-1.16 at 129 to 160 (0.56-1.08
+    // from 96 columns), 0.56-1.07 at 192, 0.54-0.94 at 256.  To 2048: the strip and two stages
+    // fill the shared memory.  The rule has no number of views in it, so that a view's
+    // result does not depend on its neighbours.
+    const bool rows = adjoint ? U >= 192 || (U >= 129 && V >= 96) : U >= 128;
+    if (A < 1 || !rows || U > 2048 || V < 16 || tc_split_bytes(U, V) > kTcChunkBytes) return 0;
     const int most = (int)std::min<long long>(16384, (long long)(kTcChunkBytes / tc_split_bytes(U, V)));
     return ceil_div(A, ceil_div(A, most));  // equal chunks
 }
@@ -681,7 +684,7 @@ size_t fdk_tc_scratch(int U, int V, bool adjoint, int views) {
 }
 
 size_t fdk_tc_bytes(int A, int U, int V, bool adjoint) {
-    const int views = fdk_tc_views(A, U, V);
+    const int views = fdk_tc_views(A, U, V, adjoint);
     return views ? fdk_tc_scratch(U, V, adjoint, views) : 0;
 }
 
@@ -689,7 +692,7 @@ size_t fdk_tc_bytes(int A, int U, int V, bool adjoint) {
 // result is the same whatever their number).
 static int views_that_fit(const FdkArgs& p, bool adjoint, const Workspace& ws) {
     const size_t room = ws.base ? ws.size - ws.used : 0;
-    int low = 0, high = fdk_tc_views(p.A, p.U, p.V);
+    int low = 0, high = fdk_tc_views(p.A, p.U, p.V, adjoint);
     if (!high || fdk_tc_scratch(p.U, p.V, adjoint, high) <= room) return high;
     while (low + 1 < high) {
         const int mid = (low + high) / 2;

@@ -183,3 +183,20 @@ def test_header_is_c99_and_links_from_c(tmp_path):
     run = subprocess.run([str(exe)], capture_output=True, text=True)
     assert run.returncode == 0, (run.returncode, run.stdout, run.stderr)
     assert "alpha" in run.stdout
+
+
+@pytest.mark.parametrize("U,V,forward,adjoint", [
+    (96, 600, False, False), (127, 256, False, False), (128, 16, True, False), (128, 600, True, False),
+    (129, 95, True, False), (129, 96, True, True), (191, 95, True, False), (192, 16, True, True),
+    (2048, 24, True, True), (2049, 300, False, False), (768, 15, False, False)])
+def test_filter_sizes_of_the_tensor_cores(U, V, forward, adjoint):
+    """Where the filter and its adjoint want scratch beyond the FP32 product's: the sizes at
+    which the tensor cores are the faster ones."""
+    from dgc_b200 import _native
+
+    lib = _native.lib()
+    for adj, wanted in ((0, forward), (1, adjoint)):
+        least, one, most = (lib.dgc_fdk_filter_workspace_bytes_at_a_time(3, U, V, adj, v) for v in (0, 1, 3))
+        assert (least < one < most) == wanted and (wanted or least == one == most)
+        query = lib.dgc_fdk_filter_backward_workspace_bytes if adj else lib.dgc_fdk_filter_workspace_bytes
+        assert query(3, U, V) == most

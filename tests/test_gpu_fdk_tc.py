@@ -171,7 +171,7 @@ def test_without_room_for_the_scratch(monkeypatch):
         assert float((got - ref).abs().max()) <= 2.0**-19 * 2.0**8 * float(ref.abs().max())
 
 
-@pytest.mark.parametrize("U,px", [(96, 1.0), (187, 1.0), (768, 3.0), (130, 0.05)])
+@pytest.mark.parametrize("U,px", [(96, 1.0), (128, 1.0), (187, 1.0), (768, 3.0), (200, 0.05)])
 def test_columns_of_small_values_keep_their_precision(U, px):
     """Every detector column to its own magnitudes, down to the subnormals, beside one of
     ordinary values.  Below FP32's smallest normal number a rounding is 2^-149 at most
@@ -219,7 +219,7 @@ def in_room(p, g, y, sod, sid, dist, views):
     return [out, gp, *gs]
 
 
-@pytest.mark.parametrize("U,V", [(97, 17), (300, 203)])
+@pytest.mark.parametrize("U,V", [(192, 17), (129, 97), (300, 203)])
 def test_fewer_views_at_a_time_give_the_same_bits(U, V):
     from dgc_b200 import _native, _ops
 

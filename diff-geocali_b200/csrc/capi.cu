@@ -643,6 +643,12 @@ static int run_filter(const FdkArgs& f, const Workspace& scratch, cudaStream_t s
     return fdk_launch_filter(f, s);
 }
 
+int dgc_fdk_limit_waits(int polls) {
+    clear_error();
+    fdk_tc_limit_waits(polls);
+    return DGC_OK;
+}
+
 static int check_fdk(int A, int U, int V, float pixel_size, float alpha) {
     DGC_REQUIRE(A > 0 && U > 0 && V > 0, "projections must have a nonempty [A, U, V] shape");
     DGC_REQUIRE(std::isfinite(pixel_size) && pixel_size > 0.0f, "pixel_size must be finite and positive");

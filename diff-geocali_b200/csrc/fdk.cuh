@@ -56,6 +56,7 @@ int fdk_tc_views(int A, int U, int V, bool adjoint);
 size_t fdk_tc_bytes(int A, int U, int V, bool adjoint);
 size_t fdk_tc_scratch(int U, int V, bool adjoint, int views);
 int fdk_tc_filter(const FdkArgs& p, bool adjoint, Workspace ws, cudaStream_t s, bool* used);
+void fdk_tc_limit_waits(int polls);  // of the calling thread's launches; < 0: the built-in limit
 // Per-view gradients from the partials: sod, sid, and, where the frame was
 // given, its distance and centres (any output may be null).
 struct FdkGrads {

@@ -203,6 +203,7 @@ struct TcArgs {
     float pixel_size;
     FdkRange* ranges;  // [views][ceil(U/8)]
     bool wide, staged;  // stores: 32 bytes a lane; rows by way of shared memory
+    int polls;          // limit of the pipeline's waits (not of those for copies in flight)
 };
 
 __global__ void __launch_bounds__(kTcThreads, 1) fdk_filter_tc_kernel(
@@ -261,7 +262,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) fdk_filter_tc_kernel(
             for (int tile = first; tile < p.columns && !*err; tile += step) {
                 const int v0 = (tile % p.col_tiles) * p.n, a = tile / p.col_tiles;
                 for (int kt = 0; kt < nk && !*err; ++kt) {
-                    if (!mbar_wait(tma_smem_u32(&empty[s]), phase)) {
+                    if (!mbar_wait(tma_smem_u32(&empty[s]), phase, p.polls)) {
                         *err = 1;
                         break;
                     }
@@ -285,15 +286,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) fdk_filter_tc_kernel(
             const uint64_t b0 = smem_desc(sbase, kTcBox, 1024u, 2u);
             const uint32_t a_part = strip_bytes / 16, b_stage = stage_bytes / 16;
             constexpr uint32_t b_part = kTcPart / 16;
-            bool ok = mbar_wait(tma_smem_u32(&strip_full), 0);
+            bool ok = mbar_wait(tma_smem_u32(&strip_full), 0, p.polls);
             int g = 0, s = 0;        // stages so far, this one's slot
             uint32_t phase = 0;      // of the slots' full barriers
             uint32_t done_tiles = 0;
             for (int tile = first; ok && tile < p.columns; tile += step, ++done_tiles) {
                 for (int kt = 0; kt < nk; ++kt) {
-                    ok = mbar_wait(tma_smem_u32(&full[s]), phase);
+                    ok = mbar_wait(tma_smem_u32(&full[s]), phase, p.polls);
                     // the last stage's leading product has been taken
-                    if (ok && g > 0) ok = mbar_wait(tma_smem_u32(&hi_empty), (g - 1) & 1);
+                    if (ok && g > 0) ok = mbar_wait(tma_smem_u32(&hi_empty), (g - 1) & 1, p.polls);
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t at = a0 + kt * kTcStageK, bt = b0 + s * b_stage;
@@ -303,7 +304,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) fdk_filter_tc_kernel(
                     umma_commit(tma_smem_u32(&hi_full));
                     // the other five, smallest first
                     if (kt == 0 && done_tiles > 0) {
-                        ok = mbar_wait(tma_smem_u32(&low_empty), (done_tiles - 1) & 1);
+                        ok = mbar_wait(tma_smem_u32(&low_empty), (done_tiles - 1) & 1, p.polls);
                         if (!ok) break;
                         tc_fence_after();
                     }
@@ -360,11 +361,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) fdk_filter_tc_kernel(
 #pragma unroll
             for (int i = 0; i < 128; ++i) acc[i] = 0.0f;
             for (int c = 0; c < nk; ++c, ++chunk) {
-                ok = __all_sync(0xffffffffu, mbar_wait(tma_smem_u32(&hi_full), chunk & 1));
+                ok = __all_sync(0xffffffffu, mbar_wait(tma_smem_u32(&hi_full), chunk & 1, p.polls));
                 if (!ok) break;
                 take(tmem_hi + at, tma_smem_u32(&hi_empty), acc);
             }
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(tma_smem_u32(&low_full), done_tiles & 1));
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(tma_smem_u32(&low_full), done_tiles & 1, p.polls));
             if (!ok) break;
             take(tmem_low + at, tma_smem_u32(&low_empty), acc);
             // the next tile's products run while this one is stored
@@ -435,6 +436,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) fdk_filter_tc_kernel(
     }
 }
 
+// Polls after which this thread's launches give a wait up.
+thread_local int tc_polls = (int)kTcWaitLimit;
+
 // 3-D map of the split rows: V columns, U rows, 3 parts a view; boxes of 64 columns x
 // kTcStageK rows x the parts, 128-byte swizzle, zero fill outside.
 bool split_map(CUtensorMap* map, const __nv_bfloat16* split, int views, int U, int V) {
@@ -481,20 +485,19 @@ int launch_tc(const FdkArgs* f, const __nv_bfloat16* strip, const __nv_bfloat16*
     p.sod = f ? f->sod : nullptr;
     p.pixel_size = f ? f->pixel_size : 1.0f;
     p.ranges = ranges;
-    static std::atomic<unsigned long long> configured{0};
+    p.polls = tc_polls;
+    static std::atomic<unsigned long long> configured{0}, unfit{0};
     const int rc = once_per_device(configured, []() -> int {
         DGC_CUDA(cudaFuncSetAttribute(fdk_filter_tc_kernel,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem + 1024));
         // the register split must fit what a launch grants, or it would wait for good
         cudaFuncAttributes attr;
         DGC_CUDA(cudaFuncGetAttributes(&attr, fdk_filter_tc_kernel));
-        if (attr.numRegs * kTcThreads < 128 * kTcRegsFew + 256 * kTcRegsMany) {
-            set_error("fdk_filter_tc_kernel: registers at launch below its split");
-            return DGC_ERR_CUDA;
-        }
+        if (attr.numRegs * kTcThreads < 128 * kTcRegsFew + 256 * kTcRegsMany) unfit.store(1);
         return DGC_OK;
     });
     if (rc != DGC_OK) return rc;
+    if (unfit.load()) return DGC_OK;  // the FP32 product takes the call
     DGC_TRACE("fdk_filter_tc_kernel", s);
     // a CTA keeps its rows (and their strip), so the grid is whole sets of row tiles
     p.columns = p.col_tiles * views;
@@ -660,6 +663,8 @@ FdkArgs views_of(const FdkArgs& p, int a0, int n) {
 }
 
 }  // namespace
+
+void fdk_tc_limit_waits(int polls) { tc_polls = polls < 0 ? (int)kTcWaitLimit : polls; }
 
 int fdk_tc_views(int A, int U, int V, bool adjoint) {
     // Below, the FP32 product's time is that of its chain over U, the tensor cores' that of

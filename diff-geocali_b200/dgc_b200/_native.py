@@ -76,6 +76,7 @@ SIGNATURES = {
     "dgc_fdk_filter_workspace_bytes": (_S, [_I] * 3),
     "dgc_fdk_filter_workspace_bytes_at_a_time": (_S, [_I] * 5),
     "dgc_fdk_filter": (_I, [_P, _I, _I, _I, _F, _P, _P, _F, _P, _P, _S, _P]),
+    "dgc_fdk_limit_waits": (_I, [_I]),
     "dgc_fdk_filter_noalloc": (_I, [_P, _I, _I, _I, _F, _P, _P, _F, _P, _P]),
     "dgc_reconstruct_fdk_workspace_bytes": (_S, [_I] * 6),
     "dgc_reconstruct_fdk": (_I, [_P, _I, _I, _I, *_GEOM, _F, _I, _I, _I, _F, _F, _F, _F, _F, _P, _P,

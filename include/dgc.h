@@ -219,6 +219,12 @@ int dgc_fdk_filter_ex(const float* projections, int A, int U, int V, float pixel
                       const float* frame_u, const float* frame_v, float alpha, float* filtered,
                       void* workspace, size_t workspace_bytes, void* stream);
 
+/* Polls after which the calling thread's later filter launches give up a wait inside
+ * the tensor-core kernel (negative: the built-in limit of 2^22, about a second); a
+ * view on which one gave up is computed by the FP32 product.  For tests of that
+ * path; 0 gives every wait up at once.  No counterpart in the reference. */
+int dgc_fdk_limit_waits(int polls);
+
 /* Maximum detector width U accepted by dgc_fdk_filter_noalloc. */
 #define DGC_FDK_NOALLOC_MAX_U 8192
 

@@ -285,3 +285,32 @@ def test_noalloc_is_the_fp32_product(U, px):
     a, b = got.double(), want.double()
     assert float(b.abs().max()) > 0
     assert float(((a - b).abs() - 2.0**-22 * b.abs() - 2.0**-49 * b.abs().max()).max()) <= 0
+
+
+@pytest.mark.parametrize("A,U,V", [(3, 192, 130), (5, 300, 96), (2, 768, 300)])
+@pytest.mark.parametrize("polls", [0, 1, 2])
+def test_waits_that_run_out(A, U, V, polls):
+    """Waits inside the tensor-core kernel given up at once (0), or after a poll or two, of
+    which some or none then run out: the views come from the FP32 product, and a view
+    whose CTAs all got through from the tensor cores -- one of the two, bit for bit, in
+    the filter, the projection gradient and the distance gradients.  The next call is
+    as if nothing had happened."""
+    from dgc_b200 import _native, _ops
+
+    p, sid, sod = scan(A, U, V, 9)
+    g = torch.randn(p.shape, generator=torch.Generator().manual_seed(4)).cuda()
+    dist = sid * 0.99
+    y = _ops.fdk_filter_framed(p, 1.0, sod, sid, 0.8, (dist, None, None))
+    fast = in_room(p, g, y, sod, sid, dist, A)
+    slow = in_room(p, g, y, sod, sid, dist, 0)
+    lib = _native.lib()
+    lib.dgc_fdk_limit_waits(polls)
+    try:
+        got = in_room(p, g, y, sod, sid, dist, A)
+        torch.cuda.synchronize()
+    finally:
+        lib.dgc_fdk_limit_waits(-1)
+    for k, (a, f, s) in enumerate(zip(got, fast, slow)):
+        for v in range(A):
+            assert torch.equal(a[v], s[v]) or (polls and torch.equal(a[v], f[v])), (k, v)
+    assert all(torch.equal(a, b) for a, b in zip(in_room(p, g, y, sod, sid, dist, A), fast))

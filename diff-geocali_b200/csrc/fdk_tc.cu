@@ -72,6 +72,13 @@ size_t tc_split_bytes(int U, int V) {  // of one view
     return 3 * sizeof(__nv_bfloat16) * (size_t)U * (size_t)tc_row_stride(V);
 }
 
+// max(a, b), NaN if either is.
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 struct Split3 {
     __nv_bfloat16 part[3];
 };
@@ -90,8 +97,11 @@ __device__ __forceinline__ Split3 split3(float x) {
 // cosine-weighted projection, or (ADJ) the upstream gradient; ranges[view][k / 8] =
 // the range of its magnitudes.  grid: x = groups of 8 rows, y = view; the blocks
 // of the row after the last view fill strip[part][q][8r + c] = part of f[8q + r + c].
+// Six blocks per SM (42 registers; left to itself the compiler takes 53): 360 x 384^2
+// 78.7 -> 70.4 us, 100 x 768^2 82.8 -> 74.1, of which the ranges' two instructions an
+// element are 4.
 template <bool ADJ>
-__global__ void __launch_bounds__(256) fdk_split_kernel(FdkArgs p, int stride,
+__global__ void __launch_bounds__(256, 6) fdk_split_kernel(FdkArgs p, int stride,
                                                         __nv_bfloat16* __restrict__ split,
                                                         FdkRange* __restrict__ ranges, int cores,
                                                         __nv_bfloat16* __restrict__ strip) {
@@ -108,22 +118,22 @@ __global__ void __launch_bounds__(256) fdk_split_kernel(FdkArgs p, int stride,
     const int a = blockIdx.y;
     const float sid = p.sid[a];
     const float dn = p.frame_dist ? p.frame_dist[a] : sid;
-    const float dn2 = dn * dn;
+    const float dn2 = __fmul_rn(dn, dn);
     const float cu = p.frame_u ? p.frame_u[a] : 0.5f * (p.U - 1);
     const float cv = p.frame_v ? p.frame_v[a] : 0.5f * (p.V - 1);
     const float* __restrict__ src =
         (ADJ ? p.grad_filtered : p.projections) + (long long)a * p.U * p.V;
     const int groups = stride / 4;
     const bool wide = (p.V & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
-    // as bits, which order as the magnitudes do: a NaN is above the infinities, and a
-    // zero, less one as unsigned, above all
-    int high = 0;
-    unsigned low = 0x7fffffffu;
+    // the largest magnitude (a NaN stays one) and the smallest but zero, as twice its
+    // bits less one: a zero is then above all
+    float high = 0.0f;
+    unsigned low = 0xffffffffu;
     __shared__ int s_high;
     __shared__ unsigned s_low;
     if (threadIdx.x == 0) {
         s_high = 0;
-        s_low = 0x7fffffffu;
+        s_low = 0xffffffffu;
     }
     __syncthreads();
     for (int i = threadIdx.x; i < 8 * groups; i += 256) {
@@ -148,18 +158,15 @@ __global__ void __launch_bounds__(256) fdk_split_kernel(FdkArgs p, int stride,
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const float vv = ((float)(v0 + j) - cv) * p.pixel_size;
-                const float dist = sqrtf(dn2 + uu * uu + vv * vv);
+                const float dist = sqrtf(fmaf(vv, vv, fmaf(uu, uu, dn2)));
                 x[j] = x[j] * (dn / dist) * wk;
             }
         }
         __align__(8) __nv_bfloat16 h[3][4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            if (v0 + j < p.V) {
-                const int bits = __float_as_int(x[j]) & 0x7fffffff;
-                high = max(high, bits);
-                low = min(low, (unsigned)bits - 1u);
-            }
+            high = max_nan(high, fabsf(x[j]));
+            low = min(low, 2u * __float_as_uint(x[j]) - 1u);
             const Split3 s = split3(x[j]);
             h[0][j] = s.part[0];
             h[1][j] = s.part[1];
@@ -171,16 +178,16 @@ __global__ void __launch_bounds__(256) fdk_split_kernel(FdkArgs p, int stride,
                 split + (((size_t)a * 3 + s) * p.U + (p.U - 1 - k)) * stride + v0) =
                 *reinterpret_cast<const uint2*>(h[s]);
     }
-    high = __reduce_max_sync(0xffffffffu, high);
+    const int top = __reduce_max_sync(0xffffffffu, __float_as_int(high));
     low = __reduce_min_sync(0xffffffffu, low);
     if ((threadIdx.x & 31) == 0) {
-        atomicMax(&s_high, high);
+        atomicMax(&s_high, top);
         atomicMin(&s_low, low);
     }
     __syncthreads();
     if (threadIdx.x == 0)
         ranges[(long long)a * gridDim.x + blockIdx.x] =
-            FdkRange{s_low == 0x7fffffffu ? INT_MAX : (int)s_low + 1, s_high};
+            FdkRange{s_low == 0xffffffffu ? INT_MAX : (int)((s_low + 1u) >> 1), s_high};
 }
 
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes,
@@ -203,9 +210,12 @@ struct TcArgs {
     float pixel_size;
     FdkRange* ranges;  // [views][ceil(U/8)]
     bool wide, staged;  // stores: 32 bytes a lane; rows by way of shared memory
-    int polls;          // limit of the pipeline's waits (not of those for copies in flight)
+    int polls;          // LIMIT: of the pipeline's waits (not of those for copies in flight)
 };
 
+// LIMIT: the pipeline's waits give up after p.polls polls (as an argument the limit costs
+// the kernel 7-10 % of its time, so that calls without one have a constant).
+template <bool LIMIT>
 __global__ void __launch_bounds__(kTcThreads, 1) fdk_filter_tc_kernel(
     const __grid_constant__ CUtensorMap map, TcArgs p) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -245,6 +255,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) fdk_filter_tc_kernel(
     tc_fence_after();
     const uint32_t tmem_hi = tmem_slot, tmem_low = tmem_hi + 256;
     volatile int* err = &s_err;
+    const long long polls = LIMIT ? p.polls : kTcWaitLimit;
 
     int issued = 0;  // stages, over all tiles (warp 0)
     bool strip_issued = false;
@@ -262,7 +273,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) fdk_filter_tc_kernel(
             for (int tile = first; tile < p.columns && !*err; tile += step) {
                 const int v0 = (tile % p.col_tiles) * p.n, a = tile / p.col_tiles;
                 for (int kt = 0; kt < nk && !*err; ++kt) {
-                    if (!mbar_wait(tma_smem_u32(&empty[s]), phase, p.polls)) {
+                    if (!mbar_wait(tma_smem_u32(&empty[s]), phase, polls)) {
                         *err = 1;
                         break;
                     }
@@ -286,15 +297,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) fdk_filter_tc_kernel(
             const uint64_t b0 = smem_desc(sbase, kTcBox, 1024u, 2u);
             const uint32_t a_part = strip_bytes / 16, b_stage = stage_bytes / 16;
             constexpr uint32_t b_part = kTcPart / 16;
-            bool ok = mbar_wait(tma_smem_u32(&strip_full), 0, p.polls);
+            bool ok = mbar_wait(tma_smem_u32(&strip_full), 0, polls);
             int g = 0, s = 0;        // stages so far, this one's slot
             uint32_t phase = 0;      // of the slots' full barriers
             uint32_t done_tiles = 0;
             for (int tile = first; ok && tile < p.columns; tile += step, ++done_tiles) {
                 for (int kt = 0; kt < nk; ++kt) {
-                    ok = mbar_wait(tma_smem_u32(&full[s]), phase, p.polls);
+                    ok = mbar_wait(tma_smem_u32(&full[s]), phase, polls);
                     // the last stage's leading product has been taken
-                    if (ok && g > 0) ok = mbar_wait(tma_smem_u32(&hi_empty), (g - 1) & 1, p.polls);
+                    if (ok && g > 0) ok = mbar_wait(tma_smem_u32(&hi_empty), (g - 1) & 1, polls);
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t at = a0 + kt * kTcStageK, bt = b0 + s * b_stage;
@@ -304,7 +315,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) fdk_filter_tc_kernel(
                     umma_commit(tma_smem_u32(&hi_full));
                     // the other five, smallest first
                     if (kt == 0 && done_tiles > 0) {
-                        ok = mbar_wait(tma_smem_u32(&low_empty), (done_tiles - 1) & 1, p.polls);
+                        ok = mbar_wait(tma_smem_u32(&low_empty), (done_tiles - 1) & 1, polls);
                         if (!ok) break;
                         tc_fence_after();
                     }
@@ -361,11 +372,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) fdk_filter_tc_kernel(
 #pragma unroll
             for (int i = 0; i < 128; ++i) acc[i] = 0.0f;
             for (int c = 0; c < nk; ++c, ++chunk) {
-                ok = __all_sync(0xffffffffu, mbar_wait(tma_smem_u32(&hi_full), chunk & 1, p.polls));
+                ok = __all_sync(0xffffffffu, mbar_wait(tma_smem_u32(&hi_full), chunk & 1, polls));
                 if (!ok) break;
                 take(tmem_hi + at, tma_smem_u32(&hi_empty), acc);
             }
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(tma_smem_u32(&low_full), done_tiles & 1, p.polls));
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(tma_smem_u32(&low_full), done_tiles & 1, polls));
             if (!ok) break;
             take(tmem_low + at, tma_smem_u32(&low_empty), acc);
             // the next tile's products run while this one is stored
@@ -436,8 +447,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) fdk_filter_tc_kernel(
     }
 }
 
-// Polls after which this thread's launches give a wait up.
-thread_local int tc_polls = (int)kTcWaitLimit;
+// Polls after which this thread's launches give a wait up, or -1: the constant.
+thread_local int tc_polls = -1;
 
 // 3-D map of the split rows: V columns, U rows, 3 parts a view; boxes of 64 columns x
 // kTcStageK rows x the parts, 128-byte swizzle, zero fill outside.
@@ -488,12 +499,14 @@ int launch_tc(const FdkArgs* f, const __nv_bfloat16* strip, const __nv_bfloat16*
     p.polls = tc_polls;
     static std::atomic<unsigned long long> configured{0}, unfit{0};
     const int rc = once_per_device(configured, []() -> int {
-        DGC_CUDA(cudaFuncSetAttribute(fdk_filter_tc_kernel,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem + 1024));
-        // the register split must fit what a launch grants, or it would wait for good
-        cudaFuncAttributes attr;
-        DGC_CUDA(cudaFuncGetAttributes(&attr, fdk_filter_tc_kernel));
-        if (attr.numRegs * kTcThreads < 128 * kTcRegsFew + 256 * kTcRegsMany) unfit.store(1);
+        for (const auto kernel : {fdk_filter_tc_kernel<false>, fdk_filter_tc_kernel<true>}) {
+            DGC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          kTcSmem + 1024));
+            // the register split must fit what a launch grants, or it would wait for good
+            cudaFuncAttributes attr;
+            DGC_CUDA(cudaFuncGetAttributes(&attr, kernel));
+            if (attr.numRegs * kTcThreads < 128 * kTcRegsFew + 256 * kTcRegsMany) unfit.store(1);
+        }
         return DGC_OK;
     });
     if (rc != DGC_OK) return rc;
@@ -506,7 +519,9 @@ int launch_tc(const FdkArgs* f, const __nv_bfloat16* strip, const __nv_bfloat16*
     DGC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const unsigned grid =
         (unsigned)(p.row_tiles * std::min(p.columns, std::max(1, sms / p.row_tiles)));
-    fdk_filter_tc_kernel<<<grid, kTcThreads, p.stages * stage_bytes + strip_bytes + turn_bytes + 1024, s>>>(map, p);
+    const size_t smem = p.stages * stage_bytes + strip_bytes + turn_bytes + 1024;
+    if (p.polls < 0) fdk_filter_tc_kernel<false><<<grid, kTcThreads, smem, s>>>(map, p);
+    else fdk_filter_tc_kernel<true><<<grid, kTcThreads, smem, s>>>(map, p);
     DGC_LAUNCH_CHECK("fdk_filter_tc_kernel");
     *used = true;
     return DGC_OK;
@@ -664,7 +679,7 @@ FdkArgs views_of(const FdkArgs& p, int a0, int n) {
 
 }  // namespace
 
-void fdk_tc_limit_waits(int polls) { tc_polls = polls < 0 ? (int)kTcWaitLimit : polls; }
+void fdk_tc_limit_waits(int polls) { tc_polls = std::max(polls, -1); }
 
 int fdk_tc_views(int A, int U, int V, bool adjoint) {
     // Below, the FP32 product's time is that of its chain over U, the tensor cores' that of

@@ -37,7 +37,6 @@ angle 0.3 deg, source 1 mm, detector centre 2 mm, sid/sod 0.5 %.
 from __future__ import annotations
 
 import math
-import os
 import time
 from dataclasses import dataclass, replace
 
@@ -160,13 +159,20 @@ def gemm(A, B, bias=None, relu=False, out_bf16=False, out=None, accumulate=False
     return out
 
 
+def _as_tensor_maps_take(x):
+    """Whether dgc_gemm_bf16_tn takes the rows of ``x`` as they lie: 16-byte rows and start.
+    (A matrix of one row or column may carry any stride there.)"""
+    return x.data_ptr() % 16 == 0 and x.stride(0) % 8 == 0 and x.stride(0) >= x.shape[1] \
+        and (x.stride(1) == 1 or x.shape[1] == 1)
+
+
 def gemm_tn(A, B):
     """out[m, n] = sum_k A[k, m] * B[k, n] in fp32: the product of two bf16 matrices
     over their rows (a weight gradient), as they lie."""
     K, M = A.shape
     N = B.shape[1]
     lib = _native.lib()
-    if os.environ.get("DGC_GEMM") != "cpasync" and A.stride(0) % 8 == 0 and B.stride(0) % 8 == 0:
+    if _as_tensor_maps_take(A) and _as_tensor_maps_take(B):
         out = torch.empty((M, N), device=A.device, dtype=torch.float32)
         rc = lib.dgc_gemm_bf16_tn(
             A.data_ptr(), B.data_ptr(), out.data_ptr(), M, N, K, A.stride(0), B.stride(0),
@@ -175,17 +181,16 @@ def gemm_tn(A, B):
         if rc != _native.ERR_UNSUPPORTED:
             _native.check(rc)
             return out
-    # without tensor maps or with rows off 16 bytes: transposed copies for the
+    # without the TMA pipeline, or operands off its 16 bytes: transposed copies for the
     # K-major product
     Kp = _round8(K)
     return gemm(_padded_t(A, Kp), _padded_t(B, Kp))
 
 
 def _padded_t(x, cols):
-    """x.T as a contiguous bf16 [x.shape[1], cols] with zero columns beyond x.shape[0]."""
-    if x.shape[0] == cols:
-        return x.t().contiguous()
-    out = torch.zeros((x.shape[1], cols), dtype=torch.bfloat16, device=x.device)
+    """x.T as a new contiguous bf16 [x.shape[1], cols] with zero columns beyond x.shape[0]."""
+    make = torch.empty if x.shape[0] == cols else torch.zeros
+    out = make((x.shape[1], cols), dtype=torch.bfloat16, device=x.device)
     out[:, : x.shape[0]] = x.t()
     return out
 

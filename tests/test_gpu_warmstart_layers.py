@@ -71,3 +71,20 @@ def test_view_conv_and_network():
     assert out.shape == (12, 8) and torch.isfinite(out).all()
     out.square().sum().backward()
     assert all(p.grad is not None and torch.isfinite(p.grad).all() for p in net.parameters())
+
+
+def test_one_channel_head():
+    """A head of one channel over a multiple of eight views: the weight gradient's operand
+    is a column, whose row stride no tensor map takes."""
+    from dgc_b200.warmstart import _ViewConv
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    A, Cin, k = 16, 32, 3
+    f = torch.randn(A, Cin, device="cuda", generator=g).to(torch.bfloat16).requires_grad_()
+    w = (torch.randn(1, k * Cin, device="cuda", generator=g) * 0.1).to(torch.bfloat16).float()
+    w.requires_grad_()
+    y = _ViewConv.apply(f, w, torch.zeros(1, device="cuda"), k, False)
+    gy = torch.randn(A, 1, device="cuda", generator=g)
+    (gw,) = torch.autograd.grad(y, [w], grad_outputs=gy)
+    col = torch.cat([torch.roll(f.detach().float(), shifts=k // 2 - j, dims=0) for j in range(k)], 1)
+    assert rel(gw, gy.t() @ col) < 2e-2

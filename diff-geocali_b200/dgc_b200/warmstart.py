@@ -211,6 +211,8 @@ def _relu_grad(gy, y, relu):
         g = (gy * (y > 0) if relu else gy).to(torch.bfloat16).contiguous()
         return g, g.float().sum(0)
     gy = gy.contiguous()
+    if gy.data_ptr() % 16:  # a slice of another gradient
+        gy = gy.clone()
     M, C = gy.shape
     g = torch.empty_like(gy) if relu else gy
     db = torch.empty(C, dtype=torch.float32, device=gy.device)

@@ -88,3 +88,22 @@ def test_one_channel_head():
     (gw,) = torch.autograd.grad(y, [w], grad_outputs=gy)
     col = torch.cat([torch.roll(f.detach().float(), shifts=k // 2 - j, dims=0) for j in range(k)], 1)
     assert rel(gw, gy.t() @ col) < 2e-2
+
+
+def test_gradient_that_starts_off_16_bytes():
+    """An upstream gradient that is a slice of a longer one (as torch.cat's is)."""
+    from dgc_b200.warmstart import _Conv2d, _round8
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    B, H, Cin, Cout = 2, 10, 8, 16
+    x = torch.randn(B, H, H, Cin, device="cuda", generator=g).to(torch.bfloat16).requires_grad_()
+    w = (torch.randn(Cout, _round8(9 * Cin), device="cuda", generator=g) * 0.2).requires_grad_()
+    b = torch.zeros(Cout, device="cuda", requires_grad=True)
+    y = _Conv2d.apply(x, w, b, 3, 1, 1, True)
+    long = torch.randn(3 + y.numel(), device="cuda", generator=g).to(torch.bfloat16)
+    piece = long[3:].view(y.shape)
+    assert piece.data_ptr() % 16
+    got = torch.autograd.grad(y, [x, w, b], grad_outputs=piece, retain_graph=True)
+    want = torch.autograd.grad(y, [x, w, b], grad_outputs=piece.clone())
+    assert torch.equal(got[0], want[0]) and torch.equal(got[2], want[2])
+    assert rel(got[1], want[1]) < 1e-5  # split K: sums in any order

@@ -319,7 +319,14 @@ int dgc_project_backward(const float* grad_projection, const float* volume, int 
 
 size_t dgc_project_adjoint_workspace_bytes(int D, int H, int W) {
     if (D <= 0 || H <= 0 || W <= 0) return 0;
-    return gradient_buffer_bytes(D, H, W);
+    FpArgs p;
+    memset(&p, 0, sizeof(p));
+    p.D = D;
+    p.H = H;
+    p.W = W;
+    p.voxel_size = 1.0f;
+    fp_fill_layout(p);
+    return Workspace::align(fp_edge_bytes(p));
 }
 
 int dgc_project_adjoint(const float* grad_projection, int D, int H, int W, const float* angles,
@@ -353,7 +360,7 @@ int dgc_project_adjoint(const float* grad_projection, int D, int H, int W, const
     fp_fill_layout(p);
     Workspace ws(workspace, workspace_bytes);
     p.grad_projections = grad_projection;
-    p.grad_edges = reinterpret_cast<float2*>(ws.take<char>(gradient_buffer_bytes(D, H, W)));
+    p.grad_edges = reinterpret_cast<float2*>(ws.take<char>(fp_edge_bytes(p)));
     if (!p.grad_edges) {
         set_error("workspace too small: dgc_project_adjoint needs " +
                   std::to_string(dgc_project_adjoint_workspace_bytes(D, H, W)) + " bytes");

@@ -540,16 +540,16 @@ int launch_split(const FdkArgs& p, __nv_bfloat16* split, FdkRange* ranges, __nv_
 
 // The epilogue of the FP32 adjoint from a stored z = H(g) (the tensor cores'
 // product), with its tiles and sums, for the views that these hold.  1024 threads, so
-// that a thread's chain of FP64 divisions is 16 elements long, a warp reads whole
-// rows, and four elements' loads are in flight (64 elements a
-// thread in the product's layout: 4.12 ms at 720 x 768 x 768 and 26.7 us at 90 x 128 x
-// 96; so 2.38 ms and 15.1 us).
+// that a thread's chain of FP64 divisions is 16 elements long and a warp reads whole
+// rows: 4.12 -> 2.38 ms at 720 x 768 x 768 against 64 elements a thread in the product's
+// layout; with an element's four loads ahead of its branch 100 x 768 x 768 takes 0.283 ms
+// for 0.341 (all gradients), 0.251 for 0.275 (the distances' alone).
 constexpr int kEpilogueThreads = 1024;
 
 template <bool CG>
 __global__ void __launch_bounds__(kEpilogueThreads, 2) fdk_adjoint_epilogue_kernel(
     FdkLeft p, const float* __restrict__ z) {
-    constexpr int kWarps = kEpilogueThreads / 32, kRows = kEpilogueThreads / kFdkTileColumns, kBatch = 1;
+    constexpr int kWarps = kEpilogueThreads / 32, kRows = kEpilogueThreads / kFdkTileColumns;
     __shared__ double s_part[kWarps][kFdkPartials];
     const int a = blockIdx.z;
     if (!fdk_tc_holds(p, a)) return;
@@ -565,37 +565,28 @@ __global__ void __launch_bounds__(kEpilogueThreads, 2) fdk_adjoint_epilogue_kern
     const float vv = ((float)v - cv) * p.pixel_size;
     double s_gy = 0.0, s_zpw = 0.0, s_zpu = 0.0, s_zpv = 0.0;
 #pragma unroll 4
-    for (int i = 0; i < kFdkTileRows; i += kBatch * kRows) {
-        float zz[kBatch], pp[kBatch], gg[kBatch], yy[kBatch];
-#pragma unroll
-        for (int k = 0; k < kBatch; ++k) {
-            const int u = u0 + i + k * kRows;
-            const bool in = u < p.U && v < p.V;
-            const long long idx = base + (long long)u * p.V + v;
-            zz[k] = in ? z[idx] : 0.0f;
-            pp[k] = in && sums ? p.projections[idx] : 0.0f;
-            gg[k] = in && sums ? p.grad_filtered[idx] : 0.0f;
-            yy[k] = in && sums ? p.forward_out[idx] : 0.0f;
-        }
-#pragma unroll
-        for (int k = 0; k < kBatch; ++k) {
-            const int u = u0 + i + k * kRows;
-            if (u >= p.U || v >= p.V) continue;
-            const float uu = ((float)u - cu) * p.pixel_size;
-            const float r2 = uu * uu + vv * vv;
-            const float dist = sqrtf(dn2 + r2);
-            if (p.grad_projections)
-                p.grad_projections[base + (long long)u * p.V + v] =
-                    (zz[k] * p.pixel_size) * ratio * (dn / dist);
-            if (sums) {
-                const double zp = (double)zz[k] * (double)pp[k];
-                const double d3 = (double)dist * dist * dist;
-                s_gy += (double)gg[k] * (double)yy[k];
-                s_zpw += zp * ((double)r2 / d3);
-                if (CG) {
-                    s_zpu += zp * ((double)uu / d3);
-                    s_zpv += zp * ((double)vv / d3);
-                }
+    for (int i = 0; i < kFdkTileRows; i += kRows) {
+        const int u = u0 + i;
+        const bool in = u < p.U && v < p.V;
+        const long long idx = base + (long long)u * p.V + v;
+        // the loads together, ahead of the branch
+        const float zv = in ? z[idx] : 0.0f;
+        const float pv = in && sums ? p.projections[idx] : 0.0f;
+        const float gv = in && sums ? p.grad_filtered[idx] : 0.0f;
+        const float yv = in && sums ? p.forward_out[idx] : 0.0f;
+        if (!in) continue;
+        const float uu = ((float)u - cu) * p.pixel_size;
+        const float r2 = uu * uu + vv * vv;
+        const float dist = sqrtf(dn2 + r2);
+        if (p.grad_projections) p.grad_projections[idx] = (zv * p.pixel_size) * ratio * (dn / dist);
+        if (sums) {
+            const double zp = (double)zv * (double)pv;
+            const double d3 = (double)dist * dist * dist;
+            s_gy += (double)gv * (double)yv;
+            s_zpw += zp * ((double)r2 / d3);
+            if (CG) {
+                s_zpu += zp * ((double)uu / d3);
+                s_zpv += zp * ((double)vv / d3);
             }
         }
     }

@@ -48,8 +48,26 @@ size_t quad_volume_bytes(int D, int H, int W) {
     return Workspace::align(sizeof(float4) * (size_t)(D + 2) * (size_t)(H + 1) * (size_t)(W + 1));
 }
 
-// volume-gradient buffer: the edge records (fp_edge_bytes) take about half of it
-size_t gradient_buffer_bytes(int D, int H, int W) { return quad_volume_bytes(D, H, W); }
+// The edge records of a volume gradient, in as many copies as any number of rays gives.
+size_t edge_record_bytes(int D, int H, int W) {
+    if ((D + 2.0) * (H + 1.0) * (W + 1.0) >= 2147483648.0) return quad_volume_bytes(D, H, W);  // refused
+    FpArgs p;
+    memset(&p, 0, sizeof(p));
+    p.D = D;
+    p.H = H;
+    p.W = W;
+    p.voxel_size = 1.0f;
+    p.A = p.U = p.V = INT_MAX;
+    fp_fill_layout(p);
+    fp_spread_edges(p, kEdgeSpreadBytes);
+    return Workspace::align(fp_edge_bytes(p));
+}
+
+// The volume-gradient buffer beside the quads: of large volumes the edge records take
+// about half of it
+size_t gradient_buffer_bytes(int D, int H, int W) {
+    return std::max(quad_volume_bytes(D, H, W), edge_record_bytes(D, H, W));
+}
 
 // Ray tile of the forward projector (8 detector columns x 32 rows per CTA):
 // the batched launches take per-instance tiles from the autotuner.
@@ -303,6 +321,7 @@ int dgc_project_backward(const float* grad_projection, const float* volume, int 
     p.quads = quads;
     p.grad_projections = grad_projection;
     p.grad_edges = edges;
+    if (edges) fp_spread_edges(p, gradient_buffer_bytes(D, H, W));
     p.partials = partials;
     rc = build_volume_quads(volume, D, H, W, quads, s);
     if (rc != DGC_OK) return rc;
@@ -319,14 +338,7 @@ int dgc_project_backward(const float* grad_projection, const float* volume, int 
 
 size_t dgc_project_adjoint_workspace_bytes(int D, int H, int W) {
     if (D <= 0 || H <= 0 || W <= 0) return 0;
-    FpArgs p;
-    memset(&p, 0, sizeof(p));
-    p.D = D;
-    p.H = H;
-    p.W = W;
-    p.voxel_size = 1.0f;
-    fp_fill_layout(p);
-    return Workspace::align(fp_edge_bytes(p));
+    return edge_record_bytes(D, H, W);
 }
 
 int dgc_project_adjoint(const float* grad_projection, int D, int H, int W, const float* angles,
@@ -360,6 +372,7 @@ int dgc_project_adjoint(const float* grad_projection, int D, int H, int W, const
     fp_fill_layout(p);
     Workspace ws(workspace, workspace_bytes);
     p.grad_projections = grad_projection;
+    fp_spread_edges(p, workspace_bytes & ~size_t(255));
     p.grad_edges = reinterpret_cast<float2*>(ws.take<char>(fp_edge_bytes(p)));
     if (!p.grad_edges) {
         set_error("workspace too small: dgc_project_adjoint needs " +

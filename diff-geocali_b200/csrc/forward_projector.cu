@@ -988,6 +988,11 @@ struct EdgeRun {
     f32x2 bb = 0, ba = 0, ab = 0, aa = 0;  // (x, y) behind / ahead: z and z+1 weights
 };
 
+// First record of the copy that this CTA adds into.
+__device__ __forceinline__ uint32_t edge_copy(const FpArgs& p) {
+    return (blockIdx.x & (p.ge_copies - 1u)) * p.ge_count;
+}
+
 // Per ray: one cell ahead in x, in y and in both as record-index steps, and the
 // bias that turns biased floors into the index of the edge behind.  An axis one
 // voxel thick has stride 0 (all its padded voxels are the one voxel), so its
@@ -997,6 +1002,7 @@ struct EdgeSteps {
     bool fx, fy;  // direction >= 0 along x, y
 };
 
+template <bool COPIES>
 __device__ __forceinline__ EdgeSteps edge_steps(const RaySetup& r, const FpArgs& p) {
     EdgeSteps e;
     e.fx = r.dx >= 0.0f;
@@ -1004,7 +1010,7 @@ __device__ __forceinline__ EdgeSteps edge_steps(const RaySetup& r, const FpArgs&
     e.dx = e.fx ? p.ge_x : 0u - p.ge_x;
     e.dy = e.fy ? p.ge_y : 0u - p.ge_y;
     e.bias = (1u - kFloorMagicBits) * (1u + p.ge_x + p.ge_y) + (e.fx ? 0u : p.ge_x) +
-             (e.fy ? 0u : p.ge_y);
+             (e.fy ? 0u : p.ge_y) + (COPIES ? edge_copy(p) : 0u);
     return e;
 }
 
@@ -1059,15 +1065,16 @@ __device__ __forceinline__ void add_sample(EdgeRun& run, const Cell& c, const Ed
     run.aa = fma2(pack2(aa, aa), z, run.aa);
 }
 
-// Spatial-gradient sums of a ray; GRADVOL: also its adjoint into p.grad_edges.
-template <bool CLAMP, bool GRADVOL, bool POW2, bool OFF, bool GUARD>
+// Spatial-gradient sums of a ray; GRADVOL: also its adjoint into p.grad_edges, 1 into
+// their one copy, 2 into this CTA's (looking for the copy costs the march 1 %).
+template <bool CLAMP, int GRADVOL, bool POW2, bool OFF, bool GUARD>
 __device__ __forceinline__ RayGrad march_grad(const RaySetup& r, const ViewGeo& vg,
                                               const FpArgs& p, float gs) {
     const ulonglong2* __restrict__ Q = reinterpret_cast<const ulonglong2*>(p.quads);
     const XYPacks k = make_xy_packs<!POW2>(r, vg, p);
     RayGrad rg{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     const int nmax = step_bound(r, p.step_size);
-    const EdgeSteps es = edge_steps(r, p);
+    const EdgeSteps es = edge_steps<GRADVOL == 2>(r, p);
     EdgeRun run;
     if (GRADVOL)
         run.eb = edge_index(sample_cell<CLAMP, false, OFF, POW2>(r.tmin, r, vg, p, k), p, es);
@@ -1131,7 +1138,7 @@ __device__ __forceinline__ void march_adjoint(const RaySetup& r, const ViewGeo& 
     EdgeSteps es;
     es.dx = sx > 0.0f ? p.ge_x : 0u - p.ge_x;
     es.dy = sy > 0.0f ? p.ge_y : 0u - p.ge_y;
-    es.bias = 1u + p.ge_x + p.ge_y - kFloorMagicBits * (1u + es.dx + es.dy);
+    es.bias = 1u + p.ge_x + p.ge_y - kFloorMagicBits * (1u + es.dx + es.dy) + edge_copy(p);
 
     struct Place {
         f32x2 ahead;
@@ -1250,7 +1257,7 @@ __device__ __forceinline__ void ray_geometry_terms(const FpArgs& p, const ViewGe
 // The eight per-view geometry terms of one ray (zero for rays outside the
 // detector, missing the volume or with a zero upstream gradient); with
 // GRADVOL (march_grad) the ray's adjoint samples go into p.grad_edges.
-template <bool GRADVOL, bool POW2, bool OFF>
+template <int GRADVOL, bool POW2, bool OFF>
 __device__ __forceinline__ void backward_ray(const FpArgs& p, const ViewGeo& vg, int a, int u,
                                              int v, float (&terms)[8]) {
 #pragma unroll
@@ -1299,7 +1306,7 @@ __device__ __forceinline__ void reduce_terms_to_partials(const float (&terms)[8]
 // POW2 without OFF is the march for power-of-two voxel sizes and no ROI offset
 // (sample_cell's packed form); every other case runs the general one, POW2 =
 // false and OFF = true, which is right for all of them.
-template <int TU, bool GRADVOL, bool POW2, bool OFF>
+template <int TU, int GRADVOL, bool POW2, bool OFF>
 __global__ void __launch_bounds__(256) fp_backward_kernel(FpArgs p) {
     constexpr int TV = 256 / TU;
     __shared__ ViewGeo s_view;
@@ -1459,6 +1466,7 @@ __device__ __forceinline__ float fold_column(const float2* __restrict__ e, int D
 
 // One 32 x 32 (x, z) tile of the folded gradient at row y: block (32, 8).  Reads
 // run along z and writes along x, through shared memory.
+template <bool COPIES>
 __device__ __forceinline__ void fold_edges_tile(const FpArgs& p, float* __restrict__ grad, int bx,
                                                 int by, float (&tile)[32][33]) {
     const int xtiles = (p.W + 31) / 32;
@@ -1473,8 +1481,16 @@ __device__ __forceinline__ void fold_edges_tile(const FpArgs& p, float* __restri
             const int xlo = p.ge_x && x == 0 ? -1 : 0, xhi = p.ge_x && x == p.W - 1 ? 1 : 0;
             const int ylo = p.ge_y && y == 0 ? -1 : 0, yhi = p.ge_y && y == p.H - 1 ? 1 : 0;
             for (int dy = ylo; dy <= yhi; ++dy)
-                for (int dx = xlo; dx <= xhi; ++dx)
-                    acc += fold_column(e + dy * (long long)p.ge_y + dx * (long long)p.ge_x, p.D, z);
+                for (int dx = xlo; dx <= xhi; ++dx) {
+                    const float2* c = e + dy * (long long)p.ge_y + dx * (long long)p.ge_x;
+                    if (!COPIES) {
+                        acc += fold_column(c, p.D, z);
+                        continue;
+                    }
+#pragma unroll 4
+                    for (uint32_t copy = 0; copy < p.ge_copies; ++copy, c += p.ge_count)
+                        acc += fold_column(c, p.D, z);
+                }
         }
         tile[xl][tx] = acc;
     }
@@ -1487,9 +1503,10 @@ __device__ __forceinline__ void fold_edges_tile(const FpArgs& p, float* __restri
 
 // grid: x = ceil(W/32) * H, y = ceil(D/32); block (32, 8).  Bound by memory: 12
 // bytes a voxel.
+template <bool COPIES>
 __global__ void __launch_bounds__(256) fold_edges_kernel(FpArgs p, float* __restrict__ grad) {
     __shared__ float tile[32][33];
-    fold_edges_tile(p, grad, blockIdx.x, blockIdx.y, tile);
+    fold_edges_tile<COPIES>(p, grad, blockIdx.x, blockIdx.y, tile);
 }
 
 // ---------------------------------------------------------------------------
@@ -1607,12 +1624,12 @@ __device__ __forceinline__ void backward_item(const FpArgs& p, const ViewGeo& vg
     tile_ray<TU>(tc, u, v);
     switch (flags & (kBatchDiv | kBatchOff)) {
         case 0:
-            if (p.grad_edges) backward_ray<true, true, false>(p, vg, tc.a, u, v, terms);
-            else backward_ray<false, true, false>(p, vg, tc.a, u, v, terms);
+            if (p.grad_edges) backward_ray<1, true, false>(p, vg, tc.a, u, v, terms);
+            else backward_ray<0, true, false>(p, vg, tc.a, u, v, terms);
             break;
         default:
-            if (p.grad_edges) backward_ray<true, false, true>(p, vg, tc.a, u, v, terms);
-            else backward_ray<false, false, true>(p, vg, tc.a, u, v, terms);
+            if (p.grad_edges) backward_ray<1, false, true>(p, vg, tc.a, u, v, terms);
+            else backward_ray<0, false, true>(p, vg, tc.a, u, v, terms);
             break;
     }
 }
@@ -1658,7 +1675,7 @@ __global__ void __launch_bounds__(256) batch_fold_kernel(BatchTables t) {
     const int i = find_instance(t.fold_block, t.n, blockIdx.x);
     const BatchInstance& in = t.inst[i];
     const long long b = blockIdx.x - t.fold_block[i];
-    fold_edges_tile(in.p, in.grad_volume, (int)(b % in.fold_gx), (int)(b / in.fold_gx), tile);
+    fold_edges_tile<false>(in.p, in.grad_volume, (int)(b % in.fold_gx), (int)(b / in.fold_gx), tile);
 }
 
 // ---------------------------------------------------------------------------
@@ -1690,11 +1707,16 @@ int launch_backward_tu(const FpArgs& p, bool gradvol, cudaStream_t s) {
     const bool fast = is_pow2_float(p.voxel_size) && p.off_x == 0.0f && p.off_y == 0.0f &&
                       p.off_z == 0.0f;
     if (gradvol) {
-        if (fast) fp_backward_kernel<TU, true, true, false><<<(unsigned)blocks, 256, 0, s>>>(p);
-        else fp_backward_kernel<TU, true, false, true><<<(unsigned)blocks, 256, 0, s>>>(p);
+        if (p.ge_copies > 1) {
+            if (fast) fp_backward_kernel<TU, 2, true, false><<<(unsigned)blocks, 256, 0, s>>>(p);
+            else fp_backward_kernel<TU, 2, false, true><<<(unsigned)blocks, 256, 0, s>>>(p);
+        } else {
+            if (fast) fp_backward_kernel<TU, 1, true, false><<<(unsigned)blocks, 256, 0, s>>>(p);
+            else fp_backward_kernel<TU, 1, false, true><<<(unsigned)blocks, 256, 0, s>>>(p);
+        }
     } else {
-        if (fast) fp_backward_kernel<TU, false, true, false><<<(unsigned)blocks, 256, 0, s>>>(p);
-        else fp_backward_kernel<TU, false, false, true><<<(unsigned)blocks, 256, 0, s>>>(p);
+        if (fast) fp_backward_kernel<TU, 0, true, false><<<(unsigned)blocks, 256, 0, s>>>(p);
+        else fp_backward_kernel<TU, 0, false, true><<<(unsigned)blocks, 256, 0, s>>>(p);
     }
     DGC_LAUNCH_CHECK("fp_backward_kernel");
     return DGC_OK;
@@ -1703,13 +1725,29 @@ int launch_backward_tu(const FpArgs& p, bool gradvol, cudaStream_t s) {
 }  // namespace
 
 size_t fp_edge_bytes(const FpArgs& p) {
-    return sizeof(float2) * p.ge_count;
+    return sizeof(float2) * (size_t)p.ge_count * p.ge_copies;
+}
+
+// A small volume under many rays: all of them add to the same few records, an addition
+// at a time.  A copy per 32 rays a record, up to 16 and 512 KB, takes that apart.  Volume
+// gradient alone, one copy -> several: 4 x 4 x 14 / 91 x 310 x 82 1.52 -> 0.19 ms, 14 x 5 x
+// 15 / 172 x 71 x 131 0.73 -> 0.18, 13 x 21 x 36 / 127 x 653 x 167 4.67 -> 2.96; with one
+// copy such volumes took up to 2.1 times what the 16-byte level records of a cell had,
+// which share no address between cells.  Below 32 the
+// fold of the copies costs more than they save.
+void fp_spread_edges(FpArgs& p, size_t bytes) {
+    const size_t most = std::min<size_t>(bytes, kEdgeSpreadBytes);
+    const double rays = (double)p.A * p.U * p.V / (32.0 * (double)p.ge_count);
+    p.ge_copies = 1;
+    while (p.ge_copies < 16 && 2 * p.ge_copies <= rays && 2 * fp_edge_bytes(p) <= most)
+        p.ge_copies *= 2;
 }
 
 int fp_fold_edges(const FpArgs& p, float* grad, cudaStream_t s) {
     DGC_TRACE("fold_edges", s);
     const dim3 grid((unsigned)(ceil_div(p.W, 32) * (long long)p.H), (unsigned)ceil_div(p.D, 32));
-    fold_edges_kernel<<<grid, dim3(32, 8), 0, s>>>(p, grad);
+    if (p.ge_copies > 1) fold_edges_kernel<true><<<grid, dim3(32, 8), 0, s>>>(p, grad);
+    else fold_edges_kernel<false><<<grid, dim3(32, 8), 0, s>>>(p, grad);
     DGC_LAUNCH_CHECK("fold_edges");
     return DGC_OK;
 }
@@ -1731,7 +1769,8 @@ void fp_fill_layout(FpArgs& p) {
     const uint32_t column = (uint32_t)(p.D >= 16 ? (p.D + 4) & ~3 : p.D + 1);
     p.ge_x = p.W > 1 ? column : 0u;
     p.ge_y = p.H > 1 ? column * (uint32_t)(p.W > 1 ? p.W + 2 : 1) : 0u;
-    p.ge_count = (size_t)column * (size_t)(p.W > 1 ? p.W + 2 : 1) * (size_t)(p.H > 1 ? p.H + 2 : 1);
+    p.ge_count = column * (uint32_t)(p.W > 1 ? p.W + 2 : 1) * (uint32_t)(p.H > 1 ? p.H + 2 : 1);
+    p.ge_copies = 1;
     p.inv_voxel = 1.0f / p.voxel_size;
 }
 

@@ -19,7 +19,8 @@ struct FpArgs {
     const float* grad_projections;  // [A][U][V]
     float2* grad_edges;             // edge records E[yp*ge_y + xp*ge_x + zp] or null
     uint32_t ge_x, ge_y;
-    size_t ge_count;                // records in all
+    uint32_t ge_count;              // records of a copy (below 2^32: two a padded quad at most)
+    uint32_t ge_copies;             // copies, a power of two: CTAs add into one in turn
     double* partials;  // [A][tiles][8]
     int* error;        // device word set to 1 when a bounded wait gives up (TMA arm), or null
     int view_block;    // CTA order: 0 = u tile fastest; B > 0 = views in blocks of B (tile_coord),
@@ -75,9 +76,12 @@ void fp_fill_layout(FpArgs& p);
 long long fp_tiles_per_view(int U, int V, int tu);
 // Volume gradient of the backward: the weights of a ray's samples are gathered
 // in registers and emitted as 8-byte reductions into edge records
-// (fp_edge_bytes, after fp_fill_layout; at most the 16 bytes per padded quad
-// that the workspace queries grant), then folded onto the voxels.
+// (fp_edge_bytes, after fp_fill_layout; a copy at most the 16 bytes per padded quad
+// that the workspace queries grant), then folded onto the voxels.  fp_fill_layout
+// gives one copy; fp_spread_edges as many as suit the volume and `bytes` hold.
+constexpr size_t kEdgeSpreadBytes = 512 << 10;
 size_t fp_edge_bytes(const FpArgs& p);
+void fp_spread_edges(FpArgs& p, size_t bytes);
 int fp_fold_edges(const FpArgs& p, float* grad, cudaStream_t s);
 int build_volume_quads(const float* vol, int D, int H, int W, float4* quads, cudaStream_t s);
 // The forward's arm, slab, unroll and CTA order for a volume (the arm rules).

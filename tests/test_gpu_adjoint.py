@@ -50,3 +50,41 @@ def test_volume_gradient_alone(options, oracle):
     assert rel_l2(alone.cpu(), truth) < GRAD_RTOL
     assert rel_l2(nine.cpu(), truth) < GRAD_RTOL
     assert rel_l2(alone.cpu(), nine.cpu()) < SAME_RTOL
+
+
+@pytest.mark.parametrize("shape,A,U,V", [
+    ((9, 8, 7), 8, 40, 30),      # 13 rays a record: one copy of the records
+    ((9, 8, 7), 10, 60, 100),    # two, four, eight, sixteen
+    ((9, 8, 7), 20, 60, 100), ((9, 8, 7), 40, 60, 100), ((9, 8, 7), 40, 100, 200),
+    ((20, 20, 20), 90, 100, 100),  # as many as 512 KB hold
+    ((1, 6, 5), 30, 40, 30), ((5, 1, 6), 30, 40, 30), ((2, 3, 40), 30, 60, 30)])
+def test_copies_of_the_records(shape, A, U, V):
+    """Small volumes under many rays, whose CTAs add into several copies of the records:
+    the volume gradient alone and beside the geometry's, against that in a workspace
+    of one copy, which adds the same samples."""
+    from dgc_b200 import _native
+
+    case = random_case(17, shape=shape, A=A, U=U, V=V, vs=4.0, step=1.3, off=(0.0, 0.0, 0.0))
+    out, vol, geom = run_project(case, requires_grad=True)
+    up = cuda32(np.random.default_rng(4).normal(size=tuple(out.shape)))
+    nine = torch.autograd.grad(out, [vol, *geom], grad_outputs=up)[0]
+    alone_vol = cuda32(case["vol"]).requires_grad_()
+    alone_out, _, _ = run_project(case, vol=alone_vol)
+    (alone,) = torch.autograd.grad(alone_out, [alone_vol], grad_outputs=up)
+    D, H, W = shape
+    column = (D + 4) // 4 * 4 if D >= 16 else D + 1
+    n = 8 * column * (W + 2 if W > 1 else 1) * (H + 2 if H > 1 else 1)
+    n = (n + 255) // 256 * 256
+    lib, ws, one = _native.lib(), torch.empty(n, dtype=torch.uint8, device="cuda"), torch.empty_like(alone)
+    g = [cuda32(x) for x in case["geom"]]
+
+    def call(nbytes):
+        return lib.dgc_project_adjoint(
+            up.data_ptr(), D, H, W, *[x.data_ptr() for x in g], A, case["px"], U, V, case["step"],
+            case["vs"], 0.0, 0.0, 0.0, one.data_ptr(), ws.data_ptr(), nbytes,
+            torch.cuda.current_stream().cuda_stream)
+
+    assert call(n) == 0 and call(n - 256) == 3
+    assert float(one.abs().sum()) > 0.0
+    assert rel_l2(alone.cpu(), one.cpu()) < SAME_RTOL
+    assert rel_l2(nine.cpu(), one.cpu()) < SAME_RTOL

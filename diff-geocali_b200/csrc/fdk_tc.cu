@@ -675,13 +675,14 @@ void fdk_tc_limit_waits(int polls) { tc_polls = std::max(polls, -1); }
 int fdk_tc_views(int A, int U, int V, bool adjoint) {
     // Below, the FP32 product's time is that of its chain over U, the tensor cores' that of
     // their launches and of rows that the tile of 128 pads.  Tensor cores / FP32, over
-    // 1 to 512 views of 16 to 600 columns: the filter 0.68-1.14 at U = 96, 0.66-1.09 at
-    // 112, 0.63-0.98 at 128, 0.40-0.66 at 256; the adjoint, whose epilogue is a launch of
+    // 1 to 512 views of 16 to 600 columns: the filter 0.68-1.14 at U = 96 (0.79-1.04 to 64
+    // columns), 0.66-1.09 at 112 (0.79-1.05 to 128), 0.63-0.98 at 128, 0.40-0.66 at 256; the adjoint, whose epilogue is a launch of
     // its own, 0.77-1.25 at 96, 0.82-1.20 at 128, 0.56-1.16 at 129 to 160 (0.56-1.08
     // from 96 columns), 0.56-1.07 at 192, 0.54-0.94 at 256.  To 2048: the strip and two stages
     // fill the shared memory.  The rule has no number of views in it, so that a view's
     // result does not depend on its neighbours.
-    const bool rows = adjoint ? U >= 192 || (U >= 129 && V >= 96) : U >= 128;
+    const bool rows = adjoint ? U >= 192 || (U >= 129 && V >= 96)
+                              : U >= (V <= 64 ? 96 : V <= 128 ? 112 : 128);
     if (A < 1 || !rows || U > 2048 || V < 16 || tc_split_bytes(U, V) > kTcChunkBytes) return 0;
     const int most = (int)std::min<long long>(16384, (long long)(kTcChunkBytes / tc_split_bytes(U, V)));
     return ceil_div(A, ceil_div(A, most));  // equal chunks

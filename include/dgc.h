@@ -184,10 +184,10 @@ int dgc_backproject_adjoint(const float* grad_volume, int A, int U, int V,
  * filter (filtering.py:87-103) as a symmetric Toeplitz kernel, FP64. */
 int dgc_fdk_filter_taps(int U, double pixel_size, double alpha, double* taps);
 
-/* Scratch of dgc_fdk_filter.  For U from 128 to 2048 and V >= 16 (the adjoint: U from
- * 192, or from 129 where V >= 96) the filter runs on the tensor cores, and the
- * workspace holds the split operands of up to 256 MB of views; a smaller one is
- * taken too.  ..._at_a_time is what the filter (adjoint 1:
+/* Scratch of dgc_fdk_filter.  For V >= 16 and U to 2048 from 128 (96 where V <= 64,
+ * 112 where V <= 128; the adjoint: from 192, 129 where V >= 96) the filter runs on
+ * the tensor cores, and the workspace holds the split operands of up to 256 MB of
+ * views; a smaller one is taken too.  ..._at_a_time is what the filter (adjoint 1:
  * dgc_fdk_filter_backward) takes with `views` views at a time there: the results are
  * the same bit for bit, whatever their number.  With room for none (views 0) the
  * filter is an FP32 product, whose results differ by both products' rounding

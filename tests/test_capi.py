@@ -186,7 +186,8 @@ def test_header_is_c99_and_links_from_c(tmp_path):
 
 
 @pytest.mark.parametrize("U,V,forward,adjoint", [
-    (96, 600, False, False), (127, 256, False, False), (128, 16, True, False), (128, 600, True, False),
+    (95, 40, False, False), (96, 64, True, False), (96, 65, False, False), (111, 128, False, False),
+    (112, 128, True, False), (127, 129, False, False), (128, 16, True, False), (128, 600, True, False),
     (129, 95, True, False), (129, 96, True, True), (191, 95, True, False), (192, 16, True, True),
     (2048, 24, True, True), (2049, 300, False, False), (768, 15, False, False)])
 def test_filter_sizes_of_the_tensor_cores(U, V, forward, adjoint):

@@ -683,7 +683,7 @@ __global__ void __launch_bounds__(256) bp_reduce_partials_kernel(const double* _
 // row meet another CTA's: two additions onto zero, so the result does not
 // depend on scheduling.
 //
-// Bound by issue (73 % of the slots): 34 instructions a column and pixel, the
+// Bound by issue (73 % of the slots): 30 instructions a column and pixel, the
 // listing among them 2 %.
 
 // Upstream volume as z-fastest columns, zeros around them:
@@ -1025,15 +1025,12 @@ __global__ void __launch_bounds__(32 * kAdjMaxWarps, NV < 3 ? 4 : 3)
 // Launchers
 // ---------------------------------------------------------------------------
 
-// Z values per lane (a warp covers 32*KZ voxels of a column, a CTA 8 columns).
-// Fewer Z per warp keep the projection rows a CTA reads per view short, so
-// they stay in L1; more amortise the per-(column, view) geometry.  Measured
-// (sid 1000, sod 600; 256^3 / 360 x 384^2, 128^3 / 180 x 256^2, 512^3 / 90 x
-// 512^2), forward KZ = 1 / 2 / 4 / 8: 9.07 / 8.18 / 11.6 / 14.1 ms,
-// 0.46 / 0.36 / 0.52 / 0.52 ms, 17.0 / 13.7 / 14.5 / 15.5 ms (before the
-// super-tile order).  Backward at 256^3 / 360 x 384^2 (current kernel),
-// KZ = 2 / 4 / 8: 12.6 / 10.5 / 10.9 ms without the projection gradient,
-// 22.9 / 25.1 / 28.7 ms with it.
+// Z values per lane: a warp covers 32*KZ voxels of a column.  Fewer keep the projection
+// rows that a CTA reads per view short, so that they stay in L1; more amortise the
+// per-(column, view) geometry.  The forward's choice is bp_forward_tile's.  Backward at
+// 256^3 / 360 x 384^2, 8 columns a CTA, KZ = 2 / 4 / 8: 12.6 / 10.5 / 10.9 ms without the
+// projection gradient, 22.9 / 25.1 / 28.7 ms with it.
+
 // Tile rules registered by the autotuner (dgc_bp_add_tile_rule): the first
 // rule with D <= d_max and A <= a_max applies; a zero field keeps the
 // built-in choice.

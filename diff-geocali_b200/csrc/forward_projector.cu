@@ -349,12 +349,12 @@ __device__ __forceinline__ XYPacks make_xy_packs(const RaySetup& r, const ViewGe
     return k;
 }
 
-// Cell of the sample at t.  With PACK and no clamping, x and y run as packed pairs (fma.rn / sub.rn / add.rm on
-// f32x2): lane by lane the same IEEE operations as the scalar path, so the
-// cell and weights are bitwise those of locate(to_voxel(...)).  On the forward
-// sum 1-3 % faster; the gradient marches, together with dropping the iteration
-// counter and a zero ROI offset, 48.6 -> 43.2 ms (geometry gradients) and 46.7
-// -> 45.5 ms (fused calibration step) at 256^3 / 360 x 384^2.
+// Cell of the sample at t.  With PACK and no clamping, x and y run as packed pairs
+// (fma.rn / sub.rn / add.rm on f32x2): lane by lane the same IEEE operations as the
+// scalar path, so the cell and weights are bitwise those of locate(to_voxel(...)).  On
+// the forward sum 1-3 % faster; the gradient marches, together with dropping the
+// iteration counter and a zero ROI offset, 48.6 -> 43.2 ms (geometry gradients) and
+// 46.7 -> 45.5 ms (fused calibration step) at 256^3 / 360 x 384^2.
 template <bool CLAMP, bool DIV, bool OFF, bool PACK>
 __device__ __forceinline__ Cell sample_cell(float t, const RaySetup& r, const ViewGeo& vg,
                                             const FpArgs& p, const XYPacks& k) {
@@ -396,9 +396,9 @@ __device__ __forceinline__ uint32_t quad_index(const Cell& c, const FpArgs& p) {
 // then read the same 32 bytes: those keep the previous sample's registers and
 // issue no load.  Bitwise the same values as loading every sample.  Used by
 // the value march where it goes sample by sample (the batch kernel, the unrolled
-// arm): the batched forward of that instance plus its half went
-// from 50.9 to 48.1 ms, while the gradient marches, which hold more live
-// values, slowed by 2-17 % with it.
+// arm): the batched forward of 256^3 / 360 x 384^2 plus its half went from 50.9
+// to 48.1 ms, while the gradient marches, which hold more live values, slowed
+// by 2-17 % with it.
 struct CellQuads {
     uint32_t qi = 0xffffffffu;  // no quad index reaches 2^32 - 1
     ulonglong2 q0 = {0ull, 0ull}, q1 = {0ull, 0ull};
@@ -425,8 +425,9 @@ __device__ __forceinline__ float quad_value(const ulonglong2& q0, const ulonglon
 
 // Samples whose loads fp_forward_kernel has in flight at once.  One at a time, the march
 // waited for its loads (9 of 18 warp-cycles per instruction) with issue and FMA pipe at
-// 65 %; four at a time load also where samples share their cell, and fill the L1 pipe
-// instead: 256^3 / 360 x 384^2 35.2 -> 34.1 ms, 512^3 / 96 x 768^2 86.0 -> 82.8, 128^3 of
+// 65 %; four at a time load also where samples share their cell, and take more of the L1
+// data pipe instead (77 % of its cycles at 256^3, 81 % at 512^3, with issue at 61 and 52
+// % and half of the waiting still for loads): 256^3 / 360 x 384^2 35.2 -> 34.1 ms, 512^3 / 96 x 768^2 86.0 -> 82.8, 128^3 of
 // 4.0 / 180 x 256^2 at step 2 4.48 -> 4.09, 32^3 / 24 x 48^2 28 -> 24 us.  The other
 // forms tried took 34-37 ms, 88-92 and 4.2-4.5: two, three or five in flight, three CTAs
 // per SM instead of four, whole groups without predicates, and the cell's index computed
@@ -575,8 +576,8 @@ __global__ void __launch_bounds__(256, 4) fp_forward_kernel(FpArgs p) {
     const ViewGeo vg = s_view;
     int u, v;
     // with view blocks (the order for volumes beyond L2) warps take 4 x 8 ray
-    // patches: 671.3 -> 658.9 ms at 512^3 / 720 x 768^2, while at 256^3 /
-    // 720 x 384^2 the 4 x 8 patches are 1.3 % slower than 1 x 32 columns (the
+    // patches: 671.3 -> 658.9 ms at 512^3 / 720 x 768^2 (one sample in flight), while
+    // at 256^3 / 360 x 384^2 they are slower than 1 x 32 columns, 36.5 vs 34.1 ms (the
     // autotuner's view-block arms carry the patches, so its timings include
     // them; the projections are the same)
     if (TU % 4 == 0 && p.view_block > 0) tile_ray<TU, (TU % 4 == 0 ? 4 : 1)>(tc, u, v);
@@ -971,16 +972,18 @@ __device__ __forceinline__ QuadGradient quad_gradient(const ulonglong2& q0, cons
 // edges it leaves behind and carries the two of the shared face along.  Seen
 // along the ray, "behind" and "ahead" are fixed per axis by the sign of its
 // direction, so an x crossing always leaves the edges behind in x, a y
-// crossing those behind in y.  A move in z (rare: the rays are nearly
-// horizontal) or of more than a cell emits all four.
+// crossing those behind in y.  A move in z or of more than a cell emits all four:
+// rare where the rays are nearly horizontal, as in a scan of small cone angle (at 60
+// degrees, 260 x 15 x 15 from a source at 70 voxels, 1.2 times the time of 16-byte
+// records of both z levels).
 //
 // Why: reductions cost by the element, not by the instruction (1.2-1.45e12 float
 // additions/s in L2 on a B200 whatever the vector width), and a crossing emits
 // 4 elements instead of the 8 of both z levels of all four columns (16-byte
 // level records, which the reductions bound: 1.36e11 additions a call at 256^3 /
-// 360 x 384^2).  What binds now is issue, 117 instructions a sample with the
-// gradient sums and 72 without, at 77 % of the slots, beside L2 additions at 60
-// % in the march without the sums.  Level records -> edges, all nine gradients:
+// 360 x 384^2).  What binds now is issue, 101 instructions a sample with the
+// gradient sums and 68 without, at 72 and 74 % of the slots, beside L2's additions at
+// 40 and 60 % of their cycles.  Level records -> edges, all nine gradients:
 // 103.1 -> 101.2 ms (256^3 / 360 x 384^2), 280 -> 266 ms (512^3 / 96 x 768^2).
 // Emitting through a branch per edge with the columns recomputed took 153.7 ms.
 struct EdgeRun {
@@ -1112,11 +1115,11 @@ __device__ __forceinline__ RayGrad march_grad(const RaySetup& r, const ViewGeo& 
 // weights.  109.2 -> 66.9 ms at 256^3 / 360 x 384^2, 10.1 -> 5.6 ms at 128^3 /
 // 180 x 256^2 and 287 -> 185 ms at 512^3 / 96 x 768^2 against the march with the
 // gradient sums and level records (the volume's quads are not built either).
-// Per sample and SM it takes 23.4 cycles against about 20 for its 3.1 additions a
-// lane and 18 for its 72 instructions; view blocks change nothing (186 ms).  x and y run mirrored (negated) where the ray travels towards lower
-// indices, so that "behind" is the floor along every ray and neither weights nor
-// indices need a selection by direction; the negated multiply-adds round as the
-// original ones.  At a coordinate exactly on a voxel the mirrored cell is the
+// Per sample and SM it takes 23.5 cycles against about 20 for its 3.1 additions a
+// lane and 17 for its 68 instructions; view blocks change nothing (186 ms).  x and y
+// run mirrored (negated) where the ray travels towards lower indices, so that
+// "behind" is the floor along every ray and neither weights nor indices need a
+// selection by direction; the negated multiply-adds round as the original ones.  At a coordinate exactly on a voxel the mirrored cell is the
 // one on its other side, with the same weights.
 template <bool CLAMP, bool POW2, bool OFF, bool GUARD>
 __device__ __forceinline__ void march_adjoint(const RaySetup& r, const ViewGeo& vg,
@@ -1867,9 +1870,10 @@ void fp_forward_arm(int D, int H, int W, int* arm, int* slab, int* unroll, int* 
             *view_block = g_arm_rules[i].view_block;
             return;
         }
-    // built-in choice: the L1 arm; above 2^26 voxels (512^3: 90.4 vs 94.1 ms
-    // for 96 views of 768^2) CTAs in view blocks of 16, below (256^3) the
-    // order makes no difference
+    // built-in choice: the L1 arm; above 2^26 voxels CTAs in view blocks of 16 with 4 x 8
+    // patches (512^3 / 96 x 768^2: 82.9 vs 83.7 ms), below every u tile of a view first
+    // (400^3 / 120 x 640^2 51.6 vs 52.7, 256^3 / 360 x 384^2 34.1 vs 36.5, 128^3 / 180 x
+    // 256^2 3.07 vs 3.00)
     *arm = 0;
     *slab = 0;
     *unroll = 1;
@@ -1945,9 +1949,9 @@ int fp_launch_backward(const FpArgs& p, const FpTile& tile, bool gradvol, cudaSt
 }
 
 int fp_mse_tile(int D, int H, int W) {
-    // 4 columns up to 256^3 voxels, 8 beyond: 51.0 vs 52.7 ms at 256^3 / 360 x
-    // 384^2 and 5.84 vs 6.06 ms at 128^3 / 180 x 256^2, but 1145 vs 930 ms at
-    // 512^3 / 720 x 768^2
+    // 4 columns up to 256^3 voxels, 8 beyond: 4.20 vs 4.25 ms at 128^3 / 180 x 256^2
+    // and no difference at 256^3 (45.5 / 45.3), but 59.7 vs 55.3 ms at 320^3 / 200 x 512^2
+    // and 82.1 vs 69.9 at 400^3 / 120 x 640^2
     return (long long)D * H * W <= 256LL * 256 * 256 ? 4 : 8;
 }
 

@@ -49,7 +49,7 @@ __global__ void im2col_nhwc_kernel(const __nv_bfloat16* __restrict__ x, int B, i
 }
 
 // Eight channels (16 bytes) of one tap a thread; a block walks the chunks of one
-// output row (b, oy).  @IM2COL@
+// output row (b, oy).
 __global__ void __launch_bounds__(256) im2col_row_kernel(const __nv_bfloat16* __restrict__ x, int H,
                                                          int W, int C, int kh, int kw, int stride,
                                                          int pad, int Ho, int Wo,

@@ -1119,8 +1119,9 @@ __device__ __forceinline__ RayGrad march_grad(const RaySetup& r, const ViewGeo& 
 // lane and 17 for its 68 instructions; view blocks change nothing (186 ms).  x and y
 // run mirrored (negated) where the ray travels towards lower indices, so that
 // "behind" is the floor along every ray and neither weights nor indices need a
-// selection by direction; the negated multiply-adds round as the original ones.  At a coordinate exactly on a voxel the mirrored cell is the
-// one on its other side, with the same weights.
+// selection by direction; the negated multiply-adds round as the original ones.
+// At a coordinate exactly on a voxel the mirrored cell is the one on its other
+// side, with the same weights.
 template <bool CLAMP, bool POW2, bool OFF, bool GUARD>
 __device__ __forceinline__ void march_adjoint(const RaySetup& r, const ViewGeo& vg,
                                               const FpArgs& p, float gs) {

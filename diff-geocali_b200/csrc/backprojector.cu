@@ -1217,6 +1217,7 @@ size_t bp_column_floats(int D, int H, int W) { return (size_t)(D + 3) * H * W; }
 // launch that was not taken costs: 10-30 us.
 bool bp_may_gather(int A, int U, int V, int D, int H, int W, bool with_geometry) {
     const long long area = (long long)H * W;
+    if (D > 1 << 20) return false;  // bp_columns' grid
     if (with_geometry) return D >= 100 && V >= 48 && area >= 25LL * (U - 1) && area * A >= 1600000;
     return A >= 6 && D >= 48 && V >= 48 && area >= 15LL * (U - 1);
 }

@@ -216,3 +216,16 @@ def test_volume_gradient_alone_asks_for_its_edge_records(D, H, W):
     copies = max(c for c in (1, 2, 4, 8, 16) if c == 1 or 8 * records * c <= 512 << 10)
     got = _native.lib().dgc_project_adjoint_workspace_bytes(D, H, W)
     assert got == (8 * records * copies + 255) // 256 * 256
+
+
+def test_gather_scratch_by_size():
+    """The projection gradient asks for a copy of the volume where a gather may take it:
+    deep columns, several views, and no more slices than the copy's launch holds."""
+    from dgc_b200 import _native
+
+    lib = _native.lib()
+    for A, D, H, W, copy in ((6, 48, 10, 10, True), (5, 48, 10, 10, False), (6, 47, 10, 10, False),
+                             (6, 48, 3, 4, False), (6, 1 << 20, 4, 4, True), (6, (1 << 20) + 1, 4, 4, False)):
+        extra = lib.dgc_backproject_adjoint_workspace_bytes(A, D, H, W) - \
+            lib.dgc_backproject_adjoint_least_workspace_bytes(A)
+        assert extra == ((4 * (D + 3) * H * W + 255) // 256 * 256 if copy else 0), (A, D, H, W)
